@@ -51,3 +51,14 @@ def test_order_of_gpu_ridge(rdb):
     order, starts = rdb.order_chains(S, 0.3)
     assert np.array_equal(order, O.order(S, 0.3)[0])
     assert starts[-1] == S.shape[0]
+
+
+@pytest.mark.parametrize("ns", [2, 31, 32, 33, 1023, 1024, 1025])
+def test_order_at_word_and_path_edges(rdb, ns):
+    """Around the words of the alive mask and the largest ridge the bit walk takes."""
+    S = np.random.default_rng(ns).random((ns, 2)).astype(np.float32)
+    r2 = 1.2 / np.sqrt(ns)
+    order, starts = rdb.order_chains(S, r2)
+    ref_order, ref_starts = O.order(S, r2)
+    assert np.array_equal(starts, ref_starts)
+    assert np.array_equal(order, ref_order)
