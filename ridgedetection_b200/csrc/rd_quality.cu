@@ -5,12 +5,13 @@
 //   stats(S, I)     = min, max, median (sorted[n/2]) and mean (float sum in
 //                     sorted order / n) of distance(s, I)
 //   segment(T)      = max over T of sqrt(sum over d >= 1 of t_d^2)
-// The min-distance search is all pairs, one thread per four points against
-// shared-memory tiles of the other set; the mean's ordered sum uses the exact
+// The min-distance search is all pairs, threads holding points of one set
+// against shared-memory tiles of a slice of the other; the mean's ordered sum uses the exact
 // parallel fold (rd_fold.cuh), so it equals the sequential float sum.
 #include "rd_engine.cuh"
 #include "rd_fold.cuh"
 
+#include <algorithm>
 #include <cfloat>
 #include <cub/cub.cuh>
 #include <cuda_runtime.h>
@@ -18,45 +19,88 @@
 namespace rdb {
 namespace {
 
-constexpr int Q_BLOCK = 256, Q_ITEMS = 4, Q_TILE = 1024;
+constexpr int Q_TILE = 1024;
 
+// one row of the staged tile (PadDim<DIM> floats, one vector load)
 template <int DIM>
-__global__ void __launch_bounds__(Q_BLOCK) k_min_dist(const float* __restrict__ A, int na,
-                                                      const float* __restrict__ B, int nb,
-                                                      float* __restrict__ out)
+__device__ __forceinline__ void load_tile_row(const float* sB, int k, float* s)
 {
-    __shared__ float sB[Q_TILE * DIM];
+    constexpr int DP = PadDim<DIM>::v;
+    if constexpr (DP == 4) {
+        const float4 t = reinterpret_cast<const float4*>(sB)[k];
+        s[0] = t.x; s[1] = t.y; s[2] = t.z;
+        if constexpr (DIM == 4) s[3] = t.w;
+    } else if constexpr (DP == 2) {
+        const float2 t = reinterpret_cast<const float2*>(sB)[k];
+        s[0] = t.x; s[1] = t.y;
+    } else {
+        s[0] = sB[k];
+    }
+}
+
+// Smallest squared distance of each point of A to the slice blockIdx.y of B
+// (slices of `per` points), merged over the slices with an integer minimum:
+// the values are sums of squares, so their bit patterns order as they do, and
+// a minimum does not depend on the order it is taken in.  out holds FLT_MAX
+// before; a NaN distance never passes the strict '<'.
+// Bound by the FP32 pipe once enough CTAs are in flight: 3 DIM - 1 rounded
+// operations and a minimum per pair.  The slices are what fills the chip when
+// A is a ridge of a few hundred points: 300 points against 100,000 in 3D took
+// 5,770 us as one CTA over all of B, 21 us in 148 x 4 CTAs (whose floor by
+// operations is 8 us: each slice re-reads its points through L2).
+template <int DIM, int BLOCK, int ITEMS>
+__global__ void __launch_bounds__(BLOCK) k_min_dist(const float* __restrict__ A, int na,
+                                                    const float* __restrict__ B, int nb, int per,
+                                                    unsigned* __restrict__ out)
+{
+    constexpr int DP = PadDim<DIM>::v;
+    __shared__ __align__(16) float sB[Q_TILE * DP];
     const int tid = threadIdx.x;
-    const int i0 = blockIdx.x * Q_BLOCK * Q_ITEMS + tid;
-    float p[Q_ITEMS][DIM], best[Q_ITEMS];
+    const int i0 = blockIdx.x * BLOCK * ITEMS + tid;
+    const int b0 = (int)min((int64_t)nb, (int64_t)blockIdx.y * per);
+    const int b1 = (int)min((int64_t)nb, (int64_t)b0 + per);
+    float p[ITEMS][DIM], best[ITEMS];
 #pragma unroll
-    for (int j = 0; j < Q_ITEMS; ++j) {
-        const int i = i0 + j * Q_BLOCK;
+    for (int j = 0; j < ITEMS; ++j) {
+        const int64_t i = i0 + (int64_t)j * BLOCK;
 #pragma unroll
-        for (int d = 0; d < DIM; ++d) p[j][d] = (i < na) ? A[(int64_t)i * DIM + d] : 0.0f;
+        for (int d = 0; d < DIM; ++d) p[j][d] = (i < na) ? A[i * DIM + d] : 0.0f;
         best[j] = FLT_MAX;
     }
-    for (int t0 = 0; t0 < nb; t0 += Q_TILE) {
-        const int tl = min(Q_TILE, nb - t0);
+    for (int t0 = b0; t0 < b1; t0 += Q_TILE) {
+        const int tl = min(Q_TILE, b1 - t0);
         __syncthreads();
-        for (int e = tid; e < tl * DIM; e += Q_BLOCK) sB[e] = B[(int64_t)t0 * DIM + e];
+        for (int e = tid; e < tl * DIM; e += BLOCK)
+            sB[(e / DIM) * DP + e % DIM] = B[(int64_t)t0 * DIM + e];
         __syncthreads();
+#pragma unroll 4
         for (int k = 0; k < tl; ++k) {
             float s[DIM];
+            load_tile_row<DIM>(sB, k, s);
 #pragma unroll
-            for (int d = 0; d < DIM; ++d) s[d] = sB[k * DIM + d];
-#pragma unroll
-            for (int j = 0; j < Q_ITEMS; ++j) {
+            for (int j = 0; j < ITEMS; ++j) {
                 const float dd = sqdist_exact<DIM>(p[j], s);
                 if (dd < best[j]) best[j] = dd;
             }
         }
     }
 #pragma unroll
-    for (int j = 0; j < Q_ITEMS; ++j) {
-        const int i = i0 + j * Q_BLOCK;
-        if (i < na) out[i] = sqrtf(best[j]);
+    for (int j = 0; j < ITEMS; ++j) {
+        const int64_t i = i0 + (int64_t)j * BLOCK;
+        if (i < na) atomicMin(&out[i], __float_as_uint(best[j]));
     }
+}
+
+__global__ void __launch_bounds__(256) k_fill_far(float* out, int n)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) out[i] = FLT_MAX;
+}
+
+__global__ void __launch_bounds__(256) k_sqrt(float* d, int n)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) d[i] = sqrtf(d[i]);
 }
 
 template <int DIM>
@@ -114,7 +158,23 @@ __global__ void __launch_bounds__(256) k_stats(const float* sorted, const int32_
     }
 }
 
-inline int q_grid(int n) { return (n + Q_BLOCK * Q_ITEMS - 1) / (Q_BLOCK * Q_ITEMS); }
+// Slices of B so that the grid holds at least Q_CTAS CTAs (four per SM), each
+// slice of at least Q_MIN_SLICE points (a shorter one spends more on its
+// start than on its pairs).
+constexpr int Q_CTAS = 148 * 4, Q_MIN_SLICE = 128;
+
+template <int DIM, int BLOCK, int ITEMS>
+cudaError_t min_dist_grid(const float* A, int na, const float* B, int nb, unsigned* out,
+                          cudaStream_t st)
+{
+    const int64_t gx = ((int64_t)na + BLOCK * ITEMS - 1) / (BLOCK * ITEMS);
+    const int64_t want = (Q_CTAS + gx - 1) / gx;
+    const int64_t most = std::max<int64_t>(1, ((int64_t)nb + Q_MIN_SLICE - 1) / Q_MIN_SLICE);
+    const int64_t gy = std::max<int64_t>(1, std::min(want, most));
+    const int per = (int)(((int64_t)nb + gy - 1) / gy);
+    k_min_dist<DIM, BLOCK, ITEMS><<<dim3((unsigned)gx, (unsigned)gy), BLOCK, 0, st>>>(A, na, B, nb, per, out);
+    return cudaGetLastError();
+}
 
 }  // namespace
 
@@ -122,10 +182,19 @@ cudaError_t launch_min_dist(int dim, const float* A, int na, const float* B, int
                             cudaStream_t st)
 {
     if (na <= 0) return cudaSuccess;
-    return with_dim(dim, [&](auto D) {
-        k_min_dist<decltype(D)::value><<<q_grid(na), Q_BLOCK, 0, st>>>(A, na, B, nb, out);
-        return cudaGetLastError();
+    // a small A takes one point per thread: fewer idle lanes in the last CTA
+    // (300 points fill 384 slots, not 1,024)
+    const int g = (na + 255) / 256;
+    k_fill_far<<<g, 256, 0, st>>>(out, na);
+    unsigned* bits = reinterpret_cast<unsigned*>(out);
+    cudaError_t e = with_dim(dim, [&](auto D) {
+        constexpr int DIM = decltype(D)::value;
+        return (na <= 4096) ? min_dist_grid<DIM, 128, 1>(A, na, B, nb, bits, st)
+                            : min_dist_grid<DIM, 256, 4>(A, na, B, nb, bits, st);
     });
+    if (e != cudaSuccess) return e;
+    k_sqrt<<<g, 256, 0, st>>>(out, na);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_axis_dist(int dim, const float* T, int n, float* out, cudaStream_t st)

@@ -62,3 +62,14 @@ def test_quality_of_gpu_ridge_equals_reference_quality(rdb):
     want = np.array(O.quality(S_ref, ideal, "stats"), np.float32)
     assert np.array_equal(got, want)
     assert np.float32(rdb.hausdorff(S, ideal)) == np.float32(O.quality(S_ref, ideal, "hausdorff"))
+
+
+@pytest.mark.parametrize("n,ni", [(1, 1), (1, 129), (128, 127), (129, 4097), (4096, 1025), (4097, 3),
+                                  (300, 80_000)])
+def test_min_distance_slices(rdb, n, ni):
+    """Around the points per CTA and the slices of the other set."""
+    r = np.random.default_rng(n + ni)
+    T, I = r.normal(size=(n, 3)).astype(np.float32), r.normal(size=(ni, 3)).astype(np.float32)
+    assert np.float32(rdb.hausdorff(T, I)) == np.float32(O.quality(T, I, "hausdorff"))
+    got = np.array(rdb.distance_stats(T, I), np.float32)
+    assert np.array_equal(got, np.array(O.quality(T, I, "stats"), np.float32))
