@@ -80,32 +80,168 @@ struct ActiveList {
 // Blocks of BLOCK points are visited in order.  Phase 1 (all threads) drops
 // every point that has a chosen point within r1 among those chosen by earlier
 // blocks, looked up through a hashed grid of cell edge > r1 (the grid only
-// prunes; the test itself is the exact FP32 one).  Phase 2 (warp 0) walks the
-// survivors in order and re-tests each against the grid, which by then also
-// holds the points chosen earlier in the same block, so the outcome is the
-// sequential greedy one.  Chosen coordinates and hash chains are mirrored in
-// shared memory for the first SCAP chosen points.
+// prunes; the test itself is the exact FP32 one).  Phase 2 applies the greedy
+// rule to the block's survivors (choose_survivors).  Chosen coordinates and
+// hash chains are mirrored in shared memory for the first SCAP chosen points.
 // ---------------------------------------------------------------------------
 template <int DIM>
 struct ChooseSmem {
     static constexpr int HBITS = 13;
     static constexpr int HB = 1 << HBITS;
     static constexpr int SCAP = (DIM <= 2) ? 6144 : 4096;
+    static constexpr int BLOCK = 1024;
+};
+constexpr int CHOOSE_G = 128;             // survivors resolved together
+constexpr int CHOOSE_GW = CHOOSE_G / 32;  // words of a conflict row
+
+// Scratch of choose_survivors: the conflict rows of a group, its picks, and the
+// warp counts of the compaction.
+struct ChooseResolve {
+    uint32_t adj[CHOOSE_G * CHOOSE_GW];
+    int pick[CHOOSE_G];
+    int npick;
+    int wsum[32];
 };
 
-template <int DIM, int BLOCK>
-__global__ void __launch_bounds__(BLOCK) k_choose(EngineView v)
+template <int DIM, class CS>
+constexpr int choose_smem_bytes()
 {
-    using CS = ChooseSmem<DIM>;
+    return CS::HB * 4 + CS::SCAP * 4 + CS::SCAP * DIM * 4 + CS::BLOCK * DIM * 8;
+}
+
+// The sequential greedy rule over the block's survivors s_sp[0..tot) (in
+// visiting order, none within r1 of a point chosen before the block), for the
+// whole CTA: returns the new chosen count.  A survivor is chosen when no
+// earlier chosen one lies within r1, and "within r1" among the survivors does
+// not depend on what is chosen: the first CHOOSE_G survivors write that
+// relation down as bit rows (all threads), one warp walks the group's alive
+// bits -- take the lowest, clear its row -- and the rest of the survivors drop
+// those within r1 of the group's picks and close up, in order, before the next
+// group.  Bound by the walk, about 50 ns per chosen point, and by five barriers
+// per group; a grid lookup by one warp per survivor, chosen or not, took
+// 0.25-0.4 us (first 4,096 points of the 1M helix: 436 us before,
+// 105 us now; 1,000 points of the 2D sine: 262 us before, 20 now).
+template <int DIM, class CS>
+__device__ int choose_survivors(int tot, int ns, const float rsq, float* s_sp, int32_t* s_scell,
+                                int32_t* s_heads, int32_t* s_next, float* s_S, float* gS,
+                                int32_t* gnext, const bool mirror, ChooseResolve& cr)
+{
+    constexpr int BLOCK = CS::BLOCK;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    while (tot > 0) {
+        const int m = min(CHOOSE_G, tot);
+        // conflict rows: a warp shares the word (its points j are broadcast
+        // reads) and takes consecutive rows i
+        for (int t = tid; t < CHOOSE_G * CHOOSE_GW; t += BLOCK) {
+            const int i = t % CHOOSE_G, w = t / CHOOSE_G;
+            uint32_t row = 0;
+            if (i < m && w * 32 + 31 > i) {
+                float p[DIM];
+#pragma unroll
+                for (int d = 0; d < DIM; ++d) p[d] = s_sp[i * DIM + d];
+                const int j1 = min(m - w * 32, 32);
+                for (int b = 0; b < j1; ++b) {
+                    const int j = w * 32 + b;
+                    if (sqdist_exact<DIM>(s_sp + j * DIM, p) <= rsq) row |= 1u << b;
+                }
+                // later points only
+                if (w * 32 <= i) row &= ~((2u << (i - w * 32)) - 1u);
+            }
+            cr.adj[i * CHOOSE_GW + w] = row;
+        }
+        __syncthreads();
+        if (warp == 0) {
+            uint32_t alive = 0;
+            if (lane < CHOOSE_GW) {
+                const int left = m - lane * 32;
+                alive = left >= 32 ? 0xffffffffu : (left > 0 ? (1u << left) - 1u : 0u);
+            }
+            int k = 0;
+            for (;;) {
+                const unsigned any = __ballot_sync(FULL, alive != 0);
+                if (!any) break;
+                const int l = __ffs(any) - 1;
+                const int i = l * 32 + __ffs(__shfl_sync(FULL, alive, l)) - 1;
+                if (lane == 0) cr.pick[k] = i;
+                ++k;
+                if (lane == l) alive &= alive - 1;
+                if (lane < CHOOSE_GW) alive &= ~cr.adj[i * CHOOSE_GW + lane];
+            }
+            if (lane == 0) cr.npick = k;
+        }
+        __syncthreads();
+        const int k = cr.npick;
+        for (int r = tid; r < k; r += BLOCK) {
+            const int i = cr.pick[r], q = ns + r;
+            const uint32_t b = cell_hash<DIM>(s_scell + i * DIM) & (uint32_t)(CS::HB - 1);
+            const int head = atomicExch(&s_heads[b], q);   // any order inside a bucket
+#pragma unroll
+            for (int d = 0; d < DIM; ++d) {
+                const float x = s_sp[i * DIM + d];
+                gS[(int64_t)q * DIM + d] = x;
+                if (q < CS::SCAP) s_S[q * DIM + d] = x;
+            }
+            if (q < CS::SCAP) s_next[q] = head;
+            if (mirror || q >= CS::SCAP) gnext[q] = head;
+        }
+        __syncthreads();
+        // the rest: one survivor per thread (tot <= BLOCK)
+        const int j = m + tid;
+        bool surv = j < tot;
+        float p[DIM];
+        int cc[DIM];
+        if (surv) {
+#pragma unroll
+            for (int d = 0; d < DIM; ++d) {
+                p[d] = s_sp[j * DIM + d];
+                cc[d] = s_scell[j * DIM + d];
+            }
+            for (int q = ns; q < ns + k && surv; ++q) {
+                float s[DIM];
+#pragma unroll
+                for (int d = 0; d < DIM; ++d)
+                    s[d] = (q < CS::SCAP) ? s_S[q * DIM + d] : gS[(int64_t)q * DIM + d];
+                surv = !(sqdist_exact<DIM>(p, s) <= rsq);
+            }
+        }
+        const unsigned bal = __ballot_sync(FULL, surv);
+        if (lane == 0) cr.wsum[warp] = __popc(bal);
+        __syncthreads();
+        int pos = __popc(bal & lanemask_lt()), left = 0;
+#pragma unroll
+        for (int w = 0; w < BLOCK / 32; ++w) {
+            const int x = cr.wsum[w];
+            pos += (w < warp) ? x : 0;
+            left += x;
+        }
+        if (surv) {
+#pragma unroll
+            for (int d = 0; d < DIM; ++d) {
+                s_sp[pos * DIM + d] = p[d];
+                s_scell[pos * DIM + d] = cc[d];
+            }
+        }
+        ns += k;
+        tot = left;
+        __syncthreads();
+    }
+    return ns;
+}
+
+template <int DIM, class CS>
+__global__ void __launch_bounds__(CS::BLOCK) k_choose(EngineView v)
+{
+    constexpr int BLOCK = CS::BLOCK;
     constexpr int NB = Pow3<DIM>::v;
+    __shared__ ChooseResolve s_cr;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     int32_t* s_heads = reinterpret_cast<int32_t*>(smem_raw);          // HB
     int32_t* s_next = s_heads + CS::HB;                                // SCAP
     float* s_S = reinterpret_cast<float*>(s_next + CS::SCAP);          // SCAP*DIM
     float* s_sp = s_S + CS::SCAP * DIM;                                // BLOCK*DIM
     int32_t* s_scell = reinterpret_cast<int32_t*>(s_sp + BLOCK * DIM); // BLOCK*DIM
-    __shared__ int s_ns;
     __shared__ int s_wsum[BLOCK / 32];
+    int ns = 0;   // the same in every thread
 
     const int c = blockIdx.x;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -119,7 +255,6 @@ __global__ void __launch_bounds__(BLOCK) k_choose(EngineView v)
     const float* P = v.P + cd.p_off * DIM;
 
     for (int h = tid; h < CS::HB; h += BLOCK) s_heads[h] = -1;
-    if (tid == 0) s_ns = 0;
     __syncthreads();
 
     auto coord = [&](int q, int d) -> float {
@@ -176,45 +311,12 @@ __global__ void __launch_bounds__(BLOCK) k_choose(EngineView v)
             }
         }
         __syncthreads();
-        if (warp == 0) {
-            int ns = s_ns;
-            for (int sidx = 0; sidx < tot; ++sidx) {
-                float ps[DIM];
-                int cs[DIM];
-#pragma unroll
-                for (int d = 0; d < DIM; ++d) {
-                    ps[d] = s_sp[sidx * DIM + d];
-                    cs[d] = s_scell[sidx * DIM + d];
-                }
-                bool hit = false;
-                for (int o = lane; o < NB; o += 32) hit = hit || query(ps, cs, o);
-                hit = __any_sync(FULL, hit);
-                if (!hit) {
-                    if (lane == 0) {
-                        const uint32_t b = cell_hash<DIM>(cs) & hmask;
-                        const int head = s_heads[b];
-#pragma unroll
-                        for (int d = 0; d < DIM; ++d) gS[(int64_t)ns * DIM + d] = ps[d];
-                        if (ns < CS::SCAP) {
-#pragma unroll
-                            for (int d = 0; d < DIM; ++d) s_S[ns * DIM + d] = ps[d];
-                            s_next[ns] = head;
-                        } else {
-                            gnext[ns] = head;
-                        }
-                        s_heads[b] = ns;
-                    }
-                    ++ns;
-                }
-                __syncwarp();
-            }
-            if (lane == 0) s_ns = ns;
-        }
-        __syncthreads();
+        ns = choose_survivors<DIM, CS>(tot, ns, rsq, s_sp, s_scell, s_heads, s_next, s_S, gS, gnext,
+                                       false, s_cr);
     }
     if (tid == 0) {
-        v.ns[c] = s_ns;
-        v.phase[c] = (s_ns > 0) ? PH_EVOLVE : PH_DONE;
+        v.ns[c] = ns;
+        v.phase[c] = (ns > 0) ? PH_EVOLVE : PH_DONE;
     }
 }
 
@@ -268,15 +370,16 @@ __global__ void __launch_bounds__(256) k_choose_filter(EngineView v, int c, int 
 // round, where every point of the range is a candidate).  The candidates are
 // taken in blocks of BLOCK as k_choose takes its points: all threads load
 // their candidates, compute their cells and drop those within r1 of a point
-// chosen so far (earlier rounds and earlier blocks of this one); warp 0 then
-// walks the block's survivors in order, from shared memory.
-template <int DIM, int BLOCK>
-__global__ void __launch_bounds__(BLOCK) k_choose_resolve(EngineView v, int c, int a, int b,
+// chosen so far (earlier rounds and earlier blocks of this one); choose_survivors
+// then applies the greedy rule to the block's survivors.
+template <int DIM, class CS>
+__global__ void __launch_bounds__(CS::BLOCK) k_choose_resolve(EngineView v, int c, int a, int b,
                                                           const int32_t* __restrict__ sel,
                                                           const int32_t* __restrict__ nsel,
                                                           int first)
 {
-    using CS = ChooseSmem<DIM>;
+    constexpr int BLOCK = CS::BLOCK;
+    __shared__ ChooseResolve s_cr;
     constexpr int NB = Pow3<DIM>::v;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     int32_t* s_heads = reinterpret_cast<int32_t*>(smem_raw);          // HB
@@ -284,7 +387,6 @@ __global__ void __launch_bounds__(BLOCK) k_choose_resolve(EngineView v, int c, i
     float* s_S = reinterpret_cast<float*>(s_next + CS::SCAP);          // SCAP*DIM
     float* s_sp = s_S + CS::SCAP * DIM;                                // BLOCK*DIM
     int32_t* s_scell = reinterpret_cast<int32_t*>(s_sp + BLOCK * DIM); // BLOCK*DIM
-    __shared__ int s_ns;
     __shared__ int s_wsum[BLOCK / 32];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const CloudDesc cd = v.cl[c];
@@ -301,7 +403,7 @@ __global__ void __launch_bounds__(BLOCK) k_choose_resolve(EngineView v, int c, i
 #pragma unroll
         for (int d = 0; d < DIM; ++d) s_S[q * DIM + d] = gS[(int64_t)q * DIM + d];
     }
-    if (tid == 0) s_ns = ns0;
+    int ns = ns0;   // the same in every thread
     __syncthreads();
     auto coord = [&](int q, int d) -> float {
         return (q < CS::SCAP) ? s_S[q * DIM + d] : gS[(int64_t)q * DIM + d];
@@ -357,45 +459,13 @@ __global__ void __launch_bounds__(BLOCK) k_choose_resolve(EngineView v, int c, i
             }
         }
         __syncthreads();
-        if (warp == 0) {
-            int ns = s_ns;
-            for (int sidx = 0; sidx < tot; ++sidx) {
-                float ps[DIM];
-                int cs[DIM];
-#pragma unroll
-                for (int d = 0; d < DIM; ++d) {
-                    ps[d] = s_sp[sidx * DIM + d];
-                    cs[d] = s_scell[sidx * DIM + d];
-                }
-                bool hit = false;
-                for (int o = lane; o < NB; o += 32) hit = hit || query(ps, cs, o);
-                hit = __any_sync(FULL, hit);
-                if (!hit) {
-                    if (lane == 0) {
-                        const uint32_t hb = cell_hash<DIM>(cs) & hmask;
-                        const int head = s_heads[hb];
-#pragma unroll
-                        for (int d = 0; d < DIM; ++d) gS[(int64_t)ns * DIM + d] = ps[d];
-                        gnext[ns] = head;
-                        if (ns < CS::SCAP) {
-#pragma unroll
-                            for (int d = 0; d < DIM; ++d) s_S[ns * DIM + d] = ps[d];
-                            s_next[ns] = head;
-                        }
-                        s_heads[hb] = ns;
-                    }
-                    ++ns;
-                }
-                __syncwarp();
-            }
-            if (lane == 0) s_ns = ns;
-        }
-        __syncthreads();
+        ns = choose_survivors<DIM, CS>(tot, ns, rsq, s_sp, s_scell, s_heads, s_next, s_S, gS, gnext,
+                                       true, s_cr);
     }
     for (int h = tid; h < CS::HB; h += BLOCK) v.hash[h] = s_heads[h];
     if (tid == 0) {
-        v.ns[c] = s_ns;
-        v.phase[c] = (s_ns > 0) ? PH_EVOLVE : PH_DONE;
+        v.ns[c] = ns;
+        v.phase[c] = (ns > 0) ? PH_EVOLVE : PH_DONE;
     }
 }
 
@@ -2564,25 +2634,28 @@ template <int DIM>
 cudaError_t launch_choose_dim(const EngineView& v, cudaStream_t st)
 {
     using CS = ChooseSmem<DIM>;
-    constexpr int B = 1024;
-    const int bytes = CS::HB * 4 + CS::SCAP * 4 + CS::SCAP * DIM * 4 + B * DIM * 8;
+    constexpr int bytes = choose_smem_bytes<DIM, CS>();
     cudaError_t e =
-        cudaFuncSetAttribute(k_choose<DIM, B>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+        cudaFuncSetAttribute(k_choose<DIM, CS>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (e != cudaSuccess) return e;
-    k_choose<DIM, B><<<v.n_clouds, B, bytes, st>>>(v);
+    k_choose<DIM, CS><<<v.n_clouds, CS::BLOCK, bytes, st>>>(v);
     return cudaGetLastError();
 }
 
-// rounds over [0, n): 4096 points first, doubling; needs v.hash (HB ints) and
-// surv (n bytes)
+// rounds over [0, n): 4096 points first, then four times as many each; needs
+// v.hash (HB ints) and surv (n bytes).  The points a round leaves to the one-CTA
+// resolve are those no earlier round covers, few after the first rounds, so
+// the number of rounds (a filter, a compaction and a resolve each, 50-80 us) is
+// what counts: growing four-fold instead of two-fold takes five instead of
+// eight on 1M points.
 template <int DIM>
 cudaError_t launch_choose_rounds_dim(const EngineView& v, int c, int n, uint8_t* surv,
                                      int32_t* sel, void* tmp, size_t tmp_bytes, cudaStream_t st)
 {
     using CS = ChooseSmem<DIM>;
-    constexpr int B = 1024;
-    const int bytes = CS::HB * 4 + CS::SCAP * 4 + CS::SCAP * DIM * 4 + B * DIM * 8;
-    cudaError_t e = cudaFuncSetAttribute(k_choose_resolve<DIM, B>,
+    constexpr int B = CS::BLOCK;
+    constexpr int bytes = choose_smem_bytes<DIM, CS>();
+    cudaError_t e = cudaFuncSetAttribute(k_choose_resolve<DIM, CS>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (e != cudaSuccess) return e;
     int a = 0, size = 4096, first = 1;
@@ -2590,7 +2663,7 @@ cudaError_t launch_choose_rounds_dim(const EngineView& v, int c, int n, uint8_t*
     while (a < n) {
         const int b = (int)std::min<int64_t>((int64_t)n, (int64_t)a + size);
         if (first) {
-            k_choose_resolve<DIM, B><<<1, B, bytes, st>>>(v, c, a, b, nullptr, nullptr, first);
+            k_choose_resolve<DIM, CS><<<1, B, bytes, st>>>(v, c, a, b, nullptr, nullptr, first);
         } else {
             const int grid = std::max(1, std::min((b - a + 255) / 256, 148 * 16));
             k_choose_filter<DIM><<<grid, 256, 0, st>>>(v, c, a, b, surv);
@@ -2598,10 +2671,10 @@ cudaError_t launch_choose_rounds_dim(const EngineView& v, int c, int n, uint8_t*
             e = cub::DeviceSelect::Flagged(tmp, tb, cub::CountingInputIterator<int32_t>(a), surv, sel,
                                            nsel, b - a, st);
             if (e != cudaSuccess) return e;
-            k_choose_resolve<DIM, B><<<1, B, bytes, st>>>(v, c, a, b, sel, nsel, first);
+            k_choose_resolve<DIM, CS><<<1, B, bytes, st>>>(v, c, a, b, sel, nsel, first);
         }
         a = b;
-        size = (int)std::min<int64_t>((int64_t)size * 2, 1 << 30);
+        size = (int)std::min<int64_t>((int64_t)size * 4, 1 << 30);
         first = 0;
     }
     return cudaGetLastError();
