@@ -177,6 +177,13 @@ static cudaError_t upload(DevBuf& b, const std::vector<T>& h, cudaStream_t st)
     return cudaMemcpyAsync(b.p, h.data(), sizeof(T) * h.size(), cudaMemcpyHostToDevice, st);
 }
 
+// n zero bytes (nothing to do while only sizes are planned)
+static cudaError_t upload_zero(DevBuf& b, size_t n, cudaStream_t st)
+{
+    if (DevArena* a = current_arena(); a && a->measuring()) return cudaSuccess;
+    return cudaMemsetAsync(b.p, 0, n, st);
+}
+
 int Engine::setup(int dim, const std::vector<CloudDesc>& clouds,
                   const std::vector<GroupDesc>& groups, int64_t total_points)
 {
@@ -236,12 +243,13 @@ int Engine::setup(int dim, const std::vector<CloudDesc>& clouds,
         next_off += cd.n_all;
     }
     spatial_ok_ = spatial_ok_ && next_off == total_points;
+    // list positions and edits are 31-bit, with a quarter more rows than points
+    cull_allowed_ = total_points <= (int64_t(1) << 30);
     RD_CK(bP_.ensure(sizeof(float) * (size_t)(total_points * dim + 4)));
     RD_CK(bS_.ensure(sizeof(float) * (size_t)(s_off * dim + 4)));
     RD_CK(bNext_.ensure(sizeof(int32_t) * (size_t)(s_off + 1)));
     RD_CK(bKeys_.ensure(sizeof(int32_t) * (size_t)(total_points + 1)));
     RD_CK(bGrouped_.ensure(sizeof(int32_t) * (size_t)(total_points + 4)));
-    RD_CK(bPg_.ensure(sizeof(float) * (size_t)(total_points * pad_dim(dim) + 4)));
     RD_CK(bNs_.ensure(4 * (nc + 1)));
     RD_CK(bPhase_.ensure(4 * (nc + 1)));
     RD_CK(bCont_.ensure(4 * (nc + 1)));
@@ -252,6 +260,11 @@ int Engine::setup(int dim, const std::vector<CloudDesc>& clouds,
     RD_CK(bPairs_.ensure(8 * (nc + 1)));
     RD_CK(bCtr_.ensure(4 * CTR_COUNT));
     RD_CK(bKbDone_.ensure(4 * (nc + 1)));
+    RD_CK(bFull_.ensure(4 * (nc + 1)));
+    RD_CK(bReb_.ensure(4 * (nc + 1)));
+    RD_CK(bRebNext_.ensure(4 * (nc + 1)));
+    RD_CK(bMvn_.ensure(4 * (nc + 1)));
+    RD_CK(bDmax_.ensure(4 * (nc + 1)));
     RD_CK(bActCloud_.ensure(4 * (nc + 1)));
     RD_CK(bActPre_.ensure(4 * ACT_KINDS * (nc + 1)));
     RD_CK(bGroupConv_.ensure(4 * (h_gr_.size() + 1)));
@@ -275,9 +288,21 @@ EngineView Engine::view() const
     v.perm = bGrouped_.as<int32_t>();
     v.Pg = bPg_.as<float>();
     v.hist = bHist_.as<int32_t>();
+    v.hpre = bHpre_.as<int32_t>();
     v.cnt = bCnt_.as<int32_t>();
     v.base = bBase_.as<int32_t>();
-    v.big = bBig_.as<int32_t>();
+    for (int b = 0; b < 2; ++b) {
+        // without the culled assignment the lists are regrouped in every pass
+        v.Lr[b] = cull_ ? bLr_[b].as<float>() : bPg_.as<float>();
+        v.Ls[b] = cull_ ? bLs_[b].as<int32_t>() : nullptr;
+    }
+    v.kcap = bKcap_.as<int32_t>();
+    v.par = bPar_.as<int32_t>();
+    v.edit = bEdit_.as<int32_t>();
+    v.ecnt = bEcnt_.as<int32_t>();
+    v.dlist = bDlist_.as<int32_t>();
+    v.reb = bReb_.as<int32_t>();
+    v.rebnext = bRebNext_.as<int32_t>();
     v.kbdone = bKbDone_.as<int32_t>();
     v.next = bNext_.as<int32_t>();
     v.hash = bHash_.as<int32_t>();
@@ -325,6 +350,16 @@ EngineView Engine::view() const
     v.Ps = bPs_.as<float>();
     v.sorder = bSorder_.as<int32_t>();
     v.srow = bSorder_.as<int32_t>() + total_points_;  // second half of the same buffer
+    v.ksp = bKsp_.as<int32_t>();
+    v.bbox = bBox_.as<float>();
+    v.bslack = bSlack_.as<float>();
+    v.lslack = bLslack_.as<float>();
+    v.blen = bBlen_.as<int32_t>();
+    v.blist = bBlist_.as<int32_t>();
+    v.full = bFull_.as<int32_t>();
+    v.mvn = bMvn_.as<int32_t>();
+    v.dmax = bDmax_.as<int32_t>();
+    v.mv = bMv_.as<float>();
     v.cull = cull_ ? 1 : 0;
     v.tile_order = bTileOrder_.as<int32_t>();
     v.n_heavy = n_heavy_;
@@ -353,7 +388,8 @@ int Engine::finish_setup_after_choose(cudaStream_t st)
         RD_CK(cudaMemcpyAsync(h_ns_.data(), bNs_.p, 4 * nc, cudaMemcpyDeviceToHost, st));
         RD_CK(cudaStreamSynchronize(st));
     }
-    int64_t hist = 0, key = 0, kblk = 0, kblk_warp = 0;
+    int64_t hist = 0, key = 0, kblk = 0, kblk_warp = 0, rows = 0;
+    const bool culls = cull_possible();
     int max_ns = 0;
     h_slot_cloud_.clear();
     for (size_t c = 0; c < nc; ++c) {
@@ -364,10 +400,14 @@ int Engine::finish_setup_after_choose(cudaStream_t st)
         hist += (int64_t)cd.n_chunks * cd.ns_cap;
         cd.key_off = key;
         key += cd.ns_cap;
+        // rows of the grouped lists: every key's region (list_cap in rd_kernels.cu)
+        cd.reg_off = culls ? rows : cd.p_off;
+        rows += (int64_t)cd.n_all + cd.n_all / 4 + 8 * (int64_t)cd.ns_cap;
         (cd.n_chunks > SCAN_ROWS_WARP ? kblk : kblk_warp) += (cd.ns_cap + KBLK - 1) / KBLK;
         for (int k = 0; k < cd.ns_cap; ++k) h_slot_cloud_.push_back((int32_t)c);
     }
     n_slots_ = (int32_t)key;
+    list_rows_ = rows;
     hist_ints_ = hist;
     n_kblk_ = (int32_t)kblk;
     n_kblk_warp_ = (int32_t)kblk_warp;
@@ -397,9 +437,14 @@ int Engine::finish_setup_after_choose(cudaStream_t st)
     RD_CK(upload(bDecHoff_, h_dec_hoff_, st));
     RD_CK(upload(bDecHbits_, h_dec_hbits_, st));
     RD_CK(bHist_.ensure(4 * (size_t)(hist + 1)));
+    RD_CK(bHpre_.ensure(4 * (size_t)(hist + 1)));
     RD_CK(bCnt_.ensure(4 * (size_t)(key + 1)));
     RD_CK(bBase_.ensure(4 * (size_t)(key + 1)));
-    RD_CK(bBig_.ensure(4 * (size_t)(key + 1)));
+    RD_CK(bKcap_.ensure(4 * (size_t)(key + 1)));
+    RD_CK(bPar_.ensure(4 * (size_t)(key + 1)));
+    RD_CK(bEcnt_.ensure(4 * (size_t)(key + 1)));
+    RD_CK(bDlist_.ensure(4 * (size_t)(key + 1)));
+    RD_CK(upload_zero(bEcnt_, 4 * (size_t)(key + 1), st));
     RD_CK(bDx_.ensure(4 * (size_t)(sscr * dim_ + 1)));
     RD_CK(bDcell_.ensure(4 * (size_t)(sscr * dim_ + 1)));
     RD_CK(bDalive_.ensure(4 * (size_t)(sscr + 1)));
@@ -529,18 +574,18 @@ int Engine::run(cudaStream_t st, bool use_graph, int mode)
     for (const CloudDesc& cd : h_cl_) max_ns = std::max(max_ns, cd.ns_cap);
     fused_ = fuse_tiles && h_gr_.size() == 1 && h_cl_.size() > 1 && max_ns <= TILE_NS_MAX &&
              flags_ == 0;
-    cull_ = cull_assign && assign_cull_enabled() && !fused_ && spatial_ok_ && total_points_ > 0;
+    cull_ = cull_possible() && !fused_;
     if (cull_) {
-        const size_t scratch = spatial_prep_scratch_bytes(total_points_);
-        RD_CK(bPs_.ensure(sizeof(float) * (size_t)(total_points_ * pad_dim(dim_) + 4)));
-        RD_CK(bSorder_.ensure(sizeof(int32_t) * (size_t)(2 * total_points_ + 1)));
-        RD_CK(bSpatialTmp_.ensure(scratch));
+        if (int rc = ensure_cull_buffers()) return rc;
         const EngineView vs = view();
-        RD_CK(launch_spatial_prep(dim_, vs, total_points_, bSpatialTmp_.p, scratch, bPs_.as<float>(),
-                                  bSorder_.as<int32_t>(), st));
-        // the culled assignment adds its counts into the histogram rows, which
-        // k_scatter_cta zeroes again after every pass
+        RD_CK(launch_spatial_prep(dim_, vs, tune.cull_items, total_points_, bSpatialTmp_.p,
+                                  spatial_prep_scratch_bytes(total_points_), bPs_.as<float>(),
+                                  bSorder_.as<int32_t>(), bBox_.as<float>(), st));
+        // no point has a key yet: the culled assignment keeps the counts by its
+        // changes
         RD_CK(cudaMemsetAsync(bHist_.p, 0, 4 * (size_t)(hist_ints_ + 1), st));
+    } else {
+        RD_CK(bPg_.ensure(sizeof(float) * (size_t)(total_points_ * pad_dim(dim_) + 4)));
     }
     tile_cl_grid_ = 0;
     if (fused_) RD_CK(prepare_tile_pass(dim_, view(), &tile_cl_grid_));
@@ -585,6 +630,35 @@ int Engine::run(cudaStream_t st, bool use_graph, int mode)
     return collect(st);
 }
 
+// whether the lockstep passes of this batch assign with culling
+bool Engine::cull_possible() const
+{
+    return cull_assign && cull_allowed_ && assign_cull_enabled() && spatial_ok_ && total_points_ > 0;
+}
+
+// buffers of the culled assignment (sizes known after choose)
+int Engine::ensure_cull_buffers()
+{
+    const size_t n = (size_t)total_points_;
+    const size_t blocks = (size_t)n_chunks_ * (chunk_pts_ / (32 * tune.cull_items));
+    RD_CK(bPs_.ensure(sizeof(float) * (n * pad_dim(dim_) + 4)));
+    RD_CK(bSorder_.ensure(sizeof(int32_t) * (2 * n + 1)));
+    RD_CK(bSpatialTmp_.ensure(spatial_prep_scratch_bytes(total_points_)));
+    RD_CK(bKsp_.ensure(sizeof(int32_t) * (n + 1)));
+    RD_CK(bBox_.ensure(sizeof(float) * (4 * dim_ * blocks + 1)));
+    RD_CK(bSlack_.ensure(sizeof(float) * (blocks + 1)));
+    RD_CK(bLslack_.ensure(sizeof(float) * (blocks + 1)));
+    RD_CK(bBlen_.ensure(sizeof(int32_t) * (blocks + 1)));
+    RD_CK(bBlist_.ensure(sizeof(int32_t) * (32 * blocks + 1)));
+    for (int b = 0; b < 2; ++b) {
+        RD_CK(bLr_[b].ensure(sizeof(float) * ((size_t)list_rows_ * pad_dim(dim_) + 4)));
+        RD_CK(bLs_[b].ensure(sizeof(int32_t) * ((size_t)list_rows_ + 1)));
+    }
+    RD_CK(bEdit_.ensure(sizeof(int32_t) * ((size_t)list_rows_ + 1)));
+    RD_CK(bMv_.ensure(sizeof(float) * ((size_t)(2 * dim_ + 1) * n_slots_ + 1)));
+    return 0;
+}
+
 // Tiles (clouds) by decreasing evolve points; the heavy ones (evolved by a
 // whole cluster in fused tiled runs) first.
 void Engine::build_tile_order()
@@ -617,11 +691,12 @@ int Engine::plan_workspace(int mode)
     RD_CK(upload(bTileOrder_, h_tile_order_, nullptr));
     if (mode == RUN_EVOLVE_ONLY || mode == RUN_DECIMATE_ONLY) {
         if (int rc = finish_setup_after_choose(nullptr)) return rc;
-        if (mode == RUN_EVOLVE_ONLY && cull_assign && assign_cull_enabled() && spatial_ok_ &&
-            total_points_ > 0) {
-            RD_CK(bPs_.ensure(sizeof(float) * (size_t)(total_points_ * pad_dim(dim_) + 4)));
-            RD_CK(bSorder_.ensure(sizeof(int32_t) * (size_t)(2 * total_points_ + 1)));
-            RD_CK(bSpatialTmp_.ensure(spatial_prep_scratch_bytes(total_points_)));
+        if (mode == RUN_EVOLVE_ONLY) {
+            if (cull_possible()) {
+                if (int rc = ensure_cull_buffers()) return rc;
+            } else {
+                RD_CK(bPg_.ensure(sizeof(float) * (size_t)(total_points_ * pad_dim(dim_) + 4)));
+            }
         }
         return 0;
     }
@@ -651,6 +726,8 @@ int Engine::adjoint_setup(cudaStream_t st)
     stats_ = RunStats();
     flags_ = ENG_ALWAYS_MOVE;
     cull_ = false;
+    cull_allowed_ = false;
+    RD_CK(bPg_.ensure(sizeof(float) * (size_t)(total_points_ * pad_dim(dim_) + 4)));
     RD_CK(upload(bCl_, h_cl_, st));
     RD_CK(upload(bGr_, h_gr_, st));
     EngineView v0 = view();

@@ -54,13 +54,14 @@ enum : int {
     CTR_ERR = 3,       // OR of global error bits
     CTR_NACT = 4,      // evolving clouds in the current work lists
     CTR_NREADY = 5,    // groups ready for decimation in this iteration
-    CTR_NBIG = 6,      // keys in the big-key list of the current pass
+    CTR_NDIRTY = 6,    // keys listed for folding in the current pass
     CTR_TILE_HEAVY = 7,// heavy-tile ticket of the cluster tile kernel
-    CTR_SUM_DONE = 8,  // CTAs of k_sum_shift finished (the last one runs the control step)
+    CTR_SUM_DONE = 8,  // CTAs of k_merge_fold finished (the last one runs the control step)
     CTR_DEC_DONE = 9,  // CTAs of k_decimate finished (the last one sets the loop condition)
     CTR_DEC_PASSES = 10,  // decimation passes resolved in parallel rounds (this run)
     CTR_DEC_ROUNDS = 11,  // rounds they took
-    CTR_COUNT = 12,
+    CTR_COND_DONE = 12,   // k_merge_fold ended this iteration (no group was ready)
+    CTR_COUNT = 13,
 };
 
 struct EngineView {
@@ -74,11 +75,23 @@ struct EngineView {
     int32_t* perm;               // per point slot: point indices grouped by key, index order
                                  // (tiled kernels)
     float* Pg;                   // per point slot: the points' coordinates grouped by key in
-                                 // index order, PadDim floats each (lockstep passes)
-    int32_t* hist;               // per cloud: n_chunks x ns_cap key histogram (then its prefix over chunks)
+                                 // index order, PadDim floats each (tiled kernels)
+    // lockstep passes: each key's members in index order, in its region
+    // [base, base + kcap) of its cloud's part (reg_off) of two buffers; the
+    // current list is in buffer par
+    float* Lr[2];                // coordinates, PadDim floats per row
+    int32_t* Ls[2];              // the points' positions in their cloud (culled assignment only)
+    int32_t* kcap;               // per chosen slot: rows of its region
+    int32_t* par;                // per chosen slot: buffer of its current list
+    int32_t* edit;               // per row: edits of this pass, at the key's region
+    int32_t* ecnt;               // per chosen slot: edits of this pass
+    int32_t* dlist;              // chosen slots to fold in this pass
+    int32_t* reb;                // per cloud: regroup all points in this pass
+    int32_t* rebnext;            // per cloud: and in the next one
+    int32_t* hist;               // per cloud: n_chunks x ns_cap key histogram
+    int32_t* hpre;               // the same shape: its exclusive prefix over the chunks
     int32_t* cnt;                // per chosen slot: members in the last pass
-    int32_t* base;               // per chosen slot: first slot of its segment of perm
-    int32_t* big;                // chosen slots with SUM_BIG_MIN+ members in this pass
+    int32_t* base;               // per chosen slot: first row of its region
     int32_t* kbdone;             // per cloud: key blocks of the chunk scan finished in this pass
     int32_t* hash;               // choose hash heads
     int32_t* next;               // per chosen slot: choose hash chain
@@ -130,7 +143,18 @@ struct EngineView {
     const float* Ps;             // evolve points in spatial order inside each cloud
     const int32_t* sorder;       // spatial position -> packed point slot
     const int32_t* srow;         // spatial position -> its slot's chunk in the cloud (histogram row)
-    int32_t cull;                // passes assign with k_assign_cull + k_keyhist
+    int32_t* ksp;                // spatial position -> its point's key (as keys holds it by slot)
+    const float* bbox;           // per block of 32 x cull_items spatial positions: two boxes (lo, hi)
+    float* bslack;               // per block: moves that leave its keys as they are (see k_assign_cull)
+    float* lslack;               // per block: moves that leave its candidate list complete
+    int32_t* blen;               // per block: entries of its candidate list
+    int32_t* blist;              // per block: the list (32 entries)
+    int32_t* full;               // per cloud: the next pass evaluates every block and every key
+    int32_t* mvn;                // per cloud: chosen points moved in the last pass
+    int32_t* dmax;               // per cloud: bits of the longest of those moves
+    float* mv;                   // 2*DIM+1 arrays of n_slots: each cloud's moves at its key_off
+                                 // (old place, new place, length rounded up)
+    int32_t cull;                // passes assign with k_assign_cull
     // fused tiled runs: tiles by decreasing evolve points, the first n_heavy
     // evolved by whole thread-block clusters (rd_tile_cluster.cuh)
     const int32_t* tile_order;
@@ -227,8 +251,11 @@ cudaError_t launch_ordered_sum(int dim, const float* P, const int32_t* idx, int 
 // contiguous clouds in cloud order and n_points < 2^31; scratch of
 // spatial_prep_scratch_bytes(n).
 size_t spatial_prep_scratch_bytes(int64_t n_points);
-cudaError_t launch_spatial_prep(int dim, const EngineView& v, int64_t n_points, void* scratch,
-                                size_t scratch_bytes, float* Ps, int32_t* sorder, cudaStream_t st);
+// Also writes the boxes of the blocks of 32 x items positions and clears keys
+// and ksp.
+cudaError_t launch_spatial_prep(int dim, const EngineView& v, int items, int64_t n_points,
+                                void* scratch, size_t scratch_bytes, float* Ps, int32_t* sorder,
+                                float* bbox, cudaStream_t st);
 // the five kernels of one evolve pass without control/decimation (adjoint forward)
 cudaError_t launch_evolve_step(int dim, const EngineView& v, const TuneParams& tp, int assign_grid,
                                cudaStream_t st);

@@ -146,6 +146,8 @@ public:
 
 private:
     int finish_setup_after_choose(cudaStream_t st);
+    bool cull_possible() const;
+    int ensure_cull_buffers();
     void build_tile_order();
     int collect(cudaStream_t st);
     int flags_ = 0;
@@ -170,7 +172,7 @@ private:
     RunStats stats_;
 
     DevBuf bCl_, bGr_, bChunkCloud_, bSlotCloud_;
-    DevBuf bP_, bS_, bKeys_, bGrouped_, bPg_, bHist_, bCnt_, bBase_, bBig_, bNext_, bHash_, bSurv_;
+    DevBuf bP_, bS_, bKeys_, bGrouped_, bPg_, bHist_, bCnt_, bBase_, bNext_, bHash_, bSurv_;
     DevBuf bNs_, bPhase_, bCont_, bPasses_, bTotPasses_, bOuter_, bErr_, bPairs_, bCtr_, bKbDone_;
     DevBuf bActCloud_, bActPre_, bGroupConv_, bReady_, bDnbOff_, bDnb_, bDbig_, bDcpre_;
     int dec_smem_max_ = 0;
@@ -178,7 +180,11 @@ private:
     bool fused_ = false;
     bool cull_ = false;           // this run assigns with culling
     bool spatial_ok_ = false;     // the batch layout allows the spatial order
-    DevBuf bPs_, bSorder_, bSpatialTmp_;
+    bool cull_allowed_ = true;    // and its size, and the kind of run, the culled assignment
+    int64_t list_rows_ = 0;       // rows of the grouped lists of the culled assignment
+    DevBuf bLr_[2], bLs_[2], bKcap_, bPar_, bEdit_, bEcnt_, bDlist_, bReb_, bRebNext_;
+    DevBuf bPs_, bSorder_, bSpatialTmp_, bHpre_;
+    DevBuf bKsp_, bBox_, bSlack_, bLslack_, bBlen_, bBlist_,  bFull_, bMvn_, bDmax_, bMv_;
     DevBuf bTileOrder_;
     DevBuf bSel_, bSelTmp_;       // GPU-wide choose: survivor list and its compaction scratch
     std::vector<int32_t> h_tile_order_;

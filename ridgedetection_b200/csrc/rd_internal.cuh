@@ -76,9 +76,7 @@ struct CloudDesc {
     int64_t hist_off;    // start of this cloud's chunk x key histogram (set after choose)
     int32_t ns_cap;      // chosen count right after choose (hist row length)
     int64_t key_off;     // start of this cloud's per-chosen arrays (cnt/base)
-    int64_t hash_off;    // start of this cloud's choose hash heads
-    int32_t hash_bits;   // log2 of the number of hash buckets
-    int32_t pad;
+    int64_t reg_off;     // first row of this cloud's part of the grouped lists (set after choose)
 };
 
 struct GroupDesc {

@@ -23,13 +23,11 @@ namespace rdb {
 
 namespace {
 
-// members from which a key is folded by a whole CTA of k_sum_shift (the
-// warp-segmented exact fold of rd_segfold.cuh) instead of by one warp's add
-// chain -- while the pass has at most two such keys per big-key CTA; with more
-// (a batch of large clouds) every key is folded by a warp, which keeps all
-// SMs busy.
+// members from which a key is folded by its whole CTA (the warp-segmented exact
+// fold of rd_segfold.cuh) instead of by one warp's add chain -- while the pass
+// has no more keys to fold than CTAs; with more (a batch of large clouds) every
+// key is folded by a chain, which does less work in all.
 constexpr int SUM_BIG_MIN = 16384;
-constexpr int SUM_BIG_PER_CTA = 2;
 
 // Programmatic dependent launch: the loop-body kernels are launched with
 // programmatic stream serialisation, so a kernel's CTAs may become resident
@@ -617,38 +615,67 @@ __global__ void __launch_bounds__(BLOCK) k_assign(EngineView v)
 // ---------------------------------------------------------------------------
 // Culled assignment: the same keys as k_assign, over the spatial order (Ps,
 // built once per run by launch_spatial_prep, DIM padded to PadDim) instead of
-// the slot order.  A work item is a block of AC_BLOCK x AC_ITEMS consecutive
-// points of that order; each warp takes 32 x AC_ITEMS of them and their
-// bounding box.  A chosen point s takes part in a box's argmin only when the
-// squared gap between s and the box, g2, is at most thr = r1^2 (1 + 2^-10)
-// (rounded up).  Exactness: the computed g2 exceeds the exact squared gap G by
-// at most a relative 2^-20 (a few roundings of non-negative terms), and every
-// computed distance from s to a point of the box is at least G (1 - 2^-20);
-// so g2 > thr makes every such distance > r1^2.  A skipped chosen point can
-// then neither be the nearest one within r1 nor tie with it, and the minimum
-// over the remaining points, visited in index order with strict '<', is the
-// reference's (rd/cpu/brute_force/evolve.hpp:54-66).  The bound needs r1^2 in
-// the normal range; any other r1 disables the skip.  NaN gaps never skip.
+// the slot order, and only where a key can have changed.  A block is 32 x ITEMS
+// consecutive points of that order, one warp each, with the bounding boxes of
+// its two parts (rd_spatial.cu says where they part); "the box" below is their
+// union and the gap to it the smaller of the two.
 //
-// The test runs at two levels.  The CTA's box (the union of its warps' boxes)
-// is tested against every chosen point of the cloud, each thread taking a few
-// of them; the survivors are compacted in index order into a shared list.
-// The argument above holds for any box that contains the points, so a point
-// dropped there is dropped for every warp.  Each warp then tests the short
-// list against its own box and evaluates the distances of the kept chosen
-// points, still in index order.  The chosen points stay staged in shared
-// memory across the CTA's work items while they belong to one cloud of at
-// most AC_TS chosen points.
+// Which chosen points a block looks at.  A chosen point s takes part in a
+// block's argmin only when the squared gap between s and the box, g2, is at
+// most thr = r1^2 (1 + 2^-10) (rounded up).  Exactness: the computed g2 exceeds
+// the exact squared gap G by at most a relative 2^-20 (a few roundings of
+// non-negative terms), and every computed distance from s to a point of the box
+// is at least G (1 - 2^-20); so g2 > thr makes every such distance > r1^2.  A
+// skipped chosen point can then neither be the nearest one within r1 nor tie
+// with it, and the minimum over the remaining points, visited in index order
+// with strict '<', is the reference's (rd/cpu/brute_force/evolve.hpp:54-66).
+// The bound needs r1^2 in the normal range; any other r1 disables the skip.
+// NaN gaps never skip.
 //
-// Keys are written back to the points' slots, and each assigned point adds
-// one to its key's entry in the histogram row of its slot-order chunk (the
-// rows k_assign writes itself; k_scatter_cta zeroes them again after use).
+// Which blocks are looked at.  An evaluation leaves the block's slack: the
+// smallest margin of its points.  For a point with nearest chosen point at
+// distance d1 <= r1 and the next kept one at d2 the margin is
+// (min(d2, r1) - d1) / 2; for a point with none within r1 it is d1 - r1, at
+// most 4e-4 r1; both less 1e-5 r1 for the roundings (distances carry a relative
+// error below 2^-21).  k_merge_fold lists every chosen point it moves with its
+// old and new place and the length of the move (rounded up).  Let D be the
+// largest move, in this pass, of a chosen point within thr of the box before or
+// after it.  The slack is lowered by D (rounded down), and while it stays
+// positive no key of the block can have changed: the nearest chosen point, in
+// range of the box all along, is at most d1 + sum D away.  Any other one was,
+// when last out of range, more than r1 away, or it was kept and at least d2
+// away, and came at most sum D closer since; with the margin above both stay
+// behind the nearest one, and that one within r1.  A point with none within r1
+// stays so: kept chosen points were d1 away, others at least r1 (1 + 4.8e-4).
+// `full` clouds (first pass, after a decimation, after new chosen points)
+// evaluate every block.  A block first tries the largest move of the whole
+// cloud, one comparison, and scans the list of moves only when that does not do.
+//
+// Candidates.  A block keeps the list, in index order, of the chosen points
+// within R = r1 + r1/4 of its box (with the same 2^-10 on R^2) as its last scan
+// of the whole chosen set found them, while the moves D since then -- taken
+// over the chosen points within R of the box, which covers those within r1 --
+// add up to less than r1/4: any other chosen point is then still more than
+// r1 (1 + 4.8e-4) away.  An evaluation reads that list, at most 32 entries, one
+// per lane, instead of every chosen point; a block with more candidates keeps
+// none and scans.
+//
+// Only changed keys are written: to the points' slots, to the spatial copy
+// (ksp), as -1/+1 in the histogram row of their slot-order chunk (which so
+// always holds the current counts), and as an edit of both keys' member lists
+// (push_edit); k_merge_fold then touches the keys with edits only.  A key with
+// unchanged members keeps its sum, and its chosen point has answered the
+// movement test for that sum already (it moved to the mean, or stayed within
+// the threshold).
+//
+// 1M-point helix, 285 passes: the median pass changes 0.1% of the keys; the
+// kernel that evaluated every block, with its keys and counts written anew,
+// took 36 us per pass; this one 44 us in the first pass (candidate lists built),
+// 28-40 us while every chosen point moves, 12-25 us after.  Bound by the few
+// blocks whose candidates do not fit a list, then by instruction issue.
 // ---------------------------------------------------------------------------
 constexpr int AC_BLOCK = 256;             // threads of k_assign_cull
 constexpr int AC_WARPS = AC_BLOCK / 32;
-constexpr int AC_TS = 1024;               // chosen points per shared-memory batch
-// points per lane (AC_ITEMS, a tuning parameter): a warp's box holds 32 x
-// AC_ITEMS consecutive points of the spatial order
 
 // squared gap between s and the box [lo, hi] (0 inside; NaN-free for NaN s)
 template <int DIM>
@@ -663,248 +690,265 @@ __device__ __forceinline__ float box_gap2(const float* s, const float* lo, const
     return g2;
 }
 
-template <int DIM, int AC_ITEMS>
-__global__ void __launch_bounds__(AC_BLOCK) k_assign_cull(EngineView v)
+// the same for the nearer of a block's two boxes, b[2][lo, hi] (an empty one is
+// infinitely far; a NaN gap stays NaN, which never skips)
+template <int DIM>
+__device__ __forceinline__ float block_gap2(const float* s, const float (&b)[2][2 * DIM])
+{
+    const float g0 = box_gap2<DIM>(s, b[0], b[0] + DIM), g1 = box_gap2<DIM>(s, b[1], b[1] + DIM);
+    return (g0 > g1) ? g1 : g0;
+}
+
+// One chosen point against the block's points: nearest and second nearest.
+template <int DIM, int ITEMS>
+__device__ __forceinline__ void assign_one(const float* sk, const int k, const float2 (&np2)[ITEMS / 2][DIM],
+                                           float (&best)[ITEMS], float (&sec)[ITEMS], int (&key)[ITEMS])
+{
+#pragma unroll
+    for (int jj = 0; jj < ITEMS / 2; ++jj) {
+        const float2 dd = sqdist2_exact<DIM>(sk, np2[jj]);
+        sec[2 * jj] = fminf(sec[2 * jj], fmaxf(best[2 * jj], dd.x));
+        sec[2 * jj + 1] = fminf(sec[2 * jj + 1], fmaxf(best[2 * jj + 1], dd.y));
+        if (dd.x < best[2 * jj]) { best[2 * jj] = dd.x; key[2 * jj] = k; }
+        if (dd.y < best[2 * jj + 1]) { best[2 * jj + 1] = dd.y; key[2 * jj + 1] = k; }
+    }
+}
+
+constexpr int EDIT_IN = (int)0x80000000;   // edit of a member list: this point joins (else it leaves)
+constexpr int EDIT_MAX = 512;              // edits of one key that k_merge_fold takes
+
+// rows of a key's region of the grouped lists with n members at the rebuild:
+// room for its list to grow before the next rebuild (without the culled
+// assignment every pass rebuilds)
+__device__ __forceinline__ int list_cap(const EngineView& v, const int n)
+{
+    return v.cull ? n + (n >> 2) + 8 : n;
+}
+
+// A pass regroups all points of a cloud by key: its chosen points are new or
+// renumbered, or a key got more edits than it takes.
+__device__ __forceinline__ bool rebuilds(const EngineView& v, const int c)
+{
+    return !v.cull || v.full[c] != 0 || v.reb[c] != 0;
+}
+
+// One edit of key k's member list.  The first one of the pass lists the key as
+// work for k_merge_fold.
+__device__ __forceinline__ void push_edit(const EngineView& v, const int c, const CloudDesc& cd,
+                                          const int k, const int edit)
+{
+    const int64_t s = cd.key_off + k;
+    const int at = atomicAdd(&v.ecnt[s], 1);
+    if (at == 0) v.dlist[atomicAdd(&v.ctr[CTR_NDIRTY], 1)] = (int)s;
+    if (at < min(EDIT_MAX, v.kcap[s])) v.edit[cd.reg_off + v.base[s] + at] = edit;
+    else v.reb[c] = 1;
+}
+
+// resident CTAs the registers are held to: the evaluation waits on memory
+// (points, keys, candidates, in three dependent steps), so warps in flight
+// count; eight points per lane need the registers
+template <int DIM, int ITEMS>
+__global__ void __launch_bounds__(AC_BLOCK, ITEMS <= 4 ? 4 : 2) k_assign_cull(EngineView v)
 {
     pdl_enter();
-    static_assert(AC_ITEMS % 2 == 0, "points are evaluated in pairs");
+    static_assert(ITEMS % 2 == 0, "points are evaluated in pairs");
     constexpr int DP = PadDim<DIM>::v;
-    constexpr int WPTS = 32 * AC_ITEMS;
-    constexpr int SUBPTS = AC_BLOCK * AC_ITEMS;
-    __shared__ __align__(16) float sS[AC_TS * DP];  // staged chosen batch
-    __shared__ int sK[2][AC_TS];                     // CTA survivors: batch positions
-    __shared__ float s_box[2][AC_WARPS][2 * DIM];    // warp boxes
-    __shared__ float s_cbox[2][2 * DIM];             // the CTA's box
-    __shared__ int s_wcnt[2][AC_WARPS];              // survivors per warp range
-    __shared__ int s_staged;                         // cloud whose whole chosen set is in sS
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-
+    constexpr int WPTS = 32 * ITEMS;
+    const int lane = threadIdx.x & 31;
     const ActiveList al(v, ACT_CHUNK);
-    // Each cloud is cut into blocks of SUBPTS consecutive positions of its
-    // spatial order, `subs` blocks per assignment chunk (a power of two: both
-    // sizes are); blocks past the cloud's end are empty.  The block bounds
-    // need no division.
-    const int subs = (v.chunk_pts + SUBPTS - 1) / SUBPTS;
-    const int subs_log = 31 - __clz(subs);
-    const int total = al.total * subs;
-
-    // A work item's cloud, point range and this lane's points with their
-    // slots and histogram rows; the next item's are loaded while the current
-    // one is evaluated.
-    struct Item {
-        int c, b0, b1;
-        float p[AC_ITEMS][DIM];
-        int slot[AC_ITEMS], row[AC_ITEMS];
-    };
-    auto load_item = [&](const int item, Item& t) {
-        t.c = -1;
-        t.b0 = t.b1 = 0;
-#pragma unroll
-        for (int j = 0; j < AC_ITEMS; ++j) {
-            t.slot[j] = -1;
-            t.row[j] = 0;
-#pragma unroll
-            for (int d = 0; d < DIM; ++d) t.p[j][d] = 0.0f;
-        }
-        if (item >= total) return;
-        int lc;
-        al.locate(item >> subs_log, t.c, lc);
-        const int n_all = v.cl[t.c].n_all;
-        const int64_t p_off = v.cl[t.c].p_off;
-        t.b0 = min(n_all, ((lc << subs_log) + (item & (subs - 1))) * SUBPTS);
-        t.b1 = min(n_all, t.b0 + SUBPTS);
-        const float* Ps = v.Ps + p_off * DP;
-#pragma unroll
-        for (int j = 0; j < AC_ITEMS; ++j) {
-            const int i = t.b0 + warp * WPTS + j * 32 + lane;
-            if (i < t.b1) {
-                load_chosen<DIM>(Ps, i, t.p[j]);
-                t.slot[j] = v.sorder[p_off + i];
-                t.row[j] = v.srow[p_off + i];
+    const int wpc_log = 31 - __clz(v.chunk_pts / WPTS);   // blocks per chunk, a power of two
+    const int total = al.total << wpc_log;
+    const int nw = gridDim.x * AC_WARPS;
+    // a warp takes blocks nw apart, one per lane: the lanes find their blocks'
+    // clouds and make the one-comparison test at the same time
+    for (int64_t base = blockIdx.x * AC_WARPS + (threadIdx.x >> 5); base < total; base += (int64_t)32 * nw) {
+        const int64_t t = base + (int64_t)lane * nw;
+        int my_c = 0, my_i = 0, my_full = 0;
+        float my_slack = 0.0f;
+        bool need = false;
+        if (t < total) {
+            int lc;
+            al.locate((int)(t >> wpc_log), my_c, lc);
+            my_i = (lc << wpc_log) + ((int)t & ((1 << wpc_log) - 1));
+            if ((int64_t)my_i * WPTS < v.cl[my_c].n_all) {
+                const int64_t wb = (v.cl[my_c].chunk_begin << wpc_log) + my_i;
+                my_full = v.full[my_c];
+                const float dmax = __int_as_float(v.dmax[my_c]);
+                my_slack = v.bslack[wb];
+                need = my_full || !(my_slack > dmax);
+                if (!need && dmax > 0.0f) {
+                    v.bslack[wb] = __fsub_rd(my_slack, dmax);
+                    v.lslack[wb] = __fsub_rd(v.lslack[wb], dmax);
+                }
             }
         }
-    };
-
-    if (tid == 0) s_staged = -1;
-    // Items are dealt to the CTAs round robin (they are of equal size), so
-    // every CTA knows its next item at once: its points are loaded while the
-    // current one is evaluated.  Shared arrays indexed by `buf` alternate
-    // between items, so a warp still reading the previous item's list never
-    // races the next item's writes; sS is rewritten only after the barrier
-    // that every warp reaches once it is done with the previous item.
-    Item cur;
-    load_item(blockIdx.x, cur);
-    int it = 0;
-    for (int item = blockIdx.x; item < total; item += gridDim.x, ++it) {
-        const int buf = it & 1;
-        Item nxt;
-        load_item(item + gridDim.x, nxt);
-        const int c = cur.c;
-        const CloudDesc cd = v.cl[c];
-        const int ns = v.ns[c];
-        const float* gS = v.S + cd.s_off * DIM;
-        const float rsq = sqr_rn(cd.r1);
-        const bool may_skip = rsq >= 1.0e-30f && rsq <= 1.0e30f;
-        const float thr = __fmul_ru(rsq, 1.0009765625f);
-
-        // this warp's box (empty when the item has no points here)
-        float blo[DIM], bhi[DIM];
+        for (unsigned todo = __ballot_sync(FULL, need); todo; todo &= todo - 1) {
+            const int src = __ffs(todo) - 1;
+            const int c = __shfl_sync(FULL, my_c, src);
+            const int bi = __shfl_sync(FULL, my_i, src);
+            const int full = __shfl_sync(FULL, my_full, src);
+            const CloudDesc cd = v.cl[c];
+            const int ns = v.ns[c];
+            const int64_t wb = (cd.chunk_begin << wpc_log) + bi;
+            const float rsq = sqr_rn(cd.r1);
+            const bool may_skip = rsq >= 1.0e-30f && rsq <= 1.0e30f;
+            const float thr = __fmul_ru(rsq, 1.0009765625f);
+            float box[2][2 * DIM];
 #pragma unroll
-        for (int d = 0; d < DIM; ++d) {
-            blo[d] = INFINITY;
-            bhi[d] = -INFINITY;
-        }
+            for (int e = 0; e < 2 * DIM; ++e) {
+                box[0][e] = v.bbox[wb * 4 * DIM + e];
+                box[1][e] = v.bbox[wb * 4 * DIM + 2 * DIM + e];
+            }
+            // this lane's points and their keys (positions past the cloud: slot < 0)
+            const int pos0 = bi * WPTS + lane;
+            const float* Ps = v.Ps + cd.p_off * DP;
+            int32_t* ksp = v.ksp + cd.p_off;
+            const int m = v.mvn[c];
+            const float reach = __fadd_ru(cd.r1, 0.25f * cd.r1);
+            const float thr_list = __fmul_ru(__fmul_ru(reach, reach), 1.0009765625f);
+            float dl = __int_as_float(v.dmax[c]);
+            // a list longer than half the chosen set costs about as much as the
+            // evaluation it may save
+            if (!full && 2 * m <= ns + 64) {
+                unsigned dloc = 0;
+                const float* mv = v.mv + cd.key_off;
+                for (int j = lane; j < m; j += 32) {
+                    float o[DIM], q[DIM];
 #pragma unroll
-        for (int j = 0; j < AC_ITEMS; ++j)
-            if (cur.slot[j] >= 0)
+                    for (int d = 0; d < DIM; ++d) {
+                        o[d] = mv[(int64_t)d * v.n_slots + j];
+                        q[d] = mv[(int64_t)(DIM + d) * v.n_slots + j];
+                    }
+                    const bool out = may_skip && block_gap2<DIM>(o, box) > thr_list &&
+                                     block_gap2<DIM>(q, box) > thr_list;
+                    // lengths are not negative (or NaN): they order as their bits do
+                    if (!out) dloc = max(dloc, __float_as_uint(mv[(int64_t)(2 * DIM) * v.n_slots + j]));
+                }
+                dl = __uint_as_float(__reduce_max_sync(FULL, dloc));
+                const float slack = __shfl_sync(FULL, my_slack, src);
+                if (slack > dl) {
+                    if (lane == 0 && dl > 0.0f) {
+                        v.bslack[wb] = __fsub_rd(slack, dl);
+                        v.lslack[wb] = __fsub_rd(v.lslack[wb], dl);
+                    }
+                    continue;
+                }
+            }
+            const float list_left = full ? 0.0f : __fsub_rd(v.lslack[wb], dl);
+            const int n_list = (list_left > 0.0f) ? v.blen[wb] : -1;
+            int32_t* list = v.blist + wb * 32;
+            float2 np2[ITEMS / 2][DIM];
+            int old[ITEMS];
+#pragma unroll
+            for (int j = 0; j < ITEMS; ++j) {
+                const int i = pos0 + j * 32;
+                float p[DIM];
+#pragma unroll
+                for (int d = 0; d < DIM; ++d) p[d] = 0.0f;
+                old[j] = -1;
+                if (i < cd.n_all) {
+                    load_chosen<DIM>(Ps, i, p);
+                    old[j] = ksp[i];
+                }
 #pragma unroll
                 for (int d = 0; d < DIM; ++d) {
-                    blo[d] = fminf(blo[d], cur.p[j][d]);
-                    bhi[d] = fmaxf(bhi[d], cur.p[j][d]);
-                }
-#pragma unroll
-        for (int d = 0; d < DIM; ++d) {
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                blo[d] = fminf(blo[d], __shfl_xor_sync(FULL, blo[d], o));
-                bhi[d] = fmaxf(bhi[d], __shfl_xor_sync(FULL, bhi[d], o));
-            }
-        }
-        if (lane == 0) {
-#pragma unroll
-            for (int d = 0; d < DIM; ++d) {
-                s_box[buf][warp][d] = blo[d];
-                s_box[buf][warp][DIM + d] = bhi[d];
-            }
-        }
-        float2 np2[AC_ITEMS / 2][DIM];
-        float best[AC_ITEMS];
-        int bi[AC_ITEMS];
-#pragma unroll
-        for (int jj = 0; jj < AC_ITEMS / 2; ++jj)
-#pragma unroll
-            for (int d = 0; d < DIM; ++d)
-                np2[jj][d] = make_float2(-cur.p[2 * jj][d], -cur.p[2 * jj + 1][d]);
-#pragma unroll
-        for (int j = 0; j < AC_ITEMS; ++j) {
-            best[j] = FLT_MAX;
-            bi[j] = -1;
-        }
-        __syncthreads();  // warp boxes visible; the previous item is done
-        if (warp == 0 && lane < 2 * DIM) {
-            const bool hi = lane >= DIM;
-            float x = s_box[buf][0][lane];
-            for (int w = 1; w < AC_WARPS; ++w)
-                x = hi ? fmaxf(x, s_box[buf][w][lane]) : fminf(x, s_box[buf][w][lane]);
-            s_cbox[buf][lane] = x;
-        }
-        const bool cached = s_staged == c && ns <= AC_TS;
-        for (int t0 = 0; t0 < ns; t0 += AC_TS) {
-            const int tl = min(AC_TS, ns - t0);
-            if (!(t0 == 0 && cached)) {
-                if (t0 > 0) __syncthreads();  // the previous batch is no longer read
-                for (int e = tid; e < tl; e += AC_BLOCK) {
-                    float s[DIM];
-#pragma unroll
-                    for (int d = 0; d < DIM; ++d) s[d] = gS[(int64_t)(t0 + e) * DIM + d];
-#pragma unroll
-                    for (int d = 0; d < DIM; ++d) sS[e * DP + d] = s[d];
+                    if (j & 1) np2[j / 2][d].y = -p[d];
+                    else np2[j / 2][d].x = -p[d];
                 }
             }
-            __syncthreads();  // batch staged, CTA box known
-            if (t0 == 0 && !cached && tid == 0) s_staged = (ns <= AC_TS) ? c : -1;
-            float clo[DIM], chi[DIM];
+            float best[ITEMS], sec[ITEMS];
+            int key[ITEMS];
 #pragma unroll
-            for (int d = 0; d < DIM; ++d) {
-                clo[d] = s_cbox[buf][d];
-                chi[d] = s_cbox[buf][DIM + d];
+            for (int j = 0; j < ITEMS; ++j) {
+                best[j] = FLT_MAX;
+                sec[j] = FLT_MAX;
+                key[j] = -1;
             }
-            // CTA-level test: warp w takes batch positions [w*cw, (w+1)*cw)
-            const int cw = ((tl + AC_BLOCK - 1) / AC_BLOCK) * 32;
-            unsigned keepbits = 0;
-            int wc = 0;
-            for (int r = 0; r * 32 < cw; ++r) {
-                const int e = warp * cw + r * 32 + lane;
-                bool keep = false;
-                if (e < tl) {
-                    float s[DIM];
-                    load_chosen<DIM>(sS, e, s);
-                    keep = !(may_skip && box_gap2<DIM>(s, clo, chi) > thr);
+            const float* gS = v.S + cd.s_off * DIM;
+            // kept chosen points in index order, from their lanes' registers
+            auto take = [&](unsigned kept, const float (&s)[DIM], const int k_of_lane) {
+                while (kept) {
+                    const int b = __ffs(kept) - 1;
+                    kept &= kept - 1;
+                    float sk[DIM];
+#pragma unroll
+                    for (int d = 0; d < DIM; ++d) sk[d] = __shfl_sync(FULL, s[d], b);
+                    assign_one<DIM, ITEMS>(sk, __shfl_sync(FULL, k_of_lane, b), np2, best, sec, key);
                 }
-                keepbits |= keep ? (1u << r) : 0u;
-                wc += __popc(__ballot_sync(FULL, keep));
-            }
-            if (lane == 0) s_wcnt[buf][warp] = wc;
-            __syncthreads();
-            int pos = 0, nk = 0;
+            };
+            float s[DIM];
+            if (n_list >= 0) {
+                const int k = (lane < n_list) ? list[lane] : 0;
 #pragma unroll
-            for (int w = 0; w < AC_WARPS; ++w) {
-                const int x = s_wcnt[buf][w];
-                pos += (w < warp) ? x : 0;
-                nk += x;
-            }
-            for (int r = 0; r * 32 < cw; ++r) {
-                const bool keep = (keepbits >> r) & 1u;
-                const unsigned bal = __ballot_sync(FULL, keep);
-                if (keep) sK[buf][pos + __popc(bal & ((1u << lane) - 1u))] = warp * cw + r * 32 + lane;
-                pos += __popc(bal);
-            }
-            __syncthreads();
-            // warp level: the survivors against this warp's box, then distances
-            for (int q0 = 0; q0 < nk; q0 += 32) {
-                const int q = q0 + lane;
-                int e = 0;
-                bool keep = false;
-                if (q < nk) {
-                    e = sK[buf][q];
-                    float s[DIM];
-                    load_chosen<DIM>(sS, e, s);
-                    keep = !(may_skip && box_gap2<DIM>(s, blo, bhi) > thr);
+                for (int d = 0; d < DIM; ++d) s[d] = gS[(int64_t)k * DIM + d];
+                take(__ballot_sync(FULL, lane < n_list && !(may_skip && block_gap2<DIM>(s, box) > thr)),
+                     s, k);
+                if (lane == 0) v.lslack[wb] = list_left;
+            } else {
+                float sn[DIM];
+                int len = 0;
+#pragma unroll
+                for (int d = 0; d < DIM; ++d) sn[d] = (lane < ns) ? gS[(int64_t)lane * DIM + d] : 0.0f;
+                for (int q0 = 0; q0 < ns; q0 += 32) {
+                    const int q = q0 + lane;
+#pragma unroll
+                    for (int d = 0; d < DIM; ++d) {
+                        s[d] = sn[d];
+                        sn[d] = (q + 32 < ns) ? gS[(int64_t)(q + 32) * DIM + d] : 0.0f;
+                    }
+                    const float g2 = block_gap2<DIM>(s, box);
+                    const bool near = q < ns && !(may_skip && g2 > thr_list);
+                    const unsigned nb = __ballot_sync(FULL, near);
+                    if (!nb) continue;
+                    const int at = len + __popc(nb & lanemask_lt());
+                    if (near && at < 32) list[at] = q;
+                    len += __popc(nb);
+                    take(__ballot_sync(FULL, q < ns && !(may_skip && g2 > thr)), s, q);
                 }
-                unsigned bal = __ballot_sync(FULL, keep);
-                // kept chosen points in index order, warp-uniform, two per
-                // step: both distances are in flight together, and the
-                // minimum is updated with the first one before the second
-                while (bal) {
-                    const int b1 = __ffs(bal) - 1;
-                    bal &= bal - 1;
-                    const bool two = bal != 0u;
-                    const int b2 = two ? __ffs(bal) - 1 : b1;
-                    bal &= bal - 1;
-                    const int e1 = __shfl_sync(FULL, e, b1), e2 = __shfl_sync(FULL, e, b2);
-                    float s1[DIM], s2[DIM];
-                    load_chosen<DIM>(sS, e1, s1);
-                    load_chosen<DIM>(sS, e2, s2);
-                    const int k1 = t0 + e1, k2 = t0 + e2;
+                if (lane == 0) {
+                    v.blen[wb] = len;
+                    v.lslack[wb] = (may_skip && len <= 32) ? 0.25f * cd.r1 : 0.0f;
+                }
+            }
+            const float r1 = cd.r1;
+            float margin = FLT_MAX;
+            int32_t* hist = v.hist + cd.hist_off;
 #pragma unroll
-                    for (int jj = 0; jj < AC_ITEMS / 2; ++jj) {
-                        const float2 d1 = sqdist2_exact<DIM>(s1, np2[jj]);
-                        const float2 d2 = sqdist2_exact<DIM>(s2, np2[jj]);
-                        if (d1.x < best[2 * jj]) { best[2 * jj] = d1.x; bi[2 * jj] = k1; }
-                        if (d1.y < best[2 * jj + 1]) { best[2 * jj + 1] = d1.y; bi[2 * jj + 1] = k1; }
-                        if (two && d2.x < best[2 * jj]) { best[2 * jj] = d2.x; bi[2 * jj] = k2; }
-                        if (two && d2.y < best[2 * jj + 1]) { best[2 * jj + 1] = d2.y; bi[2 * jj + 1] = k2; }
+            for (int j = 0; j < ITEMS; ++j) {
+                const int i = pos0 + j * 32;
+                if (i >= cd.n_all) continue;
+                const bool in = best[j] <= rsq;
+                const int k = in ? key[j] : -1;
+                const float d1 = sqrtf(best[j]);
+                const float mj = in ? 0.5f * (fminf(sqrtf(sec[j]), r1) - d1) : fminf(d1 - r1, 4.0e-4f * r1);
+                margin = fminf(margin, mj);
+                if (k != old[j]) {
+                    const int slot = v.sorder[cd.p_off + i];
+                    int32_t* row = hist + (int64_t)v.srow[cd.p_off + i] * cd.ns_cap;
+                    v.keys[slot] = k;
+                    ksp[i] = k;
+                    if (old[j] >= 0) {
+                        atomicAdd(&row[old[j]], -1);
+                        if (!full) push_edit(v, c, cd, old[j], (int)(slot - cd.p_off));
+                    }
+                    if (k >= 0) {
+                        atomicAdd(&row[k], 1);
+                        if (!full) push_edit(v, c, cd, k, (int)(slot - cd.p_off) | EDIT_IN);
                     }
                 }
             }
+            // never negative, so that it orders as its bits do; 0: evaluate again
+            margin = may_skip ? fmaxf(margin - 1.0e-5f * r1, 0.0f) : 0.0f;
+            const unsigned mb = __reduce_min_sync(FULL, __float_as_uint(margin));
+            if (lane == 0) v.bslack[wb] = __uint_as_float(mb);
         }
-        int32_t* hist = v.hist + cd.hist_off;
-#pragma unroll
-        for (int j = 0; j < AC_ITEMS; ++j) {
-            if (cur.slot[j] >= 0) {
-                const int key = (best[j] <= rsq) ? bi[j] : -1;
-                v.keys[cur.slot[j]] = key;
-                if (key >= 0) atomicAdd(&hist[(int64_t)cur.row[j] * cd.ns_cap + key], 1);
-            }
-        }
-        cur = nxt;
     }
 }
 
 // ---------------------------------------------------------------------------
-// Chunk scan: for every chosen point k of a cloud, the exclusive prefix over
-// the cloud's chunks of the chunk x key histogram (in place: afterwards row lc
-// holds, for each key, the members in earlier chunks) and the member count
+// Chunk scan, for the clouds that regroup in this pass (rebuilds): for every
+// chosen point k, the exclusive prefix over the cloud's chunks of the chunk x
+// key histogram (hpre row lc: members in earlier chunks) and the member count
 // cnt[k].  Work item = block of KBLK keys, one key per lane.
 //   k_chunkscan_cta   clouds with more than SCAN_ROWS_WARP chunk rows: one CTA
 //                     per item; the CS_W warps take contiguous row ranges, sum
@@ -913,14 +957,33 @@ __global__ void __launch_bounds__(AC_BLOCK) k_assign_cull(EngineView v)
 //   k_chunkscan_warp  the other clouds: one warp per item, a single pass.
 // The key bases follow in the same kernel: the CTA (warp) that finishes the
 // last key block of a cloud -- a per-cloud counter of finished blocks says
-// which -- forms the exclusive prefix of the cloud's member counts (each
-// key's first grouped slot) and lists the keys of SUM_BIG_MIN or more members
-// for the CTA-wide folds of k_sum_shift.
+// which -- lays out the cloud's lists (each key's region starts after the
+// regions of the keys before it) and lists every key as work for k_merge_fold.
+// In most passes no cloud regroups: the threads of a CTA (lanes of a warp) look
+// at its next items' clouds together, so that it is done after one look.
 // ---------------------------------------------------------------------------
 constexpr int CS_W = 16;   // warps of the CTA-wide scan
 constexpr int CSW_W = 8;   // items (warps) per CTA of the warp-wide scan
 constexpr int CS_LOADS = 16;  // histogram loads in flight per lane
 constexpr int CS_REG = 32;    // rows per warp kept in registers between the two passes
+
+// the moves of the last pass have been read: empty every active cloud's list
+__device__ __forceinline__ void clear_moves(const EngineView& v, const int first, const int stride)
+{
+    const int nact = v.ctr[CTR_NACT];
+    for (int a = first; a < nact; a += stride) {
+        v.mvn[v.act_cloud[a]] = 0;
+        v.dmax[v.act_cloud[a]] = 0;
+    }
+}
+
+// key k (global slot s) of a rebuilt cloud: its region [at, at + cap)
+__device__ __forceinline__ void place_key(const EngineView& v, const int64_t s, const int at, const int cap)
+{
+    v.base[s] = at;
+    v.kcap[s] = cap;
+    if (v.ecnt[s] == 0) v.dlist[atomicAdd(&v.ctr[CTR_NDIRTY], 1)] = (int)s;  // else push_edit did
+}
 
 // key bases of cloud c by the whole CTA (any multiple of 32 threads)
 __device__ void key_bases_cta(const EngineView& v, const int c, int* s_w, int& s_carry)
@@ -929,13 +992,12 @@ __device__ void key_bases_cta(const EngineView& v, const int c, int* s_w, int& s
     const CloudDesc cd = v.cl[c];
     const int ns = v.ns[c];
     const int32_t* cnt = v.cnt + cd.key_off;
-    int32_t* base = v.base + cd.key_off;
     __syncthreads();  // earlier readers of s_w / s_carry are done
     if (threadIdx.x == 0) s_carry = 0;
     for (int k0 = 0; k0 < ns; k0 += blockDim.x) {
         __syncthreads();
         const int k = k0 + threadIdx.x;
-        const int x = (k < ns) ? cnt[k] : 0;
+        const int x = (k < ns) ? list_cap(v, cnt[k]) : 0;
         int incl = x;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -950,8 +1012,7 @@ __device__ void key_bases_cta(const EngineView& v, const int c, int* s_w, int& s
             tot += s_w[w];
         }
         const int carry = s_carry;
-        if (k < ns) base[k] = carry + wpre + incl - x;
-        if (x >= SUM_BIG_MIN) v.big[atomicAdd(&v.ctr[CTR_NBIG], 1)] = (int)(cd.key_off + k);
+        if (k < ns) place_key(v, cd.key_off + k, carry + wpre + incl - x, x);
         __syncthreads();
         if (threadIdx.x == 0) s_carry = carry + tot;
     }
@@ -963,19 +1024,17 @@ __device__ void key_bases_warp(const EngineView& v, const int c, const int lane)
     const CloudDesc cd = v.cl[c];
     const int ns = v.ns[c];
     const int32_t* cnt = v.cnt + cd.key_off;
-    int32_t* base = v.base + cd.key_off;
     int carry = 0;
     for (int k0 = 0; k0 < ns; k0 += 32) {
         const int k = k0 + lane;
-        const int x = (k < ns) ? cnt[k] : 0;
+        const int x = (k < ns) ? list_cap(v, cnt[k]) : 0;
         int incl = x;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             const int y = __shfl_up_sync(FULL, incl, o);
             if (lane >= o) incl += y;
         }
-        if (k < ns) base[k] = carry + incl - x;
-        if (x >= SUM_BIG_MIN) v.big[atomicAdd(&v.ctr[CTR_NBIG], 1)] = (int)(cd.key_off + k);
+        if (k < ns) place_key(v, cd.key_off + k, carry + incl - x, x);
         carry += __shfl_sync(FULL, incl, 31);
     }
 }
@@ -985,19 +1044,38 @@ __global__ void __launch_bounds__(CS_W * 32) k_chunkscan_cta(EngineView v)
     pdl_enter();
     __shared__ int s_part[CS_W][32];
     __shared__ int s_w[CS_W];
-    __shared__ int s_carry, s_last;
+    __shared__ int s_carry, s_last, s_n;
+    __shared__ int2 s_item[CS_W * 32];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    clear_moves(v, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
     const ActiveList al(v, ACT_KBLK);
-    for (int item = blockIdx.x; item < al.total; item += gridDim.x) {
-        int c, kb;
-        al.locate(item, c, kb);
+    for (int64_t item0 = blockIdx.x; item0 < al.total; item0 += (int64_t)gridDim.x * blockDim.x) {
+        // this thread's look: the CTA's threadIdx.x-th next item
+        const int64_t mine = item0 + (int64_t)threadIdx.x * gridDim.x;
+        int my_c = -1, my_kb = 0;
+        if (mine < al.total) {
+            al.locate((int)mine, my_c, my_kb);
+            if (!rebuilds(v, my_c)) my_c = -1;
+        }
+        if (!__syncthreads_or(my_c >= 0)) continue;
+        if (threadIdx.x == 0) s_n = 0;
+        __syncthreads();
+        if (my_c >= 0) {
+            const int at = atomicAdd(&s_n, 1);
+            s_item[at] = make_int2(my_c, my_kb);
+        }
+        __syncthreads();
+        const int n_items = s_n;
+        for (int q = 0; q < n_items; ++q) {
+        const int c = s_item[q].x, kb = s_item[q].y;
         const CloudDesc cd = v.cl[c];
         const int ns = v.ns[c];
         const int k = kb * KBLK + lane;
         const bool ok = k < ns;
         const int rows = cd.n_chunks;
         const int rw0 = (warp * rows) / CS_W, rw1 = ((warp + 1) * rows) / CS_W;
-        int32_t* h = v.hist + cd.hist_off + k;
+        const int32_t* h = v.hist + cd.hist_off + k;
+        int32_t* hp = v.hpre + cd.hist_off + k;
         // the first CS_REG rows of the warp's range stay in registers for the
         // rescan; longer ranges reload the rest
         int xr[CS_REG];
@@ -1026,7 +1104,7 @@ __global__ void __launch_bounds__(CS_W * 32) k_chunkscan_cta(EngineView v)
         }
 #pragma unroll
         for (int u = 0; u < CS_REG; ++u) {
-            if (ok && rw0 + u < rw1) h[(int64_t)(rw0 + u) * cd.ns_cap] = run;
+            if (ok && rw0 + u < rw1) hp[(int64_t)(rw0 + u) * cd.ns_cap] = run;
             run += xr[u];
         }
         for (int r0 = rw0 + CS_REG; r0 < rw1; r0 += CS_LOADS) {
@@ -1036,7 +1114,7 @@ __global__ void __launch_bounds__(CS_W * 32) k_chunkscan_cta(EngineView v)
                 x[u] = (ok && r0 + u < rw1) ? h[(int64_t)(r0 + u) * cd.ns_cap] : 0;
 #pragma unroll
             for (int u = 0; u < CS_LOADS; ++u) {
-                if (ok && r0 + u < rw1) h[(int64_t)(r0 + u) * cd.ns_cap] = run;
+                if (ok && r0 + u < rw1) hp[(int64_t)(r0 + u) * cd.ns_cap] = run;
                 run += x[u];
             }
         }
@@ -1052,6 +1130,8 @@ __global__ void __launch_bounds__(CS_W * 32) k_chunkscan_cta(EngineView v)
             key_bases_cta(v, c, s_w, s_carry);
             if (threadIdx.x == 0) v.kbdone[c] = 0;
         }
+        }
+        __syncthreads();   // s_item and s_n are read no more
     }
 }
 
@@ -1059,17 +1139,28 @@ __global__ void __launch_bounds__(CSW_W * 32) k_chunkscan_warp(EngineView v)
 {
     pdl_enter();
     const int lane = threadIdx.x & 31;
+    clear_moves(v, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
     const ActiveList al(v, ACT_KBLK_WARP);
     const int stride = gridDim.x * CSW_W;
-    for (int item = blockIdx.x * CSW_W + (threadIdx.x >> 5); item < al.total; item += stride) {
-        int c, kb;
-        al.locate(item, c, kb);
+    for (int64_t item0 = blockIdx.x * CSW_W + (threadIdx.x >> 5); item0 < al.total;
+         item0 += (int64_t)32 * stride) {
+        // this lane's look: the warp's lane-th next item
+        const int64_t mine = item0 + (int64_t)lane * stride;
+        int my_c = -1, my_kb = 0;
+        if (mine < al.total) {
+            al.locate((int)mine, my_c, my_kb);
+            if (!rebuilds(v, my_c)) my_c = -1;
+        }
+        for (unsigned todo = __ballot_sync(FULL, my_c >= 0); todo; todo &= todo - 1) {
+        const int src = __ffs(todo) - 1;
+        const int c = __shfl_sync(FULL, my_c, src), kb = __shfl_sync(FULL, my_kb, src);
         const CloudDesc cd = v.cl[c];
         const int ns = v.ns[c];
         const int k = kb * KBLK + lane;
         const bool ok = k < ns;
         const int rows = cd.n_chunks;
-        int32_t* h = v.hist + cd.hist_off + k;
+        const int32_t* h = v.hist + cd.hist_off + k;
+        int32_t* hp = v.hpre + cd.hist_off + k;
         int run = 0;
         for (int r0 = 0; r0 < rows; r0 += CS_LOADS) {
             int x[CS_LOADS];
@@ -1078,7 +1169,7 @@ __global__ void __launch_bounds__(CSW_W * 32) k_chunkscan_warp(EngineView v)
                 x[u] = (ok && r0 + u < rows) ? h[(int64_t)(r0 + u) * cd.ns_cap] : 0;
 #pragma unroll
             for (int u = 0; u < CS_LOADS; ++u) {
-                if (ok && r0 + u < rows) h[(int64_t)(r0 + u) * cd.ns_cap] = run;
+                if (ok && r0 + u < rows) hp[(int64_t)(r0 + u) * cd.ns_cap] = run;
                 run += x[u];
             }
         }
@@ -1092,6 +1183,7 @@ __global__ void __launch_bounds__(CSW_W * 32) k_chunkscan_warp(EngineView v)
             __threadfence();
             key_bases_warp(v, c, lane);
             if (lane == 0) v.kbdone[c] = 0;
+        }
         }
     }
 }
@@ -1133,6 +1225,8 @@ __device__ __forceinline__ void store_row(float* rows, int64_t r, const float (&
 // each in index order.  Ranges are in index order too, so the placement stays
 // stable while the dependent placement chain is SCAT_W times shorter.  Larger
 // chosen sets use scatter_chunk (one warp) in warp 0.
+// Only the clouds that regroup in this pass are scattered; the threads of a CTA
+// look at its next chunks' clouds together.
 // groups of more clouds than this are gathered and compacted one thread per
 // cloud (decimate_group)
 constexpr int DEC_CLOUDS_SERIAL = 32;
@@ -1148,12 +1242,25 @@ __global__ void __launch_bounds__(SCAT_W * 32) k_scatter_cta(EngineView v)
     pdl_enter();
     constexpr int DP = PadDim<DIM>::v;
     extern __shared__ int s_dyn[];
+    __shared__ int2 s_item[SCAT_W * 32];
+    __shared__ int s_n;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const ActiveList al(v, ACT_CHUNK);
-    for (int item = blockIdx.x; item < al.total; item += gridDim.x) {
+    for (int64_t item0 = blockIdx.x; item0 < al.total; item0 += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t mine = item0 + (int64_t)tid * gridDim.x;
+        int my_c = -1, my_lc = 0;
+        if (mine < al.total) {
+            al.locate((int)mine, my_c, my_lc);
+            if (!rebuilds(v, my_c)) my_c = -1;
+        }
+        if (tid == 0) s_n = 0;
+        if (!__syncthreads_or(my_c >= 0)) continue;
+        if (my_c >= 0) s_item[atomicAdd(&s_n, 1)] = make_int2(my_c, my_lc);
+        __syncthreads();
+        const int n_items = s_n;
+        for (int q = 0; q < n_items; ++q) {
         __syncthreads();  // the previous chunk's readers are done
-        int c, lc;
-        al.locate(item, c, lc);
+        const int c = s_item[q].x, lc = s_item[q].y;
         const CloudDesc cd = v.cl[c];
         const int ns = v.ns[c];
         if (ns > SCAT_HMAX) {
@@ -1166,20 +1273,22 @@ __global__ void __launch_bounds__(SCAT_W * 32) k_scatter_cta(EngineView v)
         int* s_keys = s_dyn;                 // chunk_max
         int* hw = s_dyn + v.chunk_max;       // SCAT_W x ns: counts, then start slots
         const int32_t* keys = v.keys + cd.p_off + start;
-        int32_t* row = v.hist + cd.hist_off + (int64_t)lc * cd.ns_cap;
+        const int32_t* row = v.hpre + cd.hist_off + (int64_t)lc * cd.ns_cap;
         const int32_t* bs = v.base + cd.key_off;
         const float* Pc = v.P + (cd.p_off + start) * DIM;
+        float* Pg = v.Lr[0] + cd.reg_off * DP;
+        int32_t* Ls = v.Ls[0] + cd.reg_off;
         const int r0 = (warp * len) / SCAT_W, r1 = ((warp + 1) * len) / SCAT_W;
-        // Every global load of the chunk is issued up front -- its keys, its
-        // key bases and histogram row, and the coordinates of this warp's
-        // first SCAT_SP placement steps -- so the chunk waits for one memory
-        // round trip instead of one per loop step.
         int kv[SCAT_KS];
 #pragma unroll
         for (int u = 0; u < SCAT_KS; ++u) {
             const int e = u * SCAT_W * 32 + tid;
             kv[u] = (e < len) ? keys[e] : -1;
         }
+        // Every global load of the chunk is issued up front -- its key bases
+        // and histogram row, and the coordinates of this warp's first SCAT_SP
+        // placement steps -- so the chunk waits for one memory round trip
+        // instead of one per loop step.
         int bsv[SCAT_HMAX / (SCAT_W * 32)], rwv[SCAT_HMAX / (SCAT_W * 32)];
 #pragma unroll
         for (int u = 0; u < SCAT_HMAX / (SCAT_W * 32); ++u) {
@@ -1214,7 +1323,6 @@ __global__ void __launch_bounds__(SCAT_W * 32) k_scatter_cta(EngineView v)
             const int k = u * SCAT_W * 32 + tid;
             if (k < ns) {
                 int run = bsv[u] + rwv[u];
-                row[k] = 0;  // the row is free again for the next pass's counts
 #pragma unroll
                 for (int w = 0; w < SCAT_W; ++w) {
                     const int x = hw[w * ns + k];
@@ -1225,7 +1333,6 @@ __global__ void __launch_bounds__(SCAT_W * 32) k_scatter_cta(EngineView v)
         }
         __syncthreads();
         int* cur = hw + warp * ns;
-        float* Pg = v.Pg + cd.p_off * DP;
         for (int g0 = r0; g0 < r1; g0 += 32 * SCAT_SP) {
             if (g0 > r0) {  // ranges longer than SCAT_SP steps: the next steps' coordinates
 #pragma unroll
@@ -1250,9 +1357,14 @@ __global__ void __launch_bounds__(SCAT_W * 32) k_scatter_cta(EngineView v)
                 float qv[DIM];
 #pragma unroll
                 for (int d = 0; d < DIM; ++d) qv[d] = __shfl_sync(FULL, pc[q][d], r.src);
-                if (r.key >= 0) store_row<DIM>(Pg, b + r.rank, qv);
+                if (r.key >= 0) {
+                    store_row<DIM>(Pg, b + r.rank, qv);
+                    if (v.cull) Ls[b + r.rank] = start + i0 + r.src;
+                }
             }
         }
+        }
+        __syncthreads();  // s_item and s_n are read no more
     }
 }
 
@@ -1270,9 +1382,10 @@ __device__ void scatter_chunk(const EngineView& v, int c, int lc, int* s_keys, i
     constexpr int DP = PadDim<DIM>::v;
     const CloudDesc cd = v.cl[c];
     const int ns = v.ns[c];
-    int32_t* row = v.hist + cd.hist_off + (int64_t)lc * cd.ns_cap;
+    int32_t* row = v.hpre + cd.hist_off + (int64_t)lc * cd.ns_cap;
     const int32_t* bs = v.base + cd.key_off;
     const bool in_smem = ns <= v.scat_smem;
+    // the row's prefixes are not needed after this chunk
     int32_t* ctr = in_smem ? (s_keys + v.chunk_max) : row;
     const int start = (int)(((int64_t)lc * cd.n_all) / cd.n_chunks);
     const int end = (int)(((int64_t)(lc + 1) * cd.n_all) / cd.n_chunks);
@@ -1286,7 +1399,7 @@ __device__ void scatter_chunk(const EngineView& v, int c, int lc, int* s_keys, i
 #pragma unroll
         for (int u = 0; u < 8; ++u) {
             const int e = e0 + u * 32 + lane;
-            t[u] = (e < len) ? keys[e] : 0;
+            t[u] = (e < len) ? keys[e] : -1;
         }
 #pragma unroll
         for (int u = 0; u < 8; ++u) {
@@ -1310,7 +1423,8 @@ __device__ void scatter_chunk(const EngineView& v, int c, int lc, int* s_keys, i
     }
     __syncwarp();
     const float* Pc = v.P + (cd.p_off + start) * DIM;
-    float* Pg = v.Pg + cd.p_off * DP;
+    float* Pg = v.Lr[0] + cd.reg_off * DP;
+    int32_t* Ls = v.Ls[0] + cd.reg_off;
     for (int off = 0; off < len; off += 32) {
         const int i = off + lane;
         float pc[DIM];
@@ -1326,24 +1440,20 @@ __device__ void scatter_chunk(const EngineView& v, int c, int lc, int* s_keys, i
         float q[DIM];
 #pragma unroll
         for (int d = 0; d < DIM; ++d) q[d] = __shfl_sync(FULL, pc[d], r.src);
-        if (r.key >= 0) store_row<DIM>(Pg, b + r.rank, q);
+        if (r.key >= 0) {
+            store_row<DIM>(Pg, b + r.rank, q);
+            if (v.cull) Ls[b + r.rank] = start + off + r.src;
+        }
         __syncwarp();
     }
-    for (int k = lane; k < ns; k += 32) row[k] = 0;  // free for the next pass's counts
 }
 
 // ---------------------------------------------------------------------------
-// ordered sum + shift: one warp per chosen slot.  Lane d (< DIM) folds
-// coordinate d of the key's members in index order with rounded adds,
-// exactly as rd/cpu/brute_force/evolve.hpp:71-74 accumulates, then applies the
-// movement test of evolve.hpp:143-177.  Members are gathered through the
-// permutation written by k_scatter_cta, BP at a time, the next block in flight
-// while the current one is folded.
+// ordered sums: lane d (< DIM) of a warp folds coordinate d of a key's members in
+// index order with rounded adds, exactly as rd/cpu/brute_force/evolve.hpp:71-74
+// accumulates, then applies the movement test of evolve.hpp:143-177.
 // ---------------------------------------------------------------------------
 constexpr int SUM_BP = 128;  // members staged per step of the ordered fold
-// k_sum_shift stages 256 members per step: folding a block (about 256 dependent
-// adds) then outlasts the gather of the next one from L2
-constexpr int SUM_BP_WIDE = 256;
 // points (keys) per lane loaded together by the fused tile kernel's
 // assignment (placement) loop
 constexpr int TILE_PPL = 8;
@@ -1355,57 +1465,6 @@ constexpr int FOLD_CTA_MIN = 4096;
 // keys need the CTA-wide folds, went to clusters; the others fold faster with
 // every warp on its own keys
 constexpr int FOLD_CTA_MIN_LIGHT = 1 << 30;
-
-template <int DIM>
-__device__ void sum_shift_one(const EngineView& v, int c, int k, float* buf, int lane, bool cta_big);
-
-template <int DIM>
-__device__ void sum_shift_big_one(const EngineView& v, int slot, SegFoldSmem<8, DIM>& sm);
-
-// the per-cloud control step after a pass (k_control), over clouds first,
-// first + stride, ... of the active list
-__device__ void control_clouds(const EngineView& v, const int first, const int stride);
-
-// grid = big_ctas CTAs for the listed big keys (one key at a time each), then
-// the CTAs whose warps take one smaller key each
-// with_control: the last CTA to finish runs the control step of k_control
-// (the moved flags of every fold are then complete)
-template <int DIM>
-__global__ void __launch_bounds__(256) k_sum_shift(EngineView v, int big_ctas, int with_control)
-{
-    pdl_enter();
-    __shared__ __align__(16) unsigned char s_raw[8 * SUM_BP_WIDE * (DIM + 1) * 4];
-    __shared__ int s_last;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int nbig = v.ctr[CTR_NBIG];
-    const bool cta_big = nbig <= SUM_BIG_PER_CTA * big_ctas;  // else every key goes to a warp
-    if ((int)blockIdx.x < big_ctas) {
-        static_assert(sizeof(SegFoldSmem<8, DIM>) <= sizeof(s_raw), "big-key fold scratch");
-        SegFoldSmem<8, DIM>& sm = *reinterpret_cast<SegFoldSmem<8, DIM>*>(s_raw);
-        if (cta_big)
-            for (int i = blockIdx.x; i < nbig; i += big_ctas) sum_shift_big_one<DIM>(v, v.big[i], sm);
-    } else {
-        float* s_buf = reinterpret_cast<float*>(s_raw) + warp * SUM_BP_WIDE * PadDim<DIM>::v;
-        const ActiveList al(v, ACT_SLOT);
-        const int b = (int)blockIdx.x - big_ctas, nb = (int)gridDim.x - big_ctas;
-        for (int t = b * 8 + warp; t < al.total; t += nb * 8) {
-            __syncwarp();
-            int c, k;
-            al.locate(t, c, k);
-            sum_shift_one<DIM>(v, c, k, s_buf, lane, cta_big);
-        }
-    }
-    if (!with_control) return;
-    // every thread's writes (chosen points, moved flags) before the count
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) s_last = atomicAdd(&v.ctr[CTR_SUM_DONE], 1) == (int)gridDim.x - 1;
-    __syncthreads();
-    if (!s_last) return;
-    __threadfence();
-    control_clouds(v, threadIdx.x, blockDim.x);
-    if (threadIdx.x == 0) v.ctr[CTR_SUM_DONE] = 0;
-}
 
 // Sequential FP32 fold, in list order, of the points P[perm[0..n)] (one warp;
 // the sum of coordinate d is returned in lane d < DIM).
@@ -1476,18 +1535,46 @@ template <int DIM>
 __device__ void apply_shift(const EngineView& v, int c, const CloudDesc& cd, int k, int n, float sum,
                             int lane)
 {
-    int moved = 0;
+    int moved = 0, changed = 0;
+    float was = 0.0f, now = 0.0f;
     if (lane < DIM) {
         float* s = v.S + (cd.s_off + k) * DIM + lane;
+        was = now = *s;
         if (v.flags & ENG_ALWAYS_MOVE) {
-            *s = __fdiv_rn(sum, (float)n);  // mean, no movement test
+            now = __fdiv_rn(sum, (float)n);  // mean, no movement test
+            changed = !(now == was);
+            *s = now;
         } else {
-            float cval = *s;
-            moved = shift_coord(sum, n, cval);
-            if (moved) *s = cval;
+            changed = moved = shift_coord(sum, n, now);
+            if (moved) *s = now;
         }
     }
     if (__any_sync(FULL, moved) && lane == 0) v.cont[c] = 1;
+    if (!v.cull || !__any_sync(FULL, changed)) return;
+    // the move, for the blocks of points near it (k_assign_cull): old and new
+    // place, and its length rounded up
+    const float dd = fabsf(__fsub_rn(now, was));
+    float len2 = 0.0f;
+#pragma unroll
+    for (int d = 0; d < DIM; ++d) {
+        const float x = __shfl_sync(FULL, dd, d);
+        len2 = __fadd_ru(len2, __fmul_ru(x, x));
+    }
+    // (the difference was rounded to nearest: one part in 2^20 covers it; a
+    // length that underflows counts as the smallest one that matters)
+    const float len = fmaxf(__fmul_ru(__fsqrt_ru(len2), 1.000001f), 1.0e-30f);
+    int at = 0;
+    if (lane == 0) {
+        at = atomicAdd(&v.mvn[c], 1);
+        atomicMax(&v.dmax[c], (len2 == len2) ? __float_as_int(len) : 0x7fc00000);
+    }
+    at = __shfl_sync(FULL, at, 0);
+    float* mv = v.mv + cd.key_off + at;
+    if (lane < DIM) {
+        mv[(int64_t)lane * v.n_slots] = was;
+        mv[(int64_t)(DIM + lane) * v.n_slots] = now;
+    }
+    if (lane == 0) mv[(int64_t)(2 * DIM) * v.n_slots] = (len2 == len2) ? len : __int_as_float(0x7fc00000);
 }
 
 // Sequential FP32 fold, in order, of n contiguous rows of a grouped copy
@@ -1546,39 +1633,360 @@ __device__ float fold_rows(const float* __restrict__ rows, const int n, float* b
     return sum;
 }
 
+// ---------------------------------------------------------------------------
+// Member lists, ordered sum and shift: one CTA per listed key (dlist).
+//
+// Every key keeps its members' coordinates and positions in index order, in its
+// region of the grouped lists, from pass to pass.  In a cloud that regroups
+// (rebuilds) the scatter has just written the lists anew; otherwise the key's
+// edits of this pass are merged in.  The edits are sorted by position in shared
+// memory (each counts the smaller ones).  Seven warps take the old list in
+// chunks of MF_ROWS rows, the next two chunks' loads in flight.  The position of
+// each chunk's first row says which edits fall into the chunk; a row finds by
+// binary search how many of them come before it, which gives its new place (or
+// that it leaves), and takes along the points that join right before it; a
+// chunk without edits moves as a whole.  New rows go to a ring in shared memory
+// and to the other buffer; the eighth warp folds the ring behind them with the
+// reference's chain of rounded adds (lane d: coordinate d;
+// rd/cpu/brute_force/evolve.hpp:71-74) and applies the movement test
+// (evolve.hpp:143-177).  A list that outgrows its region is folded all the
+// same, and the cloud regroups in the next pass.
+//
+// Bound by the add chain of the longest listed key, about 2.3 ns per member;
+// the merge of a chunk runs beside it and takes less.  Keys without edits cost
+// nothing.  1M-point helix, after the assignment: scan, scatter and one-warp
+// folds of every key took 70 us per pass; this kernel takes 20-40 us (790 keys of
+// 1,266 members, most with edits), 12-20 us (few keys with edits), 45-50 us (116
+// keys of 8,300 members, 20 us of it the add chain of the longest).
+// ---------------------------------------------------------------------------
+constexpr int MF_BLOCK = 256;
+constexpr int MF_PROD = MF_BLOCK - 32;      // threads that merge
+constexpr int MF_ROWS = MF_PROD;            // rows per chunk, one per thread
+constexpr int MF_RING = 1024;               // two chunks and every edit fit
+constexpr int MF_STAGES = 3;                // chunks of the old list in flight
+constexpr int MF_CUTS = 256;                // chunks whose edits are looked up at once
+constexpr int MF_CHAIN = 32;                // terms the chain takes at a time
+static_assert(2 * MF_ROWS + EDIT_MAX + MF_CHAIN <= MF_RING && MF_RING % MF_CHAIN == 0,
+              "ring of new rows");
+
 template <int DIM>
-__device__ void sum_shift_one(const EngineView& v, int c, int k, float* buf, int lane, bool cta_big)
+struct MergeSmem {
+    union {
+        float ring[DIM][MF_RING + 4];   // per coordinate: the chain loads four terms at once
+        SegFoldSmem<MF_BLOCK / 32, DIM> seg;
+    };
+    alignas(16) float old[MF_STAGES][MF_ROWS * PadDim<DIM>::v];   // chunks of the old list
+    int pos[MF_STAGES][MF_ROWS + 1];                  // their positions, after the row before's
+    alignas(16) float joins[EDIT_MAX * PadDim<DIM>::v];   // coordinates of the joining edits
+    int raw[EDIT_MAX];        // edits as listed
+    int ed[EDIT_MAX];         // by position
+    int ins[EDIT_MAX + 1];    // joining ones among the first i
+    int cut[MF_CUTS + 1];     // edits before the first row of each chunk
+};
+
+// the per-cloud control step after a pass (k_control), over clouds first,
+// first + stride, ... of the active list
+__device__ void control_clouds(const EngineView& v, const int first, const int stride);
+__device__ void loop_condition(const EngineView& v, cudaGraphConditionalHandle h, int use_handle,
+                               int count_iter);
+
+template <int DIM>
+__device__ __forceinline__ void load_row(const float* rows, const int64_t r, float (&q)[DIM])
 {
-    const CloudDesc cd = v.cl[c];
-    const int n = v.cnt[cd.key_off + k];
-    if (n == 0 || (cta_big && n >= SUM_BIG_MIN)) return;  // big keys: the CTA path
-    const float* rows = v.Pg + (cd.p_off + v.base[cd.key_off + k]) * PadDim<DIM>::v;
-    const float sum = fold_rows<DIM, SUM_BP_WIDE>(rows, n, buf, lane);
-    apply_shift<DIM>(v, c, cd, k, n, sum, lane);
+    constexpr int DP = PadDim<DIM>::v;
+    if constexpr (DP == 4) {
+        const float4 t = reinterpret_cast<const float4*>(rows)[r];
+        q[0] = t.x;
+        if constexpr (DIM > 1) q[1] = t.y;
+        if constexpr (DIM > 2) q[2] = t.z;
+        if constexpr (DIM > 3) q[3] = t.w;
+    } else if constexpr (DP == 2) {
+        const float2 t = reinterpret_cast<const float2*>(rows)[r];
+        q[0] = t.x;
+        q[1] = t.y;
+    } else {
+        q[0] = rows[r];
+    }
 }
 
-// ---------------------------------------------------------------------------
-// The same ordered sum + shift for one key of SUM_BIG_MIN or more members
-// (global chosen slot `slot`), by a whole CTA: warps 1..7 gather the members'
-// coordinates (in member order) into one of two shared buffers while warp 0
-// folds the other with the same chain of rounded adds (lane d: coordinate
-// d), so the gathers of a large cluster no longer stall its add chain.
-// ---------------------------------------------------------------------------
-// One big key folded by the whole CTA: the warp-segmented exact fold of
-// rd_segfold.cuh (eight warp segments from speculative starts, traces replayed
-// from the exact start), then the shift.
-template <int DIM>
-__device__ void sum_shift_big_one(const EngineView& v, int slot, SegFoldSmem<8, DIM>& sm)
+// edits at positions below x, which are at least lo and at most hi
+__device__ __forceinline__ int edits_below(const int* ed, int lo, int hi, const int x)
 {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if ((ed[mid] & ~EDIT_IN) < x) lo = mid + 1;
+        else hi = mid;
+    }
+    return lo;
+}
+
+__device__ __forceinline__ void lds_f32x4(const uint32_t a, float* x)
+{
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(x[0]), "=f"(x[1]), "=f"(x[2]), "=f"(x[3]) : "r"(a));
+}
+
+// copies BYTES (4, 8 or 16) of global memory to shared memory, asynchronously
+template <int BYTES>
+__device__ __forceinline__ void copy_async(void* to, const void* from)
+{
+    const uint32_t a = (uint32_t)__cvta_generic_to_shared(to);
+    if constexpr (BYTES == 16)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(a), "l"(from) : "memory");
+    else
+        asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(a), "l"(from), "n"(BYTES) : "memory");
+}
+
+// sum + term 0 + term 1 + ... (`n` groups of MF_CHAIN terms in the ring from
+// address a on, its end at `end`; in order, each add rounded): half a group is
+// loaded, four terms at a time, while the half before it is added, so that a
+// term costs its add (4 cycles) and not the load's latency.  A function of its
+// own: inlined into the merge, its registers were spilled and every add waited
+// for its load.
+__device__ __noinline__ float chain_add(uint32_t a, const int n, const uint32_t end, float sum)
+{
+    constexpr int B = MF_CHAIN / 2;
+    float x[B], y[B];
+#pragma unroll
+    for (int u = 0; u < B; u += 4) lds_f32x4(a + u * 4, x + u);
+    for (int g = 0; g < n; ++g) {
+#pragma unroll
+        for (int u = 0; u < B; u += 4) lds_f32x4(a + (B + u) * 4, y + u);
+#pragma unroll
+        for (int u = 0; u < B; ++u) sum = __fadd_rn(sum, x[u]);
+        a += MF_CHAIN * 4;
+        if (a >= end) a -= MF_RING * 4;
+        // (the group after the last one is read and not used)
+#pragma unroll
+        for (int u = 0; u < B; u += 4) lds_f32x4(a + u * 4, x + u);
+#pragma unroll
+        for (int u = 0; u < B; ++u) sum = __fadd_rn(sum, y[u]);
+    }
+    return sum;
+}
+
+// the last m < MF_CHAIN terms
+__device__ __noinline__ float chain_tail(const uint32_t a, const int m, float sum)
+{
+    float x[MF_CHAIN];
+#pragma unroll
+    for (int u = 0; u < MF_CHAIN; u += 4) lds_f32x4(a + u * 4, x + u);
+#pragma unroll
+    for (int u = 0; u < MF_CHAIN; ++u)
+        if (u < m) sum = __fadd_rn(sum, x[u]);
+    return sum;
+}
+
+// apart, so that its registers do not weigh on the merge
+template <int DIM>
+__device__ __noinline__ void fold_long_list(const float* rows, const int n,
+                                            SegFoldSmem<MF_BLOCK / 32, DIM>& sm)
+{
+    fold_members_seg_src<MF_BLOCK / 32, DIM>(RowSrc<DIM>{rows}, n, sm);
+}
+
+template <int DIM>
+__device__ void merge_fold_key(const EngineView& v, const int slot, const bool seg_ok,
+                               MergeSmem<DIM>& sm)
+{
+    constexpr int DP = PadDim<DIM>::v;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int c = v.slot_cloud[slot];
     const CloudDesc cd = v.cl[c];
     const int k = (int)(slot - cd.key_off);
-    const int n = v.cnt[slot];
-    const float* rows = v.Pg + (cd.p_off + v.base[slot]) * PadDim<DIM>::v;
-    __syncthreads();  // the previous key's scratch is no longer read
-    fold_members_seg_src<8, DIM>(RowSrc<DIM>{rows}, n, sm);
-    if (warp == 0) apply_shift<DIM>(v, c, cd, k, n, (lane < DIM) ? sm.out[lane] : 0.0f, lane);
+    const bool fresh = rebuilds(v, c);
+    const int64_t at = cd.reg_off + v.base[slot];
+    const int cap = v.kcap[slot];
+    const int par = fresh ? 0 : v.par[slot];
+    const int n_old = v.cnt[slot];
+    const int ne = fresh ? 0 : v.ecnt[slot];   // at most EDIT_MAX, or the cloud rebuilds
+    const float* src = v.Lr[par] + at * DP;
+    __syncthreads();  // the previous key's scratch, and its state, are read no more
+    for (int i = tid; i < ne; i += MF_BLOCK) sm.raw[i] = v.edit[at + i];
+    __syncthreads();
+    for (int i = tid; i < ne; i += MF_BLOCK) {
+        const int e = sm.raw[i], x = e & ~EDIT_IN;
+        int r = 0;
+        float p[DIM];
+#pragma unroll
+        for (int d = 0; d < DIM; ++d) p[d] = v.P[(cd.p_off + x) * DIM + d];
+        for (int j = 0; j < ne; ++j) r += (sm.raw[j] & ~EDIT_IN) < x;   // positions differ
+        sm.ed[r] = e;
+        store_row<DIM>(sm.joins, r, p);
+    }
+    __syncthreads();
+    if (warp == 0) {
+        int carry = 0;
+        for (int i0 = 0; i0 < ne; i0 += 32) {
+            const bool in = i0 + lane < ne && sm.ed[i0 + lane] < 0;
+            const unsigned bal = __ballot_sync(FULL, in);
+            if (i0 + lane < ne) sm.ins[i0 + lane] = carry + __popc(bal & lanemask_lt());
+            carry += __popc(bal);
+        }
+        if (lane == 0) sm.ins[ne] = carry;
+    }
+    __syncthreads();
+    const int n_new = n_old + 2 * sm.ins[ne] - ne;
+    const bool seg = seg_ok && n_new >= SUM_BIG_MIN && n_new <= cap;
+    const int steps = seg && ne == 0 ? 0 : (max(n_old, 1) + MF_ROWS - 1) / MF_ROWS;
+    float sum = 0.0f;
+    const int32_t* pos = v.cull ? v.Ls[par] + at : nullptr;
+    // edits before chunk s's first row (those before the list's first row go to chunk 0)
+    auto find_cuts = [&](const int s0) {
+        for (int i = tid; i <= MF_CUTS; i += MF_BLOCK) {
+            const int s = s0 + i;
+            sm.cut[i] = (s == 0 || ne == 0) ? 0
+                        : (s < steps) ? edits_below(sm.ed, 0, ne, pos[s * MF_ROWS]) : ne;
+        }
+    };
+    // new rows before chunk s (of the current window of chunks)
+    auto rows_before = [&](const int s, const int s0) {
+        if (s >= steps) return n_new;
+        const int e = sm.cut[s - s0];
+        return s * MF_ROWS - e + 2 * sm.ins[e];
+    };
+    int r = 0;   // rows folded (warp 0)
+    for (int s0 = 0; s0 == 0 || s0 < steps; s0 += MF_CUTS) {
+        find_cuts(s0);
+        __syncthreads();
+        const int s1 = min(steps, s0 + MF_CUTS);
+        if (warp == 0) {
+            // the chain follows the merge one chunk behind
+            for (int s = s0; s <= s1; ++s) {
+                if (s > s0 && !seg) {
+                    // whole groups; the rest waits for the next chunk
+                    const int end = rows_before(s, s0), n = (end - r) / MF_CHAIN;
+                    if (lane < DIM) {
+                        const uint32_t ring = (uint32_t)__cvta_generic_to_shared(sm.ring[lane]);
+                        if (n > 0) sum = chain_add(ring + (r & (MF_RING - 1)) * 4, n, ring + MF_RING * 4, sum);
+                        if (s == steps)
+                            sum = chain_tail(ring + ((r + n * MF_CHAIN) & (MF_RING - 1)) * 4,
+                                             end - r - n * MF_CHAIN, sum);
+                    }
+                    r += n * MF_CHAIN;
+                }
+                __syncthreads();
+            }
+        } else {
+            float* dst = v.Lr[par ^ 1] + at * DP;
+            int32_t* dpos = (v.cull ? v.Ls[par ^ 1] + at : nullptr);
+            const int pt = tid - 32;
+            auto load = [&](const int s) {
+                const int j = s * MF_ROWS + pt, b = s % MF_STAGES;
+                if (j < n_old) {
+                    copy_async<DP * 4>(sm.old[b] + pt * DP, src + (int64_t)j * DP);
+                    if (ne > 0) {
+                        copy_async<4>(&sm.pos[b][pt + 1], pos + j);
+                        if (pt == 0 && j > 0) copy_async<4>(&sm.pos[b][0], pos + j - 1);
+                    }
+                }
+                if (pt == 0 && s == 0) sm.pos[b][0] = -1;
+                asm volatile("cp.async.commit_group;" ::: "memory");
+            };
+            auto put = [&](const int r, const float (&p)[DIM], const int i) {
+#pragma unroll
+                for (int d = 0; d < DIM; ++d) sm.ring[d][r & (MF_RING - 1)] = p[d];
+                if (r < cap) {
+                    store_row<DIM>(dst, r, p);
+                    dpos[r] = i;
+                }
+            };
+            // joining edit e, right before old row j (or at the end)
+            auto join = [&](const int e, const int j) {
+                float p[DIM];
+                load_row<DIM>(sm.joins, e, p);
+                put(j - e + 2 * sm.ins[e], p, sm.ed[e] & ~EDIT_IN);
+            };
+            load(s0);
+            load(s0 + 1);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+            named_bar_sync(1, MF_PROD);   // chunk s0 is here
+            for (int s = s0; s <= s1; ++s) {
+                if (s < s1) {
+                    load(s + 2);
+                    const int e0 = sm.cut[s - s0], e1 = sm.cut[s - s0 + 1];
+                    const int last = min(n_old, (s + 1) * MF_ROWS) - 1;
+                    const int j = s * MF_ROWS + pt, b3 = s % MF_STAGES;
+                    if (j <= last) {
+                        float q[DIM];
+                        load_row<DIM>(sm.old[b3], pt, q);
+                        if (ne == 0) {
+#pragma unroll
+                            for (int d = 0; d < DIM; ++d) sm.ring[d][j & (MF_RING - 1)] = q[d];
+                        } else {
+                            const int x = sm.pos[b3][pt + 1];
+                            if (e0 == e1) {
+                                put(j + 2 * sm.ins[e0] - e0, q, x);
+                            } else {
+                                const int xp = sm.pos[b3][pt];
+                                const int b = edits_below(sm.ed, e0, e1, x);   // before this row
+                                for (int e = b - 1; e >= e0 && (sm.ed[e] & ~EDIT_IN) > xp; --e) join(e, j);
+                                const bool leaves = b < e1 && (sm.ed[b] & ~EDIT_IN) == x;
+                                if (!leaves) put(j - b + 2 * sm.ins[b], q, x);
+                                if (j == last)   // and those before the next chunk's first row
+                                    for (int e = b + (leaves ? 1 : 0); e < e1; ++e) join(e, j + 1);
+                            }
+                        }
+                    }
+                    if (n_old == 0)
+                        for (int e = pt; e < ne; e += MF_PROD) join(e, 0);
+                    asm volatile("cp.async.wait_group 1;" ::: "memory");   // chunk s + 1 is here
+                }
+                __syncthreads();
+            }
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+        }
+        if (s1 == steps) break;
+        __syncthreads();   // cut is looked up anew
+    }
+    if (seg) {
+        const float* rows = (ne > 0) ? v.Lr[par ^ 1] + at * DP : src;
+        __syncthreads();  // the ring is read no more
+        fold_long_list<DIM>(rows, n_new, sm.seg);
+        if (warp == 0 && lane < DIM) sum = sm.seg.out[lane];
+    }
+    if (warp == 0) {
+        if (lane == 0) {
+            v.ecnt[slot] = 0;
+            v.cnt[slot] = n_new;
+            if (fresh) v.par[slot] = 0;
+            else if (ne > 0) v.par[slot] = par ^ 1;
+            if (n_new > cap) v.rebnext[c] = 1;
+        }
+        if (n_new > 0) apply_shift<DIM>(v, c, cd, k, n_new, sum, lane);
+    }
+}
+
+// with_control: the last CTA to finish runs the control step of k_control (the
+// moved flags of every fold are then complete) and, when that leaves no group
+// to decimate, the loop condition, so that k_decimate has nothing to wait for
+template <int DIM>
+__global__ void __launch_bounds__(MF_BLOCK, 4) k_merge_fold(EngineView v, cudaGraphConditionalHandle h,
+                                                            int with_control, int use_handle)
+{
+    pdl_enter();
+    __shared__ __align__(16) MergeSmem<DIM> sm;
+    __shared__ int s_last;
+    const int nd = v.ctr[CTR_NDIRTY];
+    for (int t = blockIdx.x; t < nd; t += gridDim.x)
+        merge_fold_key<DIM>(v, v.dlist[t], nd <= (int)gridDim.x, sm);
+    if (!with_control) return;
+    // every thread's writes (chosen points, moved flags) before the count
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) s_last = atomicAdd(&v.ctr[CTR_SUM_DONE], 1) == (int)gridDim.x - 1;
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    control_clouds(v, threadIdx.x, blockDim.x);
+    __threadfence();
+    __syncthreads();
+    const bool idle = *reinterpret_cast<volatile int32_t*>(&v.ctr[CTR_NREADY]) == 0;
+    if (threadIdx.x == 0) {
+        v.ctr[CTR_SUM_DONE] = 0;
+        v.ctr[CTR_COND_DONE] = idle ? 1 : 0;
+    }
+    if (idle) loop_condition(v, h, use_handle, 1);
 }
 
 // ---------------------------------------------------------------------------
@@ -1926,6 +2334,9 @@ __device__ void control_clouds(const EngineView& v, const int first, const int s
             conv = true;
         }
         v.cont[c] = 0;
+        v.full[c] = 0;
+        v.reb[c] = v.rebnext[c];
+        v.rebnext[c] = 0;
         if (conv && (v.flags & ENG_EVOLVE_ONLY)) {
             v.phase[c] = PH_DONE;
         } else if (conv) {
@@ -2093,6 +2504,7 @@ __device__ void decimate_group(const EngineView& v, const int g)
         const int c = gd.cloud_begin + i;
         v.outer[c] += 1;
         v.passes[c] = 0;
+        v.full[c] = 1;   // the chosen points have new indices
         if (stable) {
             v.phase[c] = PH_DONE;
         } else if (v.outer[c] >= v.max_outer) {
@@ -2369,6 +2781,7 @@ __global__ void __launch_bounds__(BLOCK) k_decimate(EngineView v, cudaGraphCondi
     pdl_enter();
     __shared__ int s_last;
     const int nready = v.ctr[CTR_NREADY];
+    if (v.ctr[CTR_COND_DONE]) return;   // nothing ready: k_merge_fold ended the iteration
     for (int r = blockIdx.x; r < nready; r += gridDim.x) decimate_group<DIM, BLOCK>(v, v.ready[r]);
     if (!with_cond) return;
     __threadfence();
@@ -2462,7 +2875,7 @@ __device__ void loop_condition(const EngineView& v, cudaGraphConditionalHandle h
         v.ctr[CTR_NACT] = nact;
         v.ctr[CTR_WORK] = 0;
         v.ctr[CTR_NREADY] = 0;
-        v.ctr[CTR_NBIG] = 0;
+        v.ctr[CTR_NDIRTY] = 0;
         v.ctr[CTR_TILE_HEAVY] = 0;
         const int it = v.ctr[CTR_ITERS] + (count_iter ? 1 : 0);
         v.ctr[CTR_ITERS] = it;
@@ -2500,6 +2913,11 @@ __global__ void k_reset(EngineView v)
     if (c < v.n_groups) v.group_conv[c] = 0;
     if (c >= v.n_clouds) return;
     v.kbdone[c] = 0;
+    v.full[c] = 1;
+    v.reb[c] = 0;
+    v.rebnext[c] = 0;
+    v.mvn[c] = 0;
+    v.dmax[c] = 0;
     v.cont[c] = 0;
     v.passes[c] = 0;
     v.total_passes[c] = 0;
@@ -2515,7 +2933,7 @@ cudaError_t set_assign_attrs(int dyn)
                                 cudaFuncAttributeMaxDynamicSharedMemorySize, dyn);
 }
 
-// persistent grid of k_assign_cull: every resident CTA, at most one per item
+// persistent grid of k_assign_cull: every resident CTA, at most one warp per block
 template <int DIM, int ITEMS>
 cudaError_t launch_assign_cull(const EngineView& v, cudaStream_t st)
 {
@@ -2527,12 +2945,27 @@ cudaError_t launch_assign_cull(const EngineView& v, cudaStream_t st)
             b = 1;
         per_sm.store(b, std::memory_order_relaxed);
     }
-    const int subs = (v.chunk_pts + AC_BLOCK * ITEMS - 1) / (AC_BLOCK * ITEMS);
-    if (subs & (subs - 1)) return cudaErrorInvalidValue;  // the kernel's block bounds need 2^k
-    const int64_t items = (int64_t)v.n_chunks * subs;
-    const int g = (int)std::max<int64_t>(1, std::min<int64_t>(items, (int64_t)v.n_sms * b));
+    const int wpc = v.chunk_pts / (32 * ITEMS);
+    if (wpc < 1 || (wpc & (wpc - 1))) return cudaErrorInvalidValue;  // the kernel's block numbers need 2^k
+    const int64_t ctas = ((int64_t)v.n_chunks * wpc + AC_WARPS - 1) / AC_WARPS;
+    const int g = (int)std::max<int64_t>(1, std::min<int64_t>(ctas, (int64_t)v.n_sms * b));
     k_assign_cull<DIM, ITEMS><<<g, AC_BLOCK, 0, st>>>(v);
     return cudaGetLastError();
+}
+
+// grid of k_merge_fold: every resident CTA, at most one per chosen point
+template <int DIM>
+int merge_grid(const EngineView& v)
+{
+    static std::atomic<int> per_sm{0};
+    int b = per_sm.load(std::memory_order_relaxed);
+    if (b == 0) {
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_merge_fold<DIM>, MF_BLOCK, 0) !=
+                cudaSuccess || b < 1)
+            b = 1;
+        per_sm.store(b, std::memory_order_relaxed);
+    }
+    return (int)std::max<int64_t>(1, std::min<int64_t>(v.n_slots, (int64_t)v.n_sms * b));
 }
 
 template <int DIM>
@@ -2617,11 +3050,8 @@ cudaError_t launch_pass_dim(const EngineView& v, const TuneParams& tp, int assig
                        scatter_cta_smem_bytes(v), st, v);
     if (e != cudaSuccess) return e;
     if (v.n_slots > 0) {
-        // at most (points / SUM_BIG_MIN) keys can be big
-        const int big_ctas = (int)std::min<int64_t>(
-            ((int64_t)v.n_chunks * v.chunk_pts + SUM_BIG_MIN - 1) / SUM_BIG_MIN, sms);
-        e = launch_pdl(pdl, k_sum_shift<DIM>, big_ctas + std::min((v.n_slots + 7) / 8, sms * 8), 256, 0,
-                       st, v, big_ctas, 1);
+        e = launch_pdl(pdl, k_merge_fold<DIM>, merge_grid<DIM>(v), MF_BLOCK, 0, st, v, lc.h, 1,
+                       lc.use_handle);
     } else {
         e = launch_pdl(pdl, k_control, std::min((v.n_clouds + 255) / 256, sms), 256, 0, st, v);
     }
@@ -2900,10 +3330,7 @@ cudaError_t launch_evolve_step_dim(const EngineView& v, const TuneParams& tp, in
     if (v.n_chunks > 0)
         k_scatter_cta<DIM><<<std::min(v.n_chunks, sms * 8), SCAT_W * 32, scatter_cta_smem_bytes(v), st>>>(v);
     if (v.n_slots > 0) {
-        // at most (points / SUM_BIG_MIN) keys can be big
-        const int big_ctas = (int)std::min<int64_t>(
-            ((int64_t)v.n_chunks * v.chunk_pts + SUM_BIG_MIN - 1) / SUM_BIG_MIN, sms);
-        k_sum_shift<DIM><<<big_ctas + std::min((v.n_slots + 7) / 8, sms * 8), 256, 0, st>>>(v, big_ctas, 0);
+        k_merge_fold<DIM><<<merge_grid<DIM>(v), MF_BLOCK, 0, st>>>(v, 0, 0, 0);
     }
     return cudaGetLastError();
 }

@@ -81,29 +81,109 @@ __global__ void __launch_bounds__(256) k_morton(EngineView v, uint64_t* key, int
             for (int d = 0; d < DIM; ++d) p[d] = v.P[s * DIM + d];
             key[s] = ((uint64_t)(uint32_t)c << 32) | morton_code<DIM>(p, inv);
             val[s] = (int32_t)s;
+            v.keys[s] = -1;   // no point has a key before the first pass
         }
     }
 }
 
-// Ps, sorder, and (second half of sorder) each position's histogram row: the
-// chunk of its slot inside its cloud, from the sorted keys' cloud field
+// Ps, sorder, (second half of sorder) each position's histogram row -- the
+// chunk of its slot inside its cloud -- and the two bounding boxes of every
+// block of 32 x items positions of a cloud, one warp per block: the order is
+// cut where consecutive points are furthest apart, which is where it leaves one
+// occupied place for another (a block over such a jump as one box would span
+// the space between, and the culled assignment would look at every chosen
+// point there: on the 1M helix a handful of such blocks took 50 us each, as
+// long as all the others together).  A part without points has an empty box.
 template <int DIM>
-__global__ void __launch_bounds__(256) k_gather_spatial(EngineView v, int64_t n, const int32_t* val,
-                                                        const uint64_t* key, float* Ps,
-                                                        int32_t* sorder)
+__global__ void __launch_bounds__(256) k_gather_spatial(EngineView v, int items, int64_t n,
+                                                        const int32_t* val, float* Ps,
+                                                        int32_t* sorder, float* bbox)
 {
     constexpr int DP = PadDim<DIM>::v;
-    for (int64_t pos = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; pos < n;
-         pos += (int64_t)gridDim.x * blockDim.x) {
-        const int32_t s = val[pos];
-        const CloudDesc cd = v.cl[(int)(key[pos] >> 32)];
-        sorder[n + pos] = slot_chunk((int)(s - cd.p_off), cd.n_all, cd.n_chunks,
-                                     (float)cd.n_chunks / (float)cd.n_all);
+    const int lane = threadIdx.x & 31;
+    const int wpc = v.chunk_pts / (32 * items);
+    const int64_t blocks = (int64_t)v.n_chunks * wpc;
+    for (int64_t wb = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5); wb < blocks;
+         wb += (int64_t)gridDim.x * 8) {
+        const int chunk = (int)(wb / wpc);
+        const CloudDesc cd = v.cl[v.chunk_cloud[chunk]];
+        const int64_t i0 = ((chunk - cd.chunk_begin) * wpc + wb % wpc) * 32 * items;
+        const float ratio = (float)cd.n_chunks / (float)cd.n_all;
+        float far = -1.0f;      // longest step of this lane's points from their predecessors
+        int cut = 0;            // and the position it leads to
+        float last[DIM];        // the previous row's last point
+        for (int j = 0; j < items; ++j) {
+            const int64_t i = i0 + j * 32 + lane;
+            const bool in = i < cd.n_all;
+            float x[DIM], step = 0.0f;
+            const int64_t pos = cd.p_off + i;
+            const int32_t s = in ? val[pos] : 0;
+            if (in) {
+                sorder[n + pos] = slot_chunk((int)(s - cd.p_off), cd.n_all, cd.n_chunks, ratio);
+                sorder[pos] = s;
+                v.ksp[pos] = -1;
+            }
 #pragma unroll
-        for (int d = 0; d < DIM; ++d) Ps[pos * DP + d] = v.P[(int64_t)s * DIM + d];
+            for (int d = 0; d < DIM; ++d) {
+                x[d] = in ? v.P[(int64_t)s * DIM + d] : 0.0f;
+                if (in) Ps[pos * DP + d] = x[d];
+                float prev = __shfl_up_sync(0xffffffffu, x[d], 1);
+                if (lane == 0) prev = (j > 0) ? last[d] : x[d];
+                step = fmaxf(step, fabsf(x[d] - prev));
+                last[d] = __shfl_sync(0xffffffffu, x[d], 31);
+            }
+            if (in)
 #pragma unroll
-        for (int d = DIM; d < DP; ++d) Ps[pos * DP + d] = 0.0f;
-        sorder[pos] = s;
+                for (int d = DIM; d < DP; ++d) Ps[pos * DP + d] = 0.0f;
+            if (in && step > far) {
+                far = step;
+                cut = j * 32 + lane;
+            }
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const float f = __shfl_xor_sync(0xffffffffu, far, o);
+            const int q = __shfl_xor_sync(0xffffffffu, cut, o);
+            if (f > far || (f == far && q < cut)) {
+                far = f;
+                cut = q;
+            }
+        }
+        float lo[2][DIM], hi[2][DIM];
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int d = 0; d < DIM; ++d) {
+                lo[h][d] = INFINITY;
+                hi[h][d] = -INFINITY;
+            }
+        for (int j = 0; j < items; ++j) {
+            const int64_t i = i0 + j * 32 + lane;
+            if (i >= cd.n_all) break;
+            const bool second = j * 32 + lane >= cut;
+#pragma unroll
+            for (int d = 0; d < DIM; ++d) {
+                const float x = Ps[(cd.p_off + i) * DP + d];   // this lane's own writes
+                lo[0][d] = fminf(lo[0][d], second ? INFINITY : x);
+                hi[0][d] = fmaxf(hi[0][d], second ? -INFINITY : x);
+                lo[1][d] = fminf(lo[1][d], second ? x : INFINITY);
+                hi[1][d] = fmaxf(hi[1][d], second ? x : -INFINITY);
+            }
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int d = 0; d < DIM; ++d) {
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) {
+                    lo[h][d] = fminf(lo[h][d], __shfl_xor_sync(0xffffffffu, lo[h][d], o));
+                    hi[h][d] = fmaxf(hi[h][d], __shfl_xor_sync(0xffffffffu, hi[h][d], o));
+                }
+                if (lane == 0) {
+                    bbox[(wb * 2 + h) * 2 * DIM + d] = lo[h][d];
+                    bbox[(wb * 2 + h) * 2 * DIM + DIM + d] = hi[h][d];
+                }
+            }
     }
 }
 
@@ -119,8 +199,9 @@ size_t sort_temp_bytes(int64_t n)
 size_t align256(size_t x) { return (x + 255) / 256 * 256; }
 
 template <int DIM>
-cudaError_t spatial_prep_dim(const EngineView& v, int64_t n, void* scratch, size_t scratch_bytes,
-                             float* Ps, int32_t* sorder, cudaStream_t st)
+cudaError_t spatial_prep_dim(const EngineView& v, int items, int64_t n, void* scratch,
+                             size_t scratch_bytes, float* Ps, int32_t* sorder, float* bbox,
+                             cudaStream_t st)
 {
     if (n <= 0 || v.n_chunks <= 0) return cudaSuccess;
     unsigned char* p = static_cast<unsigned char*>(scratch);
@@ -141,8 +222,9 @@ cudaError_t spatial_prep_dim(const EngineView& v, int64_t n, void* scratch, size
     cub::DoubleBuffer<int32_t> vb(v0, v1);
     cudaError_t e = cub::DeviceRadixSort::SortPairs(tmp, tmp_bytes, kb, vb, (int)n, 0, end_bit, st);
     if (e != cudaSuccess) return e;
-    const int ggrid = (int)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, (int64_t)sms * 16));
-    k_gather_spatial<DIM><<<ggrid, 256, 0, st>>>(v, n, vb.Current(), kb.Current(), Ps, sorder);
+    const int64_t blocks = (int64_t)v.n_chunks * (v.chunk_pts / (32 * items));
+    const int ggrid = (int)std::max<int64_t>(1, std::min<int64_t>((blocks + 7) / 8, (int64_t)sms * 16));
+    k_gather_spatial<DIM><<<ggrid, 256, 0, st>>>(v, items, n, vb.Current(), Ps, sorder, bbox);
     return cudaGetLastError();
 }
 
@@ -154,16 +236,14 @@ size_t spatial_prep_scratch_bytes(int64_t n)
     return 2 * align256(8 * (size_t)n) + 2 * align256(4 * (size_t)n) + align256(sort_temp_bytes(n));
 }
 
-cudaError_t launch_spatial_prep(int dim, const EngineView& v, int64_t n, void* scratch,
-                                size_t scratch_bytes, float* Ps, int32_t* sorder, cudaStream_t st)
+cudaError_t launch_spatial_prep(int dim, const EngineView& v, int items, int64_t n, void* scratch,
+                                size_t scratch_bytes, float* Ps, int32_t* sorder, float* bbox,
+                                cudaStream_t st)
 {
-    switch (dim) {
-        case 1: return spatial_prep_dim<1>(v, n, scratch, scratch_bytes, Ps, sorder, st);
-        case 2: return spatial_prep_dim<2>(v, n, scratch, scratch_bytes, Ps, sorder, st);
-        case 3: return spatial_prep_dim<3>(v, n, scratch, scratch_bytes, Ps, sorder, st);
-        case 4: return spatial_prep_dim<4>(v, n, scratch, scratch_bytes, Ps, sorder, st);
-        default: return cudaErrorInvalidValue;
-    }
+    return with_dim(dim, [&](auto D) {
+        return spatial_prep_dim<decltype(D)::value>(v, items, n, scratch, scratch_bytes, Ps, sorder,
+                                                    bbox, st);
+    });
 }
 
 }  // namespace rdb

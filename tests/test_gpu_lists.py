@@ -1,0 +1,72 @@
+"""Member lists kept across passes (k_assign_cull's edits, k_merge_fold) against the
+all-pairs assignment, which regroups every point in every pass: bit for bit,
+where lists are longest, shortest, outgrow their regions, or take more edits than
+they hold."""
+import numpy as np
+import pytest
+
+from gpu_util import bits_equal, require_cuda
+from ridgedetection_b200 import generators as G
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def rdb():
+    require_cuda()
+    import ridgedetection_b200 as rdb
+    yield rdb
+    rdb.set_assign_cull(True)
+
+
+def _blob(n, dim, sigma, seed):
+    return np.random.default_rng(seed).normal(0.0, sigma, (n, dim)).astype(np.float32)
+
+
+def _steep(n, seed):
+    """Density rising steeply along x: chosen points travel and their clusters grow."""
+    x = np.random.default_rng(seed).random((n, 2))
+    return np.stack([8.0 * x[:, 0] ** 0.2, 0.1 * x[:, 1]], 1).astype(np.float32)
+
+
+CASES = {
+    # lists of more chunks than are looked up at once, folded in segments
+    "two_huge": (lambda: _blob(150_000, 2, 0.2, 1), 0.9),
+    # a long list below the segment threshold, one row around a chunk's end
+    "chunk_end": (lambda: _blob(4 * 224 + 1, 3, 0.01, 2), 0.5),
+    # more chosen points than the one-CTA scatter takes, lists of a few points
+    "many_keys": (lambda: _blob(6_000, 2, 1.0, 3), 0.02),
+    # clusters that grow past the room they were given
+    "steep": (lambda: _steep(30_000, 4), 0.35),
+    # more edits per key than are taken (early passes of a dense curve)
+    "helix": (lambda: G.helix3d(120_000, seed=5), 0.15),
+    "line": (lambda: _blob(5_000, 1, 1.0, 6), 0.1),
+    "four_dims": (lambda: _blob(20_000, 4, 0.5, 7), 0.4),
+}
+
+
+@pytest.mark.parametrize("name", list(CASES))
+def test_lists_match_all_pairs(rdb, name):
+    gen, r1 = CASES[name]
+    P = gen()
+    rdb.set_assign_cull(False)
+    try:
+        S_ref, st_ref = rdb.ridge_detection(P, r1, 2.0 * r1)
+    finally:
+        rdb.set_assign_cull(True)
+    for mode in (rdb.LOOP_GRAPH, rdb.LOOP_HOST):
+        S, st = rdb.ridge_detection(P, r1, 2.0 * r1, loop_mode=mode)
+        assert st.err_bits == 0 and st.evolve_passes == st_ref.evolve_passes
+        assert bits_equal(S, S_ref)
+
+
+def test_lists_in_a_batch(rdb):
+    clouds = [(gen(), r1, 2.0 * r1) for gen, r1 in CASES.values()]
+    packed, descs = rdb.pack_clouds(clouds)
+    b = rdb.BatchedRidgeDetection()
+    for _ in range(2):   # the second run takes over the first one's buffers
+        b.run(packed, descs)
+        for c, (P, r1, r2) in enumerate(clouds):
+            S, _ = rdb.ridge_detection(P, r1, r2)
+            assert bits_equal(b.chosen_points(c), S), c
+    b.close()
