@@ -422,6 +422,10 @@ RD_API rd_status rd_evolve_adjoint(int dim, const float* P, int64_t np, const fl
                                    int64_t ns, float r1, int iters, int checkpoint_every,
                                    const double* W, float* S_final, double* grad_P,
                                    double* grad_S0, int on_device, void* stream);
+/* The forward of rd_evolve_adjoint alone (device pointers): S_final after
+ * `iters` passes from S0. */
+RD_API rd_status rd_evolve_means(int dim, const float* d_P, int64_t np, const float* d_S0,
+                                 int64_t ns, float r1, int iters, float* d_S_final, void* stream);
 
 #ifdef __cplusplus
 }

@@ -59,6 +59,19 @@ def evolve_adjoint_device(P, S0, r1: float, iters: int, W, checkpoint_every: int
     return Sf, gP, gS
 
 
+def evolve_means_device(P, S0, r1: float, iters: int):
+    """The forward of :func:`evolve_adjoint_device` alone: S_final."""
+    import torch
+    P, S0 = P.contiguous(), S0.contiguous()
+    Sf = torch.empty_like(S0)
+    vp = ctypes.c_void_p
+    st = vp(torch.cuda.current_stream(P.device).cuda_stream)
+    L.check(L.lib().rd_evolve_means(int(P.shape[1]), vp(P.data_ptr()), int(P.shape[0]),
+                                    vp(S0.data_ptr()), int(S0.shape[0]), float(r1), int(iters),
+                                    vp(Sf.data_ptr()), st))
+    return Sf
+
+
 def _autograd_function():
     import torch
 
@@ -68,8 +81,7 @@ def _autograd_function():
         @staticmethod
         def forward(ctx, P, chosen_idx, r1, iters, checkpoint_every=0):
             S0 = P.detach()[chosen_idx].contiguous()
-            W0 = torch.zeros(S0.shape, dtype=torch.float64, device=P.device)
-            Sf, _, _ = evolve_adjoint_device(P.detach(), S0, r1, iters, W0, checkpoint_every)
+            Sf = evolve_means_device(P.detach(), S0, r1, iters)
             ctx.save_for_backward(P.detach(), chosen_idx)
             ctx.r1, ctx.iters, ctx.ckpt = r1, iters, checkpoint_every
             return Sf

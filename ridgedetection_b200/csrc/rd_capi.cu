@@ -1166,6 +1166,21 @@ rd_status rd_decimate_noalloc(int dim, float* d_S, int64_t ns, float r2, int32_t
 // ------------------------------------------------------------------------
 // evolve adjoint
 // ------------------------------------------------------------------------
+}  // extern "C"
+namespace {
+struct AdjState {
+    AdjointRunner runner;
+    DevBuf dP, dS0, dW, dSf, dgP, dgS;
+};
+// per thread, never destroyed: no CUDA calls during process exit
+AdjState& adj_state()
+{
+    thread_local AdjState& as = *new AdjState();
+    return as;
+}
+}  // namespace
+extern "C" {
+
 rd_status rd_evolve_adjoint(int dim, const float* P, int64_t np, const float* S0, int64_t ns,
                             float r1, int iters, int checkpoint_every, const double* W,
                             float* S_final, double* grad_P, double* grad_S0, int on_device,
@@ -1177,12 +1192,7 @@ rd_status rd_evolve_adjoint(int dim, const float* P, int64_t np, const float* S0
         return set_err(RD_ERR_ARG, "np/ns out of range");
     if (iters < 0 || checkpoint_every < 0) return set_err(RD_ERR_ARG, "bad iteration counts");
     if (!(r1 > 0.0f)) return set_err(RD_ERR_ARG, "r1 must be > 0");
-    // per-thread state, never destroyed: no CUDA calls during process exit
-    struct AdjState {
-        AdjointRunner runner;
-        DevBuf dP, dS0, dW, dSf, dgP, dgS;
-    };
-    thread_local AdjState& as = *new AdjState();
+    AdjState& as = adj_state();
     AdjointRunner& runner = as.runner;
     DevBuf &dP = as.dP, &dS0 = as.dS0, &dW = as.dW, &dSf = as.dSf, &dgP = as.dgP, &dgS = as.dgS;
     cudaStream_t st = (cudaStream_t)stream;
@@ -1219,6 +1229,22 @@ rd_status rd_evolve_adjoint(int dim, const float* P, int64_t np, const float* S0
             CK_CUDA(cudaMemcpyAsync(grad_S0, pgS, sizeof(double) * ns * dim, cudaMemcpyDeviceToHost, st));
         CK_CUDA(cudaStreamSynchronize(st));
     }
+    return RD_OK;
+}
+
+rd_status rd_evolve_means(int dim, const float* d_P, int64_t np, const float* d_S0, int64_t ns,
+                          float r1, int iters, float* d_S_final, void* stream)
+{
+    if (!dim_ok(dim)) return set_err(RD_ERR_UNSUPPORTED, "dim must be 1 to 4");
+    if (!d_P || !d_S0 || !d_S_final) return set_err(RD_ERR_ARG, "null argument");
+    if (np < 1 || np > INT32_MAX - 1024 || ns < 1 || ns > np)
+        return set_err(RD_ERR_ARG, "np/ns out of range");
+    if (iters < 0) return set_err(RD_ERR_ARG, "bad iteration count");
+    if (!(r1 > 0.0f)) return set_err(RD_ERR_ARG, "r1 must be > 0");
+    AdjointRunner& runner = adj_state().runner;
+    const int rc = runner.run(dim, d_P, np, d_S0, ns, r1, iters, 0, nullptr, d_S_final, nullptr,
+                              nullptr, (cudaStream_t)stream);
+    if (rc) return set_err((rd_status)rc, runner.last_error);
     return RD_OK;
 }
 

@@ -575,18 +575,7 @@ int Engine::run(cudaStream_t st, bool use_graph, int mode)
     fused_ = fuse_tiles && h_gr_.size() == 1 && h_cl_.size() > 1 && max_ns <= TILE_NS_MAX &&
              flags_ == 0;
     cull_ = cull_possible() && !fused_;
-    if (cull_) {
-        if (int rc = ensure_cull_buffers()) return rc;
-        const EngineView vs = view();
-        RD_CK(launch_spatial_prep(dim_, vs, tune.cull_items, total_points_, bSpatialTmp_.p,
-                                  spatial_prep_scratch_bytes(total_points_), bPs_.as<float>(),
-                                  bSorder_.as<int32_t>(), bBox_.as<float>(), st));
-        // no point has a key yet: the culled assignment keeps the counts by its
-        // changes
-        RD_CK(cudaMemsetAsync(bHist_.p, 0, 4 * (size_t)(hist_ints_ + 1), st));
-    } else {
-        RD_CK(bPg_.ensure(sizeof(float) * (size_t)(total_points_ * pad_dim(dim_) + 4)));
-    }
+    if (int rc = start_passes(st)) return rc;
     tile_cl_grid_ = 0;
     if (fused_) RD_CK(prepare_tile_pass(dim_, view(), &tile_cl_grid_));
     const EngineView v = view();
@@ -628,6 +617,24 @@ int Engine::run(cudaStream_t st, bool use_graph, int mode)
         if (a1) cudaEventDestroy(a1);
     }
     return collect(st);
+}
+
+// buffers and state of the lockstep passes (cull_ is set)
+int Engine::start_passes(cudaStream_t st)
+{
+    if (cull_) {
+        if (int rc = ensure_cull_buffers()) return rc;
+        const EngineView vs = view();
+        RD_CK(launch_spatial_prep(dim_, vs, tune.cull_items, total_points_, bSpatialTmp_.p,
+                                  spatial_prep_scratch_bytes(total_points_), bPs_.as<float>(),
+                                  bSorder_.as<int32_t>(), bBox_.as<float>(), st));
+        // no point has a key yet: the culled assignment keeps the counts by its
+        // changes
+        RD_CK(cudaMemsetAsync(bHist_.p, 0, 4 * (size_t)(hist_ints_ + 1), st));
+    } else {
+        RD_CK(bPg_.ensure(sizeof(float) * (size_t)(total_points_ * pad_dim(dim_) + 4)));
+    }
+    return 0;
 }
 
 // whether the lockstep passes of this batch assign with culling
@@ -725,26 +732,34 @@ int Engine::adjoint_setup(cudaStream_t st)
     }
     stats_ = RunStats();
     flags_ = ENG_ALWAYS_MOVE;
-    cull_ = false;
-    cull_allowed_ = false;
-    RD_CK(bPg_.ensure(sizeof(float) * (size_t)(total_points_ * pad_dim(dim_) + 4)));
+    fused_ = false;
+    cull_ = cull_possible();
     RD_CK(upload(bCl_, h_cl_, st));
     RD_CK(upload(bGr_, h_gr_, st));
     EngineView v0 = view();
     RD_CK(launch_reset(v0, st));
     RD_CK(cudaMemcpyAsync(bNs_.p, given_ns.data(), 4, cudaMemcpyHostToDevice, st));
+    RD_CK(upload(bChunkCloud_, h_chunk_cloud_, st));
     if (int rc = finish_setup_after_choose(st)) return rc;
+    if (int rc = start_passes(st)) return rc;
     const EngineView v = view();
     RD_CK(launch_set_given(v, 0, st));
     RD_CK(prepare_pass(dim_, v, tune));
+    RD_CK(launch_loopcond(v, cudaGraphConditionalHandle(), 0, st, 0));  // work lists and tickets
     return 0;
 }
 
 int Engine::adjoint_step(cudaStream_t st)
 {
     const EngineView v = view();
-    RD_CK(launch_loopcond(v, cudaGraphConditionalHandle(), 0, st, 0));  // lists + ticket
     RD_CK(launch_evolve_step(dim_, v, tune, assign_grid_, st));
+    return 0;
+}
+
+int Engine::adjoint_restart(cudaStream_t st)
+{
+    // any value but 0: the next pass evaluates and regroups everything
+    RD_CK(cudaMemsetAsync(bFull_.p, 1, sizeof(int32_t), st));
     return 0;
 }
 

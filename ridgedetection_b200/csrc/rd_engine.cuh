@@ -256,7 +256,8 @@ size_t spatial_prep_scratch_bytes(int64_t n_points);
 cudaError_t launch_spatial_prep(int dim, const EngineView& v, int items, int64_t n_points,
                                 void* scratch, size_t scratch_bytes, float* Ps, int32_t* sorder,
                                 float* bbox, cudaStream_t st);
-// the five kernels of one evolve pass without control/decimation (adjoint forward)
+// the kernels of one evolve pass without control and decimation (adjoint
+// forward), again and again over the work lists of one launch_loopcond
 cudaError_t launch_evolve_step(int dim, const EngineView& v, const TuneParams& tp, int assign_grid,
                                cudaStream_t st);
 int assign_smem_bytes(int dim, const TuneParams& tp, int hist_ints);

@@ -121,6 +121,8 @@ public:
     // movement test (rd_adjoint.cu); keys()/counts() then hold that pass
     int adjoint_setup(cudaStream_t st);
     int adjoint_step(cudaStream_t st);
+    // before the step that follows a change of the chosen points by the caller
+    int adjoint_restart(cudaStream_t st);
     const int32_t* keys() const { return bKeys_.as<int32_t>(); }
     const int32_t* counts() const { return bCnt_.as<int32_t>(); }
 
@@ -148,6 +150,7 @@ private:
     int finish_setup_after_choose(cudaStream_t st);
     bool cull_possible() const;
     int ensure_cull_buffers();
+    int start_passes(cudaStream_t st);
     void build_tile_order();
     int collect(cudaStream_t st);
     int flags_ = 0;

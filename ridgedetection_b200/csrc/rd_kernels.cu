@@ -1684,6 +1684,14 @@ struct MergeSmem {
     int cut[MF_CUTS + 1];     // edits before the first row of each chunk
 };
 
+// cloud c after a pass: the next one evaluates and regroups what this one left
+__device__ __forceinline__ void next_pass(const EngineView& v, const int c)
+{
+    v.full[c] = 0;
+    v.reb[c] = v.rebnext[c];
+    v.rebnext[c] = 0;
+}
+
 // the per-cloud control step after a pass (k_control), over clouds first,
 // first + stride, ... of the active list
 __device__ void control_clouds(const EngineView& v, const int first, const int stride);
@@ -1957,12 +1965,16 @@ __device__ void merge_fold_key(const EngineView& v, const int slot, const bool s
     }
 }
 
-// with_control: the last CTA to finish runs the control step of k_control (the
-// moved flags of every fold are then complete) and, when that leaves no group
-// to decimate, the loop condition, so that k_decimate has nothing to wait for
+// control: what the last CTA to finish does.  MF_CONTROL: the control step of
+// k_control (the moved flags of every fold are then complete) and, when that
+// leaves no group to decimate, the loop condition, so that k_decimate has
+// nothing to wait for.  MF_STEP (passes whose number the caller sets, over the
+// same clouds): make ready for the next pass.
+enum : int { MF_CONTROL = 1, MF_STEP = 2 };
+
 template <int DIM>
 __global__ void __launch_bounds__(MF_BLOCK, 4) k_merge_fold(EngineView v, cudaGraphConditionalHandle h,
-                                                            int with_control, int use_handle)
+                                                            int control, int use_handle)
 {
     pdl_enter();
     __shared__ __align__(16) MergeSmem<DIM> sm;
@@ -1970,7 +1982,6 @@ __global__ void __launch_bounds__(MF_BLOCK, 4) k_merge_fold(EngineView v, cudaGr
     const int nd = v.ctr[CTR_NDIRTY];
     for (int t = blockIdx.x; t < nd; t += gridDim.x)
         merge_fold_key<DIM>(v, v.dlist[t], nd <= (int)gridDim.x, sm);
-    if (!with_control) return;
     // every thread's writes (chosen points, moved flags) before the count
     __threadfence();
     __syncthreads();
@@ -1978,6 +1989,16 @@ __global__ void __launch_bounds__(MF_BLOCK, 4) k_merge_fold(EngineView v, cudaGr
     __syncthreads();
     if (!s_last) return;
     __threadfence();
+    if (control == MF_STEP) {
+        const int nact = v.ctr[CTR_NACT];
+        for (int a = threadIdx.x; a < nact; a += blockDim.x) next_pass(v, v.act_cloud[a]);
+        if (threadIdx.x == 0) {
+            v.ctr[CTR_SUM_DONE] = 0;
+            v.ctr[CTR_NDIRTY] = 0;
+            v.ctr[CTR_WORK] = 0;
+        }
+        return;
+    }
     control_clouds(v, threadIdx.x, blockDim.x);
     __threadfence();
     __syncthreads();
@@ -2334,9 +2355,7 @@ __device__ void control_clouds(const EngineView& v, const int first, const int s
             conv = true;
         }
         v.cont[c] = 0;
-        v.full[c] = 0;
-        v.reb[c] = v.rebnext[c];
-        v.rebnext[c] = 0;
+        next_pass(v, c);
         if (conv && (v.flags & ENG_EVOLVE_ONLY)) {
             v.phase[c] = PH_DONE;
         } else if (conv) {
@@ -3008,9 +3027,11 @@ static cudaError_t launch_pdl(int pdl, void (*kernel)(KArgs...), int grid, int b
     return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
+// the kernels of an evolve pass; control: see k_merge_fold
 template <int DIM>
-cudaError_t launch_pass_dim(const EngineView& v, const TuneParams& tp, int assign_grid,
-                            const LoopCond& lc, cudaStream_t st, cudaEvent_t a0, cudaEvent_t a1)
+cudaError_t launch_evolve_kernels(const EngineView& v, const TuneParams& tp, int assign_grid,
+                                  const LoopCond& lc, int control, cudaStream_t st,
+                                  cudaEvent_t a0 = nullptr, cudaEvent_t a1 = nullptr)
 {
     const int hist_bytes = v.hist_smem * 4;
     const int sms = v.n_sms;
@@ -3050,14 +3071,24 @@ cudaError_t launch_pass_dim(const EngineView& v, const TuneParams& tp, int assig
                        scatter_cta_smem_bytes(v), st, v);
     if (e != cudaSuccess) return e;
     if (v.n_slots > 0) {
-        e = launch_pdl(pdl, k_merge_fold<DIM>, merge_grid<DIM>(v), MF_BLOCK, 0, st, v, lc.h, 1,
+        e = launch_pdl(pdl, k_merge_fold<DIM>, merge_grid<DIM>(v), MF_BLOCK, 0, st, v, lc.h, control,
                        lc.use_handle);
     } else {
         e = launch_pdl(pdl, k_control, std::min((v.n_clouds + 255) / 256, sms), 256, 0, st, v);
     }
+    return e;
+}
+
+template <int DIM>
+cudaError_t launch_pass_dim(const EngineView& v, const TuneParams& tp, int assign_grid,
+                            const LoopCond& lc, cudaStream_t st, cudaEvent_t a0, cudaEvent_t a1)
+{
+    const int pdl = v.n_clouds == 1;
+    const cudaError_t e =
+        launch_evolve_kernels<DIM>(v, tp, assign_grid, lc, MF_CONTROL, st, a0, a1);
     if (e != cudaSuccess) return e;
-    return launch_pdl(pdl, k_decimate<DIM, 512>, std::min(v.n_groups, sms * 2), 512, dec_smem_bytes(v),
-                      st, v, lc.h, 1, lc.use_handle);
+    return launch_pdl(pdl, k_decimate<DIM, 512>, std::min(v.n_groups, v.n_sms * 2), 512,
+                      dec_smem_bytes(v), st, v, lc.h, 1, lc.use_handle);
 }
 
 template <int DIM>
@@ -3312,34 +3343,11 @@ cudaError_t launch_decimate(int dim, const EngineView& v, cudaStream_t st)
     return cudaGetLastError();
 }
 
-template <int DIM>
-cudaError_t launch_evolve_step_dim(const EngineView& v, const TuneParams& tp, int assign_grid,
-                                   cudaStream_t st)
-{
-    const int hist_bytes = v.hist_smem * 4;
-    const int sms = v.n_sms;
-#define RD_ASSIGN_CASE(B, I) \
-    if (tp.block == B && tp.items == I) k_assign<DIM, B, I><<<assign_grid, B, hist_bytes, st>>>(v); else
-    RD_ASSIGN_CASE(128, 8) RD_ASSIGN_CASE(128, 4) RD_ASSIGN_CASE(256, 4) RD_ASSIGN_CASE(256, 8)
-    RD_ASSIGN_CASE(128, 16)
-    { return cudaErrorInvalidValue; }
-#undef RD_ASSIGN_CASE
-    if (v.n_kblk > 0) k_chunkscan_cta<<<std::min(v.n_kblk, sms * 4), CS_W * 32, 0, st>>>(v);
-    if (v.n_kblk_warp > 0)
-        k_chunkscan_warp<<<std::min((v.n_kblk_warp + CSW_W - 1) / CSW_W, sms * 8), CSW_W * 32, 0, st>>>(v);
-    if (v.n_chunks > 0)
-        k_scatter_cta<DIM><<<std::min(v.n_chunks, sms * 8), SCAT_W * 32, scatter_cta_smem_bytes(v), st>>>(v);
-    if (v.n_slots > 0) {
-        k_merge_fold<DIM><<<merge_grid<DIM>(v), MF_BLOCK, 0, st>>>(v, 0, 0, 0);
-    }
-    return cudaGetLastError();
-}
-
 cudaError_t launch_evolve_step(int dim, const EngineView& v, const TuneParams& tp, int assign_grid,
                                cudaStream_t st)
 {
     return with_dim(dim, [&](auto D) {
-        return launch_evolve_step_dim<decltype(D)::value>(v, tp, assign_grid, st);
+        return launch_evolve_kernels<decltype(D)::value>(v, tp, assign_grid, LoopCond(), MF_STEP, st);
     });
 }
 

@@ -159,3 +159,20 @@ def test_autograd_function(adj):
     _, gP, gS = adj.evolve_adjoint(P, S0, r1, 6, W.double().cpu().numpy())
     np.add.at(gP, chosen_indices(P, S0), gS)
     np.testing.assert_allclose(Pt.grad.cpu().numpy(), gP.astype(np.float32), rtol=1e-6, atol=1e-7)
+
+
+@pytest.mark.parametrize("iters,every", [(0, 0), (1, 5), (5, 5), (6, 5), (12, 5), (12, 0)])
+def test_segments_agree(iters, every):
+    """Checkpointed segments (the last one kept from the forward, the others recomputed) against
+    every pass kept, and the forward alone against the forward of the adjoint: bit for bit."""
+    torch = require_cuda()
+    from ridgedetection_b200 import autograd as adj
+    r = np.random.default_rng(iters)
+    P = torch.from_numpy(G.helix3d(20_000, seed=3)).cuda()
+    S0 = P[:300].clone()
+    W = torch.from_numpy(r.normal(size=(300, 3))).cuda()
+    a = adj.evolve_adjoint_device(P, S0, 0.2, iters, W, every)
+    b = adj.evolve_adjoint_device(P, S0, 0.2, iters, W, 0)
+    for x, y in zip(a, b):
+        assert torch.equal(x, y)
+    assert torch.equal(adj.evolve_means_device(P, S0, 0.2, iters), a[0])
