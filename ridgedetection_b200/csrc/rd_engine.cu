@@ -296,8 +296,7 @@ EngineView Engine::view() const
         v.Lr[b] = cull_ ? bLr_[b].as<float>() : bPg_.as<float>();
         v.Ls[b] = cull_ ? bLs_[b].as<int32_t>() : nullptr;
     }
-    v.kcap = bKcap_.as<int32_t>();
-    v.par = bPar_.as<int32_t>();
+    v.kinfo = bKinfo_.as<int4>();
     v.edit = bEdit_.as<int32_t>();
     v.ecnt = bEcnt_.as<int32_t>();
     v.dlist = bDlist_.as<int32_t>();
@@ -367,6 +366,8 @@ EngineView Engine::view() const
     v.tile_seg_min = tile_seg_min_;
     v.n_sms = sms_;
     v.flags = flags_;
+    v.single = h_cl_.size() == 1 ? 1 : 0;
+    if (v.single) v.one = h_cl_[0];
     return v;
 }
 
@@ -440,8 +441,7 @@ int Engine::finish_setup_after_choose(cudaStream_t st)
     RD_CK(bHpre_.ensure(4 * (size_t)(hist + 1)));
     RD_CK(bCnt_.ensure(4 * (size_t)(key + 1)));
     RD_CK(bBase_.ensure(4 * (size_t)(key + 1)));
-    RD_CK(bKcap_.ensure(4 * (size_t)(key + 1)));
-    RD_CK(bPar_.ensure(4 * (size_t)(key + 1)));
+    RD_CK(bKinfo_.ensure(sizeof(int4) * (size_t)(key + 1)));
     RD_CK(bEcnt_.ensure(4 * (size_t)(key + 1)));
     RD_CK(bDlist_.ensure(4 * (size_t)(key + 1)));
     RD_CK(upload_zero(bEcnt_, 4 * (size_t)(key + 1), st));
@@ -656,7 +656,7 @@ int Engine::ensure_cull_buffers()
     RD_CK(bSlack_.ensure(sizeof(float) * (blocks + 1)));
     RD_CK(bLslack_.ensure(sizeof(float) * (blocks + 1)));
     RD_CK(bBlen_.ensure(sizeof(int32_t) * (blocks + 1)));
-    RD_CK(bBlist_.ensure(sizeof(int32_t) * (32 * blocks + 1)));
+    RD_CK(bBlist_.ensure(sizeof(int32_t) * (128 * blocks + 1)));   // LIST_MAX in rd_kernels.cu
     for (int b = 0; b < 2; ++b) {
         RD_CK(bLr_[b].ensure(sizeof(float) * ((size_t)list_rows_ * pad_dim(dim_) + 4)));
         RD_CK(bLs_[b].ensure(sizeof(int32_t) * ((size_t)list_rows_ + 1)));

@@ -81,8 +81,7 @@ struct EngineView {
     // current list is in buffer par
     float* Lr[2];                // coordinates, PadDim floats per row
     int32_t* Ls[2];              // the points' positions in their cloud (culled assignment only)
-    int32_t* kcap;               // per chosen slot: rows of its region
-    int32_t* par;                // per chosen slot: buffer of its current list
+    int4* kinfo;                 // per chosen slot: base, kcap, members, par
     int32_t* edit;               // per row: edits of this pass, at the key's region
     int32_t* ecnt;               // per chosen slot: edits of this pass
     int32_t* dlist;              // chosen slots to fold in this pass
@@ -139,6 +138,8 @@ struct EngineView {
     int32_t max_iters;
     int32_t n_sms;
     int32_t flags;               // ENG_* run-mode bits
+    int32_t single;              // a run of one cloud: cl[0] is also here
+    CloudDesc one;
     // exact chunk-box culling of the assignment (see k_assign_cull)
     const float* Ps;             // evolve points in spatial order inside each cloud
     const int32_t* sorder;       // spatial position -> packed point slot
@@ -148,7 +149,7 @@ struct EngineView {
     float* bslack;               // per block: moves that leave its keys as they are (see k_assign_cull)
     float* lslack;               // per block: moves that leave its candidate list complete
     int32_t* blen;               // per block: entries of its candidate list
-    int32_t* blist;              // per block: the list (32 entries)
+    int32_t* blist;              // per block: the list (LIST_MAX entries)
     int32_t* full;               // per cloud: the next pass evaluates every block and every key
     int32_t* mvn;                // per cloud: chosen points moved in the last pass
     int32_t* dmax;               // per cloud: bits of the longest of those moves

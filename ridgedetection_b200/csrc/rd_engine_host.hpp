@@ -185,7 +185,7 @@ private:
     bool spatial_ok_ = false;     // the batch layout allows the spatial order
     bool cull_allowed_ = true;    // and its size, and the kind of run, the culled assignment
     int64_t list_rows_ = 0;       // rows of the grouped lists of the culled assignment
-    DevBuf bLr_[2], bLs_[2], bKcap_, bPar_, bEdit_, bEcnt_, bDlist_, bReb_, bRebNext_;
+    DevBuf bLr_[2], bLs_[2], bKinfo_, bEdit_, bEcnt_, bDlist_, bReb_, bRebNext_;
     DevBuf bPs_, bSorder_, bSpatialTmp_, bHpre_;
     DevBuf bKsp_, bBox_, bSlack_, bLslack_, bBlen_, bBlist_,  bFull_, bMvn_, bDmax_, bMv_;
     DevBuf bTileOrder_;

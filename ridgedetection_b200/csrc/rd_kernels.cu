@@ -41,6 +41,13 @@ __device__ __forceinline__ void pdl_enter()
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
+// Cloud c's descriptor: a run of one cloud has it in the launch parameters, one
+// memory round trip less in each of a pass's latency-bound kernels.
+__device__ __forceinline__ CloudDesc cloud_desc(const EngineView& v, const int c)
+{
+    return v.single ? v.one : v.cl[c];
+}
+
 // Work lists over the clouds still evolving, rebuilt by k_loopcond after every
 // iteration: act_cloud[a] is the a-th evolving cloud and act_pre[kind] the
 // exclusive prefix of its work items (ACT_* in rd_engine.cuh), so kernels
@@ -51,16 +58,23 @@ struct ActiveList {
     const int32_t* cloud;
     int nact;
     int total;
+    bool single;
     __device__ ActiveList(const EngineView& v, int kind)
     {
         nact = v.ctr[CTR_NACT];
         pre = v.act_pre + (int64_t)kind * (v.n_clouds + 1);
         cloud = v.act_cloud;
-        total = pre[nact];
+        total = (v.single && kind == ACT_CHUNK) ? (nact ? v.one.n_chunks : 0) : pre[nact];
+        single = v.single != 0;
     }
     // item t < total -> (cloud, item index inside that cloud)
     __device__ __forceinline__ void locate(int t, int& c, int& local) const
     {
+        if (single) {
+            c = 0;
+            local = t;
+            return;
+        }
         int lo = 0, hi = nact - 1;
         while (lo < hi) {
             const int mid = (lo + hi + 1) >> 1;
@@ -656,8 +670,8 @@ __global__ void __launch_bounds__(BLOCK) k_assign(EngineView v)
 // of the whole chosen set found them, while the moves D since then -- taken
 // over the chosen points within R of the box, which covers those within r1 --
 // add up to less than r1/4: any other chosen point is then still more than
-// r1 (1 + 4.8e-4) away.  An evaluation reads that list, at most 32 entries, one
-// per lane, instead of every chosen point; a block with more candidates keeps
+// r1 (1 + 4.8e-4) away.  An evaluation reads that list, at most LIST_MAX
+// entries, instead of every chosen point; a block with more candidates keeps
 // none and scans.
 //
 // Only changed keys are written: to the points' slots, to the spatial copy
@@ -670,8 +684,8 @@ __global__ void __launch_bounds__(BLOCK) k_assign(EngineView v)
 //
 // 1M-point helix, 285 passes: the median pass changes 0.1% of the keys; the
 // kernel that evaluated every block, with its keys and counts written anew,
-// took 36 us per pass; this one 44 us in the first pass (candidate lists built),
-// 28-40 us while every chosen point moves, 12-25 us after.  Bound by the few
+// took 36 us per pass; this one 45 us in the first pass (candidate lists built),
+// 25-40 us while every chosen point moves, 11-22 us after.  Bound by the few
 // blocks whose candidates do not fit a list, then by instruction issue.
 // ---------------------------------------------------------------------------
 constexpr int AC_BLOCK = 256;             // threads of k_assign_cull
@@ -714,6 +728,12 @@ __device__ __forceinline__ void assign_one(const float* sk, const int k, const f
     }
 }
 
+// candidates of a block: the 1M helix has 17 blocks (of 7,812) with more than 32
+// (up to 119), over jumps of the spatial order that two boxes do not cover, and
+// scanning 790 chosen points for each of them outlasted the rest of the pass
+constexpr int LIST_MAX = 128;
+// moves of a single cloud staged in shared memory
+constexpr int AC_MOVES = 512;
 constexpr int EDIT_IN = (int)0x80000000;   // edit of a member list: this point joins (else it leaves)
 constexpr int EDIT_MAX = 512;              // edits of one key that k_merge_fold takes
 
@@ -740,7 +760,8 @@ __device__ __forceinline__ void push_edit(const EngineView& v, const int c, cons
     const int64_t s = cd.key_off + k;
     const int at = atomicAdd(&v.ecnt[s], 1);
     if (at == 0) v.dlist[atomicAdd(&v.ctr[CTR_NDIRTY], 1)] = (int)s;
-    if (at < min(EDIT_MAX, v.kcap[s])) v.edit[cd.reg_off + v.base[s] + at] = edit;
+    const int2 reg = *reinterpret_cast<const int2*>(v.kinfo + s);   // base, capacity
+    if (at < min(EDIT_MAX, reg.y)) v.edit[cd.reg_off + reg.x + at] = edit;
     else v.reb[c] = 1;
 }
 
@@ -755,7 +776,18 @@ __global__ void __launch_bounds__(AC_BLOCK, ITEMS <= 4 ? 4 : 2) k_assign_cull(En
     constexpr int DP = PadDim<DIM>::v;
     constexpr int WPTS = 32 * ITEMS;
     const int lane = threadIdx.x & 31;
+    __shared__ float s_mv[2 * DIM + 1][AC_MOVES];
     const ActiveList al(v, ACT_CHUNK);
+    int n_staged = 0;   // the cloud's moves are in s_mv
+    if (v.single) {
+        const int m = v.mvn[0];
+        if (m <= AC_MOVES && !v.full[0]) {
+            for (int e = threadIdx.x; e < (2 * DIM + 1) * m; e += AC_BLOCK)
+                s_mv[e / m][e % m] = v.mv[(int64_t)(e / m) * v.n_slots + e % m];
+            n_staged = m;
+        }
+        __syncthreads();
+    }
     const int wpc_log = 31 - __clz(v.chunk_pts / WPTS);   // blocks per chunk, a power of two
     const int total = al.total << wpc_log;
     const int nw = gridDim.x * AC_WARPS;
@@ -770,8 +802,10 @@ __global__ void __launch_bounds__(AC_BLOCK, ITEMS <= 4 ? 4 : 2) k_assign_cull(En
             int lc;
             al.locate((int)(t >> wpc_log), my_c, lc);
             my_i = (lc << wpc_log) + ((int)t & ((1 << wpc_log) - 1));
-            if ((int64_t)my_i * WPTS < v.cl[my_c].n_all) {
-                const int64_t wb = (v.cl[my_c].chunk_begin << wpc_log) + my_i;
+            const int my_n = v.single ? v.one.n_all : v.cl[my_c].n_all;
+            if ((int64_t)my_i * WPTS < my_n) {
+                const int64_t wb =
+                    ((v.single ? v.one.chunk_begin : v.cl[my_c].chunk_begin) << wpc_log) + my_i;
                 my_full = v.full[my_c];
                 const float dmax = __int_as_float(v.dmax[my_c]);
                 my_slack = v.bslack[wb];
@@ -787,7 +821,7 @@ __global__ void __launch_bounds__(AC_BLOCK, ITEMS <= 4 ? 4 : 2) k_assign_cull(En
             const int c = __shfl_sync(FULL, my_c, src);
             const int bi = __shfl_sync(FULL, my_i, src);
             const int full = __shfl_sync(FULL, my_full, src);
-            const CloudDesc cd = v.cl[c];
+            const CloudDesc cd = cloud_desc(v, c);
             const int ns = v.ns[c];
             const int64_t wb = (cd.chunk_begin << wpc_log) + bi;
             const float rsq = sqr_rn(cd.r1);
@@ -811,18 +845,20 @@ __global__ void __launch_bounds__(AC_BLOCK, ITEMS <= 4 ? 4 : 2) k_assign_cull(En
             // evaluation it may save
             if (!full && 2 * m <= ns + 64) {
                 unsigned dloc = 0;
-                const float* mv = v.mv + cd.key_off;
+                const bool staged = m == n_staged;
+                const float* mv = staged ? &s_mv[0][0] : v.mv + cd.key_off;
+                const int64_t pitch = staged ? AC_MOVES : v.n_slots;
                 for (int j = lane; j < m; j += 32) {
                     float o[DIM], q[DIM];
 #pragma unroll
                     for (int d = 0; d < DIM; ++d) {
-                        o[d] = mv[(int64_t)d * v.n_slots + j];
-                        q[d] = mv[(int64_t)(DIM + d) * v.n_slots + j];
+                        o[d] = mv[d * pitch + j];
+                        q[d] = mv[(DIM + d) * pitch + j];
                     }
                     const bool out = may_skip && block_gap2<DIM>(o, box) > thr_list &&
                                      block_gap2<DIM>(q, box) > thr_list;
                     // lengths are not negative (or NaN): they order as their bits do
-                    if (!out) dloc = max(dloc, __float_as_uint(mv[(int64_t)(2 * DIM) * v.n_slots + j]));
+                    if (!out) dloc = max(dloc, __float_as_uint(mv[2 * DIM * pitch + j]));
                 }
                 dl = __uint_as_float(__reduce_max_sync(FULL, dloc));
                 const float slack = __shfl_sync(FULL, my_slack, src);
@@ -836,7 +872,7 @@ __global__ void __launch_bounds__(AC_BLOCK, ITEMS <= 4 ? 4 : 2) k_assign_cull(En
             }
             const float list_left = full ? 0.0f : __fsub_rd(v.lslack[wb], dl);
             const int n_list = (list_left > 0.0f) ? v.blen[wb] : -1;
-            int32_t* list = v.blist + wb * 32;
+            int32_t* list = v.blist + wb * LIST_MAX;
             float2 np2[ITEMS / 2][DIM];
             int old[ITEMS];
 #pragma unroll
@@ -878,11 +914,13 @@ __global__ void __launch_bounds__(AC_BLOCK, ITEMS <= 4 ? 4 : 2) k_assign_cull(En
             };
             float s[DIM];
             if (n_list >= 0) {
-                const int k = (lane < n_list) ? list[lane] : 0;
+                for (int q0 = 0; q0 < n_list; q0 += 32) {
+                    const bool in = q0 + lane < n_list;
+                    const int k = in ? list[q0 + lane] : 0;
 #pragma unroll
-                for (int d = 0; d < DIM; ++d) s[d] = gS[(int64_t)k * DIM + d];
-                take(__ballot_sync(FULL, lane < n_list && !(may_skip && block_gap2<DIM>(s, box) > thr)),
-                     s, k);
+                    for (int d = 0; d < DIM; ++d) s[d] = gS[(int64_t)k * DIM + d];
+                    take(__ballot_sync(FULL, in && !(may_skip && block_gap2<DIM>(s, box) > thr)), s, k);
+                }
                 if (lane == 0) v.lslack[wb] = list_left;
             } else {
                 float sn[DIM];
@@ -901,13 +939,13 @@ __global__ void __launch_bounds__(AC_BLOCK, ITEMS <= 4 ? 4 : 2) k_assign_cull(En
                     const unsigned nb = __ballot_sync(FULL, near);
                     if (!nb) continue;
                     const int at = len + __popc(nb & lanemask_lt());
-                    if (near && at < 32) list[at] = q;
+                    if (near && at < LIST_MAX) list[at] = q;
                     len += __popc(nb);
                     take(__ballot_sync(FULL, q < ns && !(may_skip && g2 > thr)), s, q);
                 }
                 if (lane == 0) {
                     v.blen[wb] = len;
-                    v.lslack[wb] = (may_skip && len <= 32) ? 0.25f * cd.r1 : 0.0f;
+                    v.lslack[wb] = (may_skip && len <= LIST_MAX) ? 0.25f * cd.r1 : 0.0f;
                 }
             }
             const float r1 = cd.r1;
@@ -981,7 +1019,7 @@ __device__ __forceinline__ void clear_moves(const EngineView& v, const int first
 __device__ __forceinline__ void place_key(const EngineView& v, const int64_t s, const int at, const int cap)
 {
     v.base[s] = at;
-    v.kcap[s] = cap;
+    v.kinfo[s] = make_int4(at, cap, v.cnt[s], 0);
     if (v.ecnt[s] == 0) v.dlist[atomicAdd(&v.ctr[CTR_NDIRTY], 1)] = (int)s;  // else push_edit did
 }
 
@@ -1694,9 +1732,28 @@ __device__ __forceinline__ void next_pass(const EngineView& v, const int c)
 
 // the per-cloud control step after a pass (k_control), over clouds first,
 // first + stride, ... of the active list
-__device__ void control_clouds(const EngineView& v, const int first, const int stride);
+__device__ int control_clouds(const EngineView& v, const int first, const int stride);
 __device__ void loop_condition(const EngineView& v, cudaGraphConditionalHandle h, int use_handle,
                                int count_iter);
+
+// the end of an iteration that leaves `a` clouds unfinished (one thread):
+// counters for the next one, and the loop condition
+__device__ __forceinline__ void next_iteration(const EngineView& v, int a, cudaGraphConditionalHandle h,
+                                               const int use_handle, const int count_iter)
+{
+    v.ctr[CTR_WORK] = 0;
+    v.ctr[CTR_NREADY] = 0;
+    v.ctr[CTR_NDIRTY] = 0;
+    v.ctr[CTR_TILE_HEAVY] = 0;
+    const int it = v.ctr[CTR_ITERS] + (count_iter ? 1 : 0);
+    v.ctr[CTR_ITERS] = it;
+    if (it >= v.max_iters && a > 0) {
+        v.ctr[CTR_ERR] |= ERRB_EVOLVE_CAP;
+        a = 0;
+    }
+    v.ctr[CTR_ACTIVE] = a;
+    if (use_handle) cudaGraphSetConditional(h, a > 0 ? 1u : 0u);
+}
 
 template <int DIM>
 __device__ __forceinline__ void load_row(const float* rows, const int64_t r, float (&q)[DIM])
@@ -1799,15 +1856,17 @@ __device__ void merge_fold_key(const EngineView& v, const int slot, const bool s
 {
     constexpr int DP = PadDim<DIM>::v;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int c = v.slot_cloud[slot];
-    const CloudDesc cd = v.cl[c];
+    const int c = v.single ? 0 : v.slot_cloud[slot];
+    const int4 info = v.kinfo[slot];
+    const int edits = v.ecnt[slot];
+    const CloudDesc cd = cloud_desc(v, c);
     const int k = (int)(slot - cd.key_off);
     const bool fresh = rebuilds(v, c);
-    const int64_t at = cd.reg_off + v.base[slot];
-    const int cap = v.kcap[slot];
-    const int par = fresh ? 0 : v.par[slot];
-    const int n_old = v.cnt[slot];
-    const int ne = fresh ? 0 : v.ecnt[slot];   // at most EDIT_MAX, or the cloud rebuilds
+    const int64_t at = cd.reg_off + info.x;
+    const int cap = info.y;
+    const int n_old = info.z;
+    const int par = info.w;                    // (0 when fresh)
+    const int ne = fresh ? 0 : edits;          // at most EDIT_MAX, or the cloud rebuilds
     const float* src = v.Lr[par] + at * DP;
     __syncthreads();  // the previous key's scratch, and its state, are read no more
     for (int i = tid; i < ne; i += MF_BLOCK) sm.raw[i] = v.edit[at + i];
@@ -1957,8 +2016,7 @@ __device__ void merge_fold_key(const EngineView& v, const int slot, const bool s
         if (lane == 0) {
             v.ecnt[slot] = 0;
             v.cnt[slot] = n_new;
-            if (fresh) v.par[slot] = 0;
-            else if (ne > 0) v.par[slot] = par ^ 1;
+            v.kinfo[slot] = make_int4(info.x, cap, n_new, (ne > 0) ? par ^ 1 : par);
             if (n_new > cap) v.rebnext[c] = 1;
         }
         if (n_new > 0) apply_shift<DIM>(v, c, cd, k, n_new, sum, lane);
@@ -1999,7 +2057,16 @@ __global__ void __launch_bounds__(MF_BLOCK, 4) k_merge_fold(EngineView v, cudaGr
         }
         return;
     }
-    control_clouds(v, threadIdx.x, blockDim.x);
+    const int conv = __syncthreads_or(control_clouds(v, threadIdx.x, blockDim.x));
+    if (!conv) {
+        // every cloud goes on: the work lists stay as they are
+        if (threadIdx.x == 0) {
+            v.ctr[CTR_SUM_DONE] = 0;
+            v.ctr[CTR_COND_DONE] = 1;
+            next_iteration(v, v.ctr[CTR_ACTIVE], h, use_handle, 1);
+        }
+        return;
+    }
     __threadfence();
     __syncthreads();
     const bool idle = *reinterpret_cast<volatile int32_t*>(&v.ctr[CTR_NREADY]) == 0;
@@ -2338,12 +2405,14 @@ namespace {
 // ---------------------------------------------------------------------------
 // control: one thread per cloud after each pass.
 // ---------------------------------------------------------------------------
-__device__ void control_clouds(const EngineView& v, const int first, const int stride)
+// (returns whether one of this thread's clouds converged)
+__device__ int control_clouds(const EngineView& v, const int first, const int stride)
 {
+    int any = 0;
     const int nact = v.ctr[CTR_NACT];
     for (int a = first; a < nact; a += stride) {
         const int c = v.act_cloud[a];
-        const CloudDesc cd = v.cl[c];
+        const CloudDesc cd = cloud_desc(v, c);
         v.pairs[c] += (unsigned long long)cd.n_all * (unsigned long long)v.ns[c];
         v.passes[c] += 1;
         v.total_passes[c] += 1;
@@ -2356,6 +2425,7 @@ __device__ void control_clouds(const EngineView& v, const int first, const int s
         }
         v.cont[c] = 0;
         next_pass(v, c);
+        any |= conv;
         if (conv && (v.flags & ENG_EVOLVE_ONLY)) {
             v.phase[c] = PH_DONE;
         } else if (conv) {
@@ -2366,6 +2436,7 @@ __device__ void control_clouds(const EngineView& v, const int first, const int s
                 v.ready[atomicAdd(&v.ctr[CTR_NREADY], 1)] = cd.group;
         }
     }
+    return any;
 }
 
 __global__ void k_control(EngineView v)
@@ -2892,19 +2963,7 @@ __device__ void loop_condition(const EngineView& v, cudaGraphConditionalHandle h
         const int nact = s_carry[0];
         for (int q = 0; q < ACT_KINDS; ++q) v.act_pre[q * (nc + 1) + nact] = s_carry[1 + q];
         v.ctr[CTR_NACT] = nact;
-        v.ctr[CTR_WORK] = 0;
-        v.ctr[CTR_NREADY] = 0;
-        v.ctr[CTR_NDIRTY] = 0;
-        v.ctr[CTR_TILE_HEAVY] = 0;
-        const int it = v.ctr[CTR_ITERS] + (count_iter ? 1 : 0);
-        v.ctr[CTR_ITERS] = it;
-        int a = s_act;
-        if (it >= v.max_iters && a > 0) {
-            v.ctr[CTR_ERR] |= ERRB_EVOLVE_CAP;
-            a = 0;
-        }
-        v.ctr[CTR_ACTIVE] = a;
-        if (use_handle) cudaGraphSetConditional(h, a > 0 ? 1u : 0u);
+        next_iteration(v, s_act, h, use_handle, count_iter);
     }
 }
 
