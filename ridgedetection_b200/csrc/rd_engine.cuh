@@ -160,6 +160,7 @@ struct EngineView {
     // evolved by whole thread-block clusters (rd_tile_cluster.cuh)
     const int32_t* tile_order;
     int32_t n_heavy;
+    int32_t tile_clusters;       // tiles large enough for the cluster kernel
     int32_t tile_cl_grid;        // CTAs of the cluster tile kernel (0 = one-CTA kernel)
     int32_t tile_seg_min;        // members of a key the cluster folds in segments
 };

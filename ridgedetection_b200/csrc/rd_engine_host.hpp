@@ -192,6 +192,7 @@ private:
     DevBuf bSel_, bSelTmp_;       // GPU-wide choose: survivor list and its compaction scratch
     std::vector<int32_t> h_tile_order_;
     int n_heavy_ = 0;
+    bool tile_clusters_ = false;  // fused tiled runs: the cluster kernel
     int tile_cl_grid_ = 0;
     int tile_seg_min_ = 1 << 30;
     DevBuf bDx_, bDcell_, bDalive_, bDc1_, bDc2_, bDbstart_, bDitems_, bDecHoff_, bDecHbits_;

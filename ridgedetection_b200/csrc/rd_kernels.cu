@@ -2246,11 +2246,13 @@ struct TileCtaSmem {
 };
 
 // One CTA evolves tile c to convergence (see above); dyn is the dynamic
-// shared memory laid out as tile_evolve_smem_bytes describes.
-template <int DIM, int BLOCK>
-__device__ void tile_evolve_one(const EngineView& v, const int c, const int fold_cta_min,
-                                unsigned char* dyn,
-                                TileCtaSmem<DIM, BLOCK>& ts)
+// shared memory laid out as tile_evolve_smem_bytes describes.  hand_over()
+// (thread 0, after every pass): leave the tile as this pass left it to somebody
+// else; then true is returned.
+template <int DIM, int BLOCK, class HandOver>
+__device__ bool tile_evolve_one(const EngineView& v, const int c, const int fold_cta_min,
+                                unsigned char* dyn, TileCtaSmem<DIM, BLOCK>& ts,
+                                HandOver&& hand_over)
 {
     constexpr int W = BLOCK / 32;
     constexpr int DP = PadDim<DIM>::v;
@@ -2279,6 +2281,7 @@ __device__ void tile_evolve_one(const EngineView& v, const int c, const int fold
             for (int d = 0; d < DIM; ++d) sS[e * DP + d] = (e < ns) ? gS[(int64_t)e * DIM + d] : FAR;
         const int r0 = (int)(((int64_t)warp * n) / W), r1w = (int)(((int64_t)(warp + 1) * n) / W);
         int pass = 0;
+        bool handed = false;
         for (;;) {
             // 1. assignment of the warp's range + per-warp key counts
             //    (counts added once per distinct key of a warp step)
@@ -2362,6 +2365,8 @@ __device__ void tile_evolve_one(const EngineView& v, const int c, const int fold
                 if (tid == 0) v.err[c] |= ERRB_EVOLVE_CAP;
                 break;
             }
+            handed = __syncthreads_or(tid == 0 ? hand_over() : 0);
+            if (handed) break;
         }
         // results back and control (as k_control does after the last pass)
         for (int e = tid; e < ns; e += BLOCK)
@@ -2371,11 +2376,14 @@ __device__ void tile_evolve_one(const EngineView& v, const int c, const int fold
             v.passes[c] += pass;
             v.total_passes[c] += pass;
             v.cont[c] = 0;
-            v.phase[c] = PH_CONVERGED;
-            const GroupDesc gd = v.gr[cd.group];
-            if (atomicAdd(&v.group_conv[cd.group], 1) + 1 == gd.n_clouds)
-                v.ready[atomicAdd(&v.ctr[CTR_NREADY], 1)] = cd.group;
+            if (!handed) {
+                v.phase[c] = PH_CONVERGED;
+                const GroupDesc gd = v.gr[cd.group];
+                if (atomicAdd(&v.group_conv[cd.group], 1) + 1 == gd.n_clouds)
+                    v.ready[atomicAdd(&v.ctr[CTR_NREADY], 1)] = cd.group;
+            }
         }
+        return handed;
     }
 }
 
@@ -2386,7 +2394,7 @@ __global__ void __launch_bounds__(BLOCK) k_tile_evolve(EngineView v)
     __shared__ TileCtaSmem<DIM, BLOCK> ts;
     const int nact = v.ctr[CTR_NACT];
     for (int a = blockIdx.x; a < nact; a += gridDim.x)
-        tile_evolve_one<DIM, BLOCK>(v, v.act_cloud[a], FOLD_CTA_MIN, smem_raw, ts);
+        tile_evolve_one<DIM, BLOCK>(v, v.act_cloud[a], FOLD_CTA_MIN, smem_raw, ts, [] { return 0; });
 }
 
 __host__ __device__ constexpr int tile_evolve_smem_bytes(int dim)
@@ -3301,7 +3309,7 @@ cudaError_t prepare_tile_pass(int dim, const EngineView& v, int* cl_grid)
                                              cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              tile_evolve_smem_bytes(DIM));
         if (e != cudaSuccess) return e;
-        if (v.n_heavy > 0) {
+        if (v.n_heavy > 0 || v.tile_clusters) {
             e = tile_cl_prepare<DIM>(cl_grid);
             if (e != cudaSuccess) return e;
         }

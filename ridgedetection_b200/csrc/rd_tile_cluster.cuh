@@ -20,8 +20,10 @@
 //                warp folds its segment from a speculative start (the FP64 sum
 //                of the members before it) and records a trace, and one warp
 //                replays the traces in order from the exact start
-//                (rd_segfold.cuh).  Smaller keys are folded whole by the CTA
-//                that owns them (warp fold, or the CTA's segmented fold);
+//                (rd_segfold.cuh).  Smaller keys are folded whole by a warp of
+//                the CTA that owns them (one CTA's segmented fold of keys of
+//                4,096+ members took longer: 1M spiral in 70 leaves 56 -> 37 ms
+//                without it);
 //   shift        the owner of each key applies the movement test; the new
 //                coordinates and moved flags are gathered by every CTA, so all
 //                CTAs take the same loop decision.
@@ -59,6 +61,10 @@ struct ClusterSmem {
     int segmv[TSEG_KEYS][DIM];       // a segmented key's coordinate moved
     int nseg;
     int tile;
+    // rank 0's: light tiles handed over to the whole cluster
+    int idle;                        // CTAs of the cluster that found no more light tile
+    int nreq;
+    int req[TCL];
 };
 
 // dynamic shared memory of the cluster kernel: the one-CTA layout, then
@@ -87,7 +93,6 @@ __device__ void tile_evolve_cluster(const EngineView& v, const int c, unsigned c
     int* hist = reinterpret_cast<int*>(sS + TILE_NS_MAX * DP);
     int* kbase = hist + W * (TILE_NS_MAX + 1);
     auto& s_buf = ts.buf;
-    auto& s_seg = ts.seg;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     static_assert(W == TCL_W, "the cluster smem holds TCL_W warp segments per CTA");
     const CloudDesc cd = v.cl[c];
@@ -107,6 +112,7 @@ __device__ void tile_evolve_cluster(const EngineView& v, const int c, unsigned c
     const int r0 = lo_c + (int)(((int64_t)warp * (hi_c - lo_c)) / W);
     const int r1w = lo_c + (int)(((int64_t)(warp + 1) * (hi_c - lo_c)) / W);
     int pass = 0;
+    const int before = v.passes[c];   // passes of this evolve run a single CTA made
     for (;;) {
         // 1. assignment of this CTA's range (exactly as tile_evolve_one)
         for (int k = lane; k <= ns; k += 32) hist[warp * (TILE_NS_MAX + 1) + k] = 0;
@@ -218,26 +224,10 @@ __device__ void tile_evolve_cluster(const EngineView& v, const int c, unsigned c
             for (int j = 0; j < nseg; ++j) r = r || (cs.segk[j] == k);
             return r;
         };
-        for (int k = rank; k < ns; k += TCL) {
-            const int cnt = cs.kcnt[k];
-            if (cnt < FOLD_CTA_MIN || is_seg(k)) continue;
-            fold_members_seg_src<W, DIM>(RowSrc<DIM>{Pg + (int64_t)kbase[k] * DP}, cnt, s_seg);
-            if (warp == 0) {
-                int mv = 0;
-                if (lane < DIM) {
-                    float cval = sS[k * DP + lane];
-                    mv = shift_coord(s_seg.out[lane], cnt, cval);
-                    cs.res[k][lane] = cval;
-                }
-                mv = __any_sync(FULL, mv);
-                if (lane == 0) cs.res_moved[k] = mv;
-            }
-            __syncthreads();
-        }
         for (int q = warp; rank + q * TCL < ns; q += W) {
             const int k = rank + q * TCL;
             const int cnt = cs.kcnt[k];
-            if (cnt == 0 || cnt >= FOLD_CTA_MIN || is_seg(k)) continue;
+            if (cnt == 0 || is_seg(k)) continue;
             const float sum = fold_rows<DIM, SUM_BP>(Pg + (int64_t)kbase[k] * DP, cnt, s_buf[warp], lane);
             int moved = 0;
             float cval = 0.0f;
@@ -309,7 +299,7 @@ __device__ void tile_evolve_cluster(const EngineView& v, const int c, unsigned c
         ++pass;
         if (rank == 0 && tid == 0) v.pairs[c] += (unsigned long long)n * (unsigned long long)ns;
         if (!moved) break;
-        if (pass >= v.max_passes) {
+        if (before + pass >= v.max_passes) {
             if (rank == 0 && tid == 0) v.err[c] |= ERRB_EVOLVE_CAP;
             break;
         }
@@ -332,7 +322,14 @@ __device__ void tile_evolve_cluster(const EngineView& v, const int c, unsigned c
 }
 
 // Heavy tiles (tile_order[0..n_heavy), largest first) by whole clusters,
-// then the light tiles (tile_order[n_heavy..n_clouds)) by single CTAs.
+// then the light tiles (tile_order[n_heavy..n_clouds)) by single CTAs.  When no
+// light tile waits any more and most of a cluster's CTAs are done, those that
+// still evolve one (of TCL_HAND_MIN or more points) hand it over and the whole
+// cluster goes on with it: how many passes a tile takes is not known before, and
+// the few that take most of them were what a launch ended on (10M spiral 34.9 ->
+// 32.3 ms; 2M in 582 leaves, by the threshold of heavy tiles, 33-90 -> 34 ms).
+constexpr int TCL_HAND_MIN = 2048;
+constexpr int TCL_HAND_IDLE = 5;   // idle CTAs of the cluster's TCL
 template <int DIM, int BLOCK>
 __global__ void __launch_bounds__(BLOCK) k_tile_evolve_cl(EngineView v)
 {
@@ -343,6 +340,7 @@ __global__ void __launch_bounds__(BLOCK) k_tile_evolve_cl(EngineView v)
     cg::cluster_group cl = cg::this_cluster();
     const int rank = (int)cl.block_rank();
     const int tid = threadIdx.x;
+    if (rank == 0 && tid == 0) cs.idle = cs.nreq = 0;   // seen after the first barrier below
     for (;;) {
         if (rank == 0 && tid == 0) {
             const int t = atomicAdd(&v.ctr[CTR_TILE_HEAVY], 1);
@@ -366,8 +364,25 @@ __global__ void __launch_bounds__(BLOCK) k_tile_evolve_cl(EngineView v)
         const int c = s_t;
         __syncthreads();
         if (c < 0) break;
-        if (v.phase[c] == PH_EVOLVE) tile_evolve_one<DIM, BLOCK>(v, c, FOLD_CTA_MIN_LIGHT, smem_raw, ts);
+        if (v.phase[c] != PH_EVOLVE) continue;
+        ClusterSmem<DIM>* c0 = cl.map_shared_rank(&cs, 0);
+        const bool can = v.cl[c].n_all >= TCL_HAND_MIN;
+        const bool handed = tile_evolve_one<DIM, BLOCK>(v, c, FOLD_CTA_MIN_LIGHT, smem_raw, ts, [&] {
+            return can && *reinterpret_cast<volatile int32_t*>(&v.ctr[CTR_WORK]) >= n_light &&
+                   *reinterpret_cast<volatile int*>(&c0->idle) >= TCL_HAND_IDLE;
+        });
+        if (handed && tid == 0) c0->req[atomicAdd(&c0->nreq, 1)] = c;
     }
+    if (tid == 0) atomicAdd(&cl.map_shared_rank(&cs, 0)->idle, 1);
+    // every write of a handed tile's CTA (its chosen points) before the cluster's reads
+    __threadfence();
+    cl.sync();
+    const int nreq = cl.map_shared_rank(&cs, 0)->nreq;
+    for (int i = 0; i < nreq; ++i) {
+        const int c = cl.map_shared_rank(&cs, 0)->req[i];
+        tile_evolve_cluster<DIM, BLOCK>(v, c, smem_raw, ts, cs, cl, rank);
+    }
+    cl.sync();   // rank 0's list is read no more
 }
 
 }  // namespace

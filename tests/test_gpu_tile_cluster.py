@@ -71,3 +71,14 @@ def test_cluster_switch_changes_nothing(rdb):
     S_on, st, _ = rdb.tiled_ridge_detection(P, *args)
     assert st.err_bits == 0 and bits_equal(S_on, S_off)
     assert rdb.get_tile_clusters() == (True, 100000, 8192)
+
+
+@pytest.mark.parametrize("n,tiles", [(60_000, (3, 3)), (60_000, (17, 19)), (200_000, (9, 9))])
+def test_handed_over_tiles_match_oracle(rdb, n, tiles):
+    """Default thresholds on few and on many tiles: light tiles that the last busy CTAs of a
+    cluster hand over to it, and tiles heavy by their share of the points."""
+    P = G.spiral2d(n, seed=n + tiles[0])
+    S_ref, _, _ = O.ridge_tiled(P, 0.2, 0.4, n + 1, tiles)
+    for mode in (rdb.LOOP_GRAPH, rdb.LOOP_HOST):
+        S, st, _ = rdb.tiled_ridge_detection(P, 0.2, 0.4, n + 1, tiles, loop_mode=mode)
+        assert st.err_bits == 0 and bits_equal(S, S_ref)
