@@ -330,6 +330,7 @@ EngineView Engine::view() const
     v.dbig = bDbig_.as<int32_t>();
     v.dcpre = bDcpre_.as<int32_t>();
     v.dec_smem_max = dec_smem_max_;
+    v.dec_dyn = dec_dyn_bytes(dec_smem_max_);
     v.dec_nb_pp = dec_nb_pp_;
     v.dec_hoff = bDecHoff_.as<int64_t>();
     v.dec_hbits = bDecHbits_.as<int32_t>();
@@ -540,7 +541,9 @@ int Engine::run(cudaStream_t st, bool use_graph, int mode)
         const EngineView v1 = view();
         RD_CK(launch_set_given(v1, mode == RUN_DECIMATE_ONLY ? 1 : 0, st));
         if (mode == RUN_DECIMATE_ONLY) {
-            RD_CK(launch_decimate(dim_, v1, st));
+            int64_t points = 0;
+            for (const GroupDesc& gd : h_gr_) points = std::max<int64_t>(points, gd.s_cap);
+            RD_CK(launch_decimate(dim_, v1, points, st));
             return collect(st);
         }
     } else {

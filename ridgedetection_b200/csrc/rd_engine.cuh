@@ -117,10 +117,11 @@ struct EngineView {
     int32_t* ditems;             // bucket members
     int32_t* dnb_off;            // per group: neighbour-list offsets (total+1)
     int32_t* dnb;                // per group: neighbour lists, dec_nb_pp per scratch slot
-    int32_t* dbig;               // GPU-wide prepared decimation: {state, group, total}
+    int32_t* dbig;               // GPU-wide prepared decimation: {state, group, total, left}
     int32_t* dcpre;              // its members' chosen-count prefix (n_clouds+1)
     int32_t dec_smem_max;        // points whose counts fit the decimation's shared memory
     int32_t dec_nb_pp;           // neighbour-list entries per scratch slot
+    int32_t dec_dyn;             // bytes of the decimation's dynamic shared memory
     const int64_t* dec_hoff;     // per group: start of its bucket arrays
     const int32_t* dec_hbits;    // per group: log2 buckets
     int32_t n_clouds;
@@ -165,12 +166,15 @@ struct EngineView {
     int32_t tile_seg_min;        // members of a key the cluster folds in segments
 };
 
-// dynamic shared memory of the decimation kernel: two int16 counts and an
-// alive byte per point, then a candidate bit per point
-inline int dec_smem_bytes(const EngineView& v)
-{
-    return ((v.dec_smem_max * 5 + 15) / 16) * 16 + 4 * ((v.dec_smem_max + 31) / 32) + 16;
-}
+// dynamic shared memory of the decimation kernel's list path: two int16 counts
+// and an alive byte per point, then a candidate bit per point; the bit-matrix
+// path lays it out as rd_decbits.cuh describes
+inline int dec_list_bytes(int points) { return ((points * 5 + 15) / 16) * 16 + 4 * ((points + 31) / 32) + 16; }
+constexpr int DEC_BITS_MAX = 4096;           // points decimated over bit matrices
+constexpr int DEC_BITS_SMEM = 200 * 1024;    // shared memory for them
+inline int dec_smem_bytes(const EngineView& v) { return v.dec_dyn; }
+// bytes for groups of up to `points` points
+int dec_dyn_bytes(int points);
 
 // launch configuration picked by the tuner per (dim, cloud size, r1) bucket
 struct TuneParams {
@@ -230,7 +234,8 @@ cudaError_t prepare_tile_pass(int dim, const EngineView& v, int* cl_grid);
 // the iteration ends with the loop condition as in launch_pass
 cudaError_t launch_tile_pass(int dim, const EngineView& v, const LoopCond& lc, cudaStream_t st,
                              cudaEvent_t a0 = nullptr, cudaEvent_t a1 = nullptr);
-cudaError_t launch_decimate(int dim, const EngineView& v, cudaStream_t st);
+// points: of the largest group
+cudaError_t launch_decimate(int dim, const EngineView& v, int64_t points, cudaStream_t st);
 // quality metrics (rd_quality.cu)
 cudaError_t launch_min_dist(int dim, const float* A, int na, const float* B, int nb, float* out,
                             cudaStream_t st);

@@ -199,11 +199,13 @@ __device__ void decimate_scan(const float* X, const int total, const float r2, c
 
 // Visits every point q != i within 2*r2 of point i of X (bucketed by the
 // counting sort in items/bstart, cells in cell): f(q, within_r2).
+// With cell0 / step a thread takes every step-th of the neighbour cells only.
 template <int DIM, class F>
 __device__ __forceinline__ void dec_for_neighbours(const int i, const float* X,
                                                    const int32_t* cell, const int32_t* items,
                                                    const int32_t* bstart, const uint32_t hmask,
-                                                   const float rsq, const float rsq4, F&& f)
+                                                   const float rsq, const float rsq4, F&& f,
+                                                   const int cell0 = 0, const int step = 1)
 {
     constexpr int NB = Pow3<DIM>::v;
     float p[DIM];
@@ -213,7 +215,7 @@ __device__ __forceinline__ void dec_for_neighbours(const int i, const float* X,
         p[d] = X[(int64_t)i * DIM + d];
         cc[d] = cell[(int64_t)i * DIM + d];
     }
-    for (int o = 0; o < NB; ++o) {
+    for (int o = cell0; o < NB; o += step) {
         int nc[DIM];
         neighbour_cell<DIM>(cc, o, nc);
         const uint32_t b = cell_hash<DIM>(nc) & hmask;
@@ -350,14 +352,16 @@ __device__ int decimate_round_passes(const int total, int cnt, CT* c1, CT* c2, S
 // with one coalesced read of its list; counts and alive flags live in shared
 // memory (smem, 5 bytes per point) when total <= smem_max.  Falls back to
 // decimate_scan when the lists do not fit in nb_cap.  alive[] (global)
-// receives the survivors either way.
+// receives the survivors either way.  prepared: 1 = lists and counts are there,
+// 3 = and the rounds are done, with rounds_left as k_dec_rounds leaves dbig[3].
 template <int DIM, int BLOCK>
 __device__ void decimate_scan_lists(const float* X, const int total, const float r2,
                                     const int nocopy, int32_t* cell, int32_t* alive, int32_t* c1g,
                                     int32_t* c2g, int32_t* items, int32_t* bstart,
                                     const uint32_t hmask, int32_t* nb_off, int32_t* nb,
                                     const int64_t nb_cap, unsigned char* smem, const int smem_max,
-                                    int32_t* err, const int prepared = 0, int32_t* tally = nullptr)
+                                    int32_t* err, const int prepared = 0, int32_t* tally = nullptr,
+                                    const int rounds_left = 0)
 {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const float rsq = sqr_rn(r2);
@@ -378,9 +382,9 @@ __device__ void decimate_scan_lists(const float* X, const int total, const float
             if (in_smem) {
                 c1s[i] = (int16_t)c1g[i];
                 c2s[i] = (int16_t)c2g[i];
-                as[i] = 1;
+                as[i] = prepared == 3 ? (unsigned char)alive[i] : 1;
             }
-            alive[i] = 1;
+            if (prepared != 3) alive[i] = 1;
         }
         __syncthreads();
     } else {
@@ -481,7 +485,14 @@ __device__ void decimate_scan_lists(const float* X, const int total, const float
     }
     // passes in parallel rounds while the minimum-count rule cannot act
     __shared__ int s_alive, s_fallback;
-    {
+    if (prepared == 3) {   // done (the counts and alive flags are those after the last pass)
+        if (tid == 0) {
+            s_alive = rounds_left < 0 ? -1 - rounds_left : rounds_left;
+            s_fallback = rounds_left < 0;
+        }
+        __syncthreads();
+        if (!s_fallback) return;
+    } else {
         int fb = 0;
         const int left = in_smem
             ? decimate_round_passes<BLOCK>(total, total, c1s, c2s, as, nb_off, nb, &fb, err, tally)
