@@ -250,15 +250,11 @@ int Engine::setup(int dim, const std::vector<CloudDesc>& clouds,
     RD_CK(bNext_.ensure(sizeof(int32_t) * (size_t)(s_off + 1)));
     RD_CK(bKeys_.ensure(sizeof(int32_t) * (size_t)(total_points + 1)));
     RD_CK(bGrouped_.ensure(sizeof(int32_t) * (size_t)(total_points + 4)));
-    RD_CK(bNs_.ensure(4 * (nc + 1)));
+    RD_CK(bRes_.ensure(res_bytes(nc)));
     RD_CK(bPhase_.ensure(4 * (nc + 1)));
     RD_CK(bCont_.ensure(4 * (nc + 1)));
     RD_CK(bPasses_.ensure(4 * (nc + 1)));
-    RD_CK(bTotPasses_.ensure(4 * (nc + 1)));
     RD_CK(bOuter_.ensure(4 * (nc + 1)));
-    RD_CK(bErr_.ensure(4 * (nc + 1)));
-    RD_CK(bPairs_.ensure(8 * (nc + 1)));
-    RD_CK(bCtr_.ensure(4 * CTR_COUNT));
     RD_CK(bKbDone_.ensure(4 * (nc + 1)));
     RD_CK(bFull_.ensure(4 * (nc + 1)));
     RD_CK(bReb_.ensure(4 * (nc + 1)));
@@ -305,15 +301,17 @@ EngineView Engine::view() const
     v.kbdone = bKbDone_.as<int32_t>();
     v.next = bNext_.as<int32_t>();
     v.hash = bHash_.as<int32_t>();
-    v.ns = bNs_.as<int32_t>();
+    // what collect() reads back, in one piece (res_bytes)
+    const size_t nr = h_cl_.size() + 1;
+    v.pairs = bRes_.as<unsigned long long>();
+    v.ns = reinterpret_cast<int32_t*>(v.pairs + nr);
+    v.total_passes = v.ns + nr;
+    v.err = v.total_passes + nr;
+    v.ctr = v.err + nr;
     v.phase = bPhase_.as<int32_t>();
     v.cont = bCont_.as<int32_t>();
     v.passes = bPasses_.as<int32_t>();
-    v.total_passes = bTotPasses_.as<int32_t>();
     v.outer = bOuter_.as<int32_t>();
-    v.err = bErr_.as<int32_t>();
-    v.pairs = bPairs_.as<unsigned long long>();
-    v.ctr = bCtr_.as<int32_t>();
     v.act_cloud = bActCloud_.as<int32_t>();
     v.act_pre = bActPre_.as<int32_t>();
     v.group_conv = bGroupConv_.as<int32_t>();
@@ -380,15 +378,15 @@ static int ceil_log2(int64_t x)
     return b;
 }
 
-int Engine::finish_setup_after_choose(cudaStream_t st)
+int Engine::finish_setup_after_choose(cudaStream_t st, bool ns_given)
 {
     const size_t nc = h_cl_.size();
     h_ns_.resize(nc);
-    if (DevArena* a = current_arena(); a && a->measuring()) {
-        // size planning: the counts the caller will give
+    if (DevArena* a = current_arena(); (a && a->measuring()) || ns_given) {
+        // size planning: the counts the caller will give; or has given
         for (size_t c = 0; c < nc; ++c) h_ns_[c] = c < given_ns.size() ? given_ns[c] : h_cl_[c].n_own;
     } else {
-        RD_CK(cudaMemcpyAsync(h_ns_.data(), bNs_.p, 4 * nc, cudaMemcpyDeviceToHost, st));
+        RD_CK(cudaMemcpyAsync(h_ns_.data(), view().ns, 4 * nc, cudaMemcpyDeviceToHost, st));
         RD_CK(cudaStreamSynchronize(st));
     }
     int64_t hist = 0, key = 0, kblk = 0, kblk_warp = 0, rows = 0;
@@ -535,9 +533,9 @@ int Engine::run(cudaStream_t st, bool use_graph, int mode)
             }
         EngineView v0 = view();
         RD_CK(launch_reset(v0, st));
-        RD_CK(cudaMemcpyAsync(bNs_.p, given_ns.data(), 4 * given_ns.size(),
+        RD_CK(cudaMemcpyAsync(v0.ns, given_ns.data(), 4 * given_ns.size(),
                               cudaMemcpyHostToDevice, st));
-        if (int rc = finish_setup_after_choose(st)) return rc;
+        if (int rc = finish_setup_after_choose(st, true)) return rc;
         const EngineView v1 = view();
         RD_CK(launch_set_given(v1, mode == RUN_DECIMATE_ONLY ? 1 : 0, st));
         if (mode == RUN_DECIMATE_ONLY) {
@@ -564,7 +562,7 @@ int Engine::run(cudaStream_t st, bool use_graph, int mode)
             RD_CK(launch_choose(dim_, v0, st));
         if (mode == RUN_CHOOSE_ONLY) {
             h_ns_.resize(h_cl_.size());
-            RD_CK(cudaMemcpyAsync(h_ns_.data(), bNs_.p, 4 * h_ns_.size(), cudaMemcpyDeviceToHost,
+            RD_CK(cudaMemcpyAsync(h_ns_.data(), v0.ns, 4 * h_ns_.size(), cudaMemcpyDeviceToHost,
                                   st));
             RD_CK(cudaStreamSynchronize(st));
             return 0;
@@ -756,9 +754,9 @@ int Engine::adjoint_setup(cudaStream_t st)
     RD_CK(upload(bGr_, h_gr_, st));
     EngineView v0 = view();
     RD_CK(launch_reset(v0, st));
-    RD_CK(cudaMemcpyAsync(bNs_.p, given_ns.data(), 4, cudaMemcpyHostToDevice, st));
+    RD_CK(cudaMemcpyAsync(v0.ns, given_ns.data(), 4, cudaMemcpyHostToDevice, st));
     RD_CK(upload(bChunkCloud_, h_chunk_cloud_, st));
-    if (int rc = finish_setup_after_choose(st)) return rc;
+    if (int rc = finish_setup_after_choose(st, true)) return rc;
     if (int rc = start_passes(st)) return rc;
     const EngineView v = view();
     RD_CK(launch_set_given(v, 0, st));
@@ -784,16 +782,16 @@ int Engine::adjoint_restart(cudaStream_t st)
 int Engine::collect(cudaStream_t st)
 {
     const size_t nc = h_cl_.size();
-    std::vector<int32_t> tp(nc);
-    std::vector<unsigned long long> pr(nc);
-    int32_t ctr[CTR_COUNT];
-    h_err_.resize(nc);
-    RD_CK(cudaMemcpyAsync(h_ns_.data(), bNs_.p, 4 * nc, cudaMemcpyDeviceToHost, st));
-    RD_CK(cudaMemcpyAsync(h_err_.data(), bErr_.p, 4 * nc, cudaMemcpyDeviceToHost, st));
-    RD_CK(cudaMemcpyAsync(tp.data(), bTotPasses_.p, 4 * nc, cudaMemcpyDeviceToHost, st));
-    RD_CK(cudaMemcpyAsync(pr.data(), bPairs_.p, 8 * nc, cudaMemcpyDeviceToHost, st));
-    RD_CK(cudaMemcpyAsync(ctr, bCtr_.p, sizeof(ctr), cudaMemcpyDeviceToHost, st));
+    // pairs, chosen counts, passes, errors and counters in one copy (five copies of
+    // pageable memory cost about 15 us each)
+    h_res_.resize((res_bytes(nc) + 7) / 8);
+    RD_CK(cudaMemcpyAsync(h_res_.data(), bRes_.p, res_bytes(nc), cudaMemcpyDeviceToHost, st));
     RD_CK(cudaStreamSynchronize(st));
+    const uint64_t* pr = h_res_.data();
+    const int32_t* ns = reinterpret_cast<const int32_t*>(pr + nc + 1);
+    const int32_t *tp = ns + nc + 1, *er = tp + nc + 1, *ctr = er + nc + 1;
+    h_ns_.assign(ns, ns + nc);
+    h_err_.assign(er, er + nc);
     stats_.loop_iters = ctr[CTR_ITERS];
     stats_.err_bits = ctr[CTR_ERR];
     stats_.dec_passes = ctr[CTR_DEC_PASSES];

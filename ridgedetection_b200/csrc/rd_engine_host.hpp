@@ -147,7 +147,10 @@ public:
     std::string last_error;
 
 private:
-    int finish_setup_after_choose(cudaStream_t st);
+    // ns_given: the chosen counts are those in given_ns
+    int finish_setup_after_choose(cudaStream_t st, bool ns_given = false);
+    // per cloud 64-bit pairs and 32-bit chosen count, passes and errors; then the counters
+    static size_t res_bytes(size_t nc) { return 20 * (nc + 1) + 4 * CTR_COUNT; }
     bool cull_possible() const;
     int ensure_cull_buffers();
     int start_passes(cudaStream_t st);
@@ -176,7 +179,8 @@ private:
 
     DevBuf bCl_, bGr_, bChunkCloud_, bSlotCloud_;
     DevBuf bP_, bS_, bKeys_, bGrouped_, bPg_, bHist_, bCnt_, bBase_, bNext_, bHash_, bSurv_;
-    DevBuf bNs_, bPhase_, bCont_, bPasses_, bTotPasses_, bOuter_, bErr_, bPairs_, bCtr_, bKbDone_;
+    DevBuf bRes_, bPhase_, bCont_, bPasses_, bOuter_, bKbDone_;
+    std::vector<uint64_t> h_res_;
     DevBuf bActCloud_, bActPre_, bGroupConv_, bReady_, bDnbOff_, bDnb_, bDbig_, bDcpre_;
     int dec_smem_max_ = 0;
     int dec_nb_pp_ = DEC_NB_MIN_PER_POINT;

@@ -64,9 +64,10 @@ __device__ __forceinline__ void chunk_range(const CloudDesc& cd, int lc, int& lo
     hi = (int)(((int64_t)(lc + 1) * cd.n_all) / cd.n_chunks);
 }
 
-// sort keys: (cloud << 32) | Morton code; values: packed slot
-template <int DIM>
-__global__ void __launch_bounds__(256) k_morton(EngineView v, uint64_t* key, int32_t* val)
+// sort keys: (cloud << 32) | Morton code, of one cloud the code alone (half the
+// bytes of the sort's passes); values: packed slot
+template <int DIM, class Key>
+__global__ void __launch_bounds__(256) k_morton(EngineView v, Key* key, int32_t* val)
 {
     for (int ch = blockIdx.x; ch < v.n_chunks; ch += gridDim.x) {
         const int c = v.chunk_cloud[ch];
@@ -79,7 +80,8 @@ __global__ void __launch_bounds__(256) k_morton(EngineView v, uint64_t* key, int
             float p[DIM];
 #pragma unroll
             for (int d = 0; d < DIM; ++d) p[d] = v.P[s * DIM + d];
-            key[s] = ((uint64_t)(uint32_t)c << 32) | morton_code<DIM>(p, inv);
+            if constexpr (sizeof(Key) == 8) key[s] = ((uint64_t)(uint32_t)c << 32) | morton_code<DIM>(p, inv);
+            else key[s] = morton_code<DIM>(p, inv);
             val[s] = (int32_t)s;
             v.keys[s] = -1;   // no point has a key before the first pass
         }
@@ -189,11 +191,13 @@ __global__ void __launch_bounds__(256) k_gather_spatial(EngineView v, int items,
 
 size_t sort_temp_bytes(int64_t n)
 {
-    size_t bytes = 0;
+    size_t bytes = 0, bytes32 = 0;
     cub::DoubleBuffer<uint64_t> k(nullptr, nullptr);
+    cub::DoubleBuffer<uint32_t> k32(nullptr, nullptr);
     cub::DoubleBuffer<int32_t> v(nullptr, nullptr);
     cub::DeviceRadixSort::SortPairs(nullptr, bytes, k, v, (int)n, 0, 64);
-    return bytes;
+    cub::DeviceRadixSort::SortPairs(nullptr, bytes32, k32, v, (int)n, 0, 32);
+    return std::max(bytes, bytes32);
 }
 
 size_t align256(size_t x) { return (x + 255) / 256 * 256; }
@@ -205,8 +209,6 @@ cudaError_t spatial_prep_dim(const EngineView& v, int items, int64_t n, void* sc
 {
     if (n <= 0 || v.n_chunks <= 0) return cudaSuccess;
     unsigned char* p = static_cast<unsigned char*>(scratch);
-    uint64_t* k0 = reinterpret_cast<uint64_t*>(p);
-    uint64_t* k1 = reinterpret_cast<uint64_t*>(p + align256(8 * (size_t)n));
     int32_t* v0 = reinterpret_cast<int32_t*>(p + 2 * align256(8 * (size_t)n));
     int32_t* v1 = reinterpret_cast<int32_t*>(p + 2 * align256(8 * (size_t)n) + align256(4 * (size_t)n));
     unsigned char* tmp = p + 2 * align256(8 * (size_t)n) + 2 * align256(4 * (size_t)n);
@@ -215,12 +217,20 @@ cudaError_t spatial_prep_dim(const EngineView& v, int items, int64_t n, void* sc
     size_t tmp_bytes = scratch_bytes - used;
     const int sms = v.n_sms > 0 ? v.n_sms : 148;
     const int cgrid = std::max(1, std::min(v.n_chunks, sms * 8));
-    k_morton<DIM><<<cgrid, 256, 0, st>>>(v, k0, v0);
-    int end_bit = 32;
-    while (end_bit < 64 && (int64_t(1) << (end_bit - 32)) < v.n_clouds) ++end_bit;
-    cub::DoubleBuffer<uint64_t> kb(k0, k1);
     cub::DoubleBuffer<int32_t> vb(v0, v1);
-    cudaError_t e = cub::DeviceRadixSort::SortPairs(tmp, tmp_bytes, kb, vb, (int)n, 0, end_bit, st);
+    auto sort = [&](auto kind, int end_bit) -> cudaError_t {
+        using Key = decltype(kind);
+        Key* k0 = reinterpret_cast<Key*>(p);
+        Key* k1 = reinterpret_cast<Key*>(p + align256(8 * (size_t)n));
+        k_morton<DIM, Key><<<cgrid, 256, 0, st>>>(v, k0, v0);
+        cub::DoubleBuffer<Key> kb(k0, k1);
+        return cub::DeviceRadixSort::SortPairs(tmp, tmp_bytes, kb, vb, (int)n, 0, end_bit, st);
+    };
+    // 10 bits of three cell coordinates, 16 of two, 32 of one
+    const int code_bits = DIM >= 3 ? 30 : 32;
+    int cloud_bits = 0;
+    while (cloud_bits < 32 && (int64_t(1) << cloud_bits) < v.n_clouds) ++cloud_bits;
+    const cudaError_t e = v.n_clouds == 1 ? sort(uint32_t(0), code_bits) : sort(uint64_t(0), 32 + cloud_bits);
     if (e != cudaSuccess) return e;
     const int64_t blocks = (int64_t)v.n_chunks * (v.chunk_pts / (32 * items));
     const int ggrid = (int)std::max<int64_t>(1, std::min<int64_t>((blocks + 7) / 8, (int64_t)sms * 16));
