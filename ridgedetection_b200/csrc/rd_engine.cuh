@@ -216,9 +216,10 @@ struct LoopCond {
 };
 // One iteration: evolve pass, control, decimation, loop condition.  a0/a1
 // (optional) are recorded on `st` right before and after the assign kernel.
+// follows_pass: the kernel before on `st` is the last one of such an iteration.
 cudaError_t launch_pass(int dim, const EngineView& v, const TuneParams& tp, int assign_grid,
                         const LoopCond& lc, cudaStream_t st, cudaEvent_t a0 = nullptr,
-                        cudaEvent_t a1 = nullptr);
+                        cudaEvent_t a1 = nullptr, bool follows_pass = false);
 // Sets the loop condition and rebuilds the work lists of the next iteration
 // as a kernel of its own (count_iter = 0 for the initial build before the
 // first iteration).

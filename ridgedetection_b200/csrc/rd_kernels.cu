@@ -2060,6 +2060,13 @@ __global__ void __launch_bounds__(MF_BLOCK, 4) k_merge_fold(EngineView v, cudaGr
         }
         return;
     }
+    if (v.ctr[CTR_NACT] == 0) {   // a pass after the last one
+        if (threadIdx.x == 0) {
+            v.ctr[CTR_SUM_DONE] = 0;
+            v.ctr[CTR_COND_DONE] = 1;
+        }
+        return;
+    }
     const int conv = __syncthreads_or(control_clouds(v, threadIdx.x, blockDim.x));
     if (!conv) {
         // every cloud goes on: the work lists stay as they are
@@ -3205,9 +3212,31 @@ cudaError_t set_assign_attrs(int dyn)
                                 cudaFuncAttributeMaxDynamicSharedMemorySize, dyn);
 }
 
+// launch with programmatic stream serialisation (pdl != 0): the kernel may
+// start while the previous kernel on the stream drains; it waits in
+// pdl_enter(). Single-cloud passes (small, latency-bound grids) gain from it
+// (33.7 -> 33.5 ms per 1M-point helix solve); batches of thousands of clouds
+// lose 1% with it, so they launch plainly.
+template <typename... KArgs, typename... Args>
+static cudaError_t launch_pdl(int pdl, void (*kernel)(KArgs...), int grid, int block, size_t smem,
+                              cudaStream_t st, Args... args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = pdl ? 1 : 0;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
 // persistent grid of k_assign_cull: every resident CTA, at most one warp per block
 template <int DIM, int ITEMS>
-cudaError_t launch_assign_cull(const EngineView& v, cudaStream_t st)
+cudaError_t launch_assign_cull(const EngineView& v, int pdl, cudaStream_t st)
 {
     static std::atomic<int> per_sm{0};
     int b = per_sm.load(std::memory_order_relaxed);
@@ -3221,8 +3250,7 @@ cudaError_t launch_assign_cull(const EngineView& v, cudaStream_t st)
     if (wpc < 1 || (wpc & (wpc - 1))) return cudaErrorInvalidValue;  // the kernel's block numbers need 2^k
     const int64_t ctas = ((int64_t)v.n_chunks * wpc + AC_WARPS - 1) / AC_WARPS;
     const int g = (int)std::max<int64_t>(1, std::min<int64_t>(ctas, (int64_t)v.n_sms * b));
-    k_assign_cull<DIM, ITEMS><<<g, AC_BLOCK, 0, st>>>(v);
-    return cudaGetLastError();
+    return launch_pdl(pdl, k_assign_cull<DIM, ITEMS>, g, AC_BLOCK, 0, st, v);
 }
 
 // grid of k_merge_fold: every resident CTA, at most one per chosen point
@@ -3258,42 +3286,21 @@ cudaError_t prepare_pass_dim(const EngineView& v, const TuneParams& tp)
                                 scatter_cta_smem_bytes(v));
 }
 
-// launch with programmatic stream serialisation (pdl != 0): the kernel may
-// start while the previous kernel on the stream drains; it waits in
-// pdl_enter(). Single-cloud passes (small, latency-bound grids) gain from it
-// (33.7 -> 33.5 ms per 1M-point helix solve); batches of thousands of clouds
-// lose 1% with it, so they launch plainly.
-template <typename... KArgs, typename... Args>
-static cudaError_t launch_pdl(int pdl, void (*kernel)(KArgs...), int grid, int block, size_t smem,
-                              cudaStream_t st, Args... args)
-{
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(block);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = pdl ? 1 : 0;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, args...);
-}
-
 // the kernels of an evolve pass; control: see k_merge_fold
 template <int DIM>
 cudaError_t launch_evolve_kernels(const EngineView& v, const TuneParams& tp, int assign_grid,
                                   const LoopCond& lc, int control, cudaStream_t st,
-                                  cudaEvent_t a0 = nullptr, cudaEvent_t a1 = nullptr)
+                                  cudaEvent_t a0 = nullptr, cudaEvent_t a1 = nullptr,
+                                  int assign_pdl = 0)
 {
     const int hist_bytes = v.hist_smem * 4;
     const int sms = v.n_sms;
     if (a0) cudaEventRecord(a0, st);
     if (v.cull) {
         cudaError_t e;
-        if (tp.cull_items == 2) e = launch_assign_cull<DIM, 2>(v, st);
-        else if (tp.cull_items == 8) e = launch_assign_cull<DIM, 8>(v, st);
-        else e = launch_assign_cull<DIM, 4>(v, st);
+        if (tp.cull_items == 2) e = launch_assign_cull<DIM, 2>(v, assign_pdl, st);
+        else if (tp.cull_items == 8) e = launch_assign_cull<DIM, 8>(v, assign_pdl, st);
+        else e = launch_assign_cull<DIM, 4>(v, assign_pdl, st);
         if (e != cudaSuccess) return e;
     } else {
 #define RD_ASSIGN_CASE(B, I)                                                                  \
@@ -3334,11 +3341,12 @@ cudaError_t launch_evolve_kernels(const EngineView& v, const TuneParams& tp, int
 
 template <int DIM>
 cudaError_t launch_pass_dim(const EngineView& v, const TuneParams& tp, int assign_grid,
-                            const LoopCond& lc, cudaStream_t st, cudaEvent_t a0, cudaEvent_t a1)
+                            const LoopCond& lc, cudaStream_t st, cudaEvent_t a0, cudaEvent_t a1,
+                            bool follows_pass)
 {
     const int pdl = v.n_clouds == 1;
-    const cudaError_t e =
-        launch_evolve_kernels<DIM>(v, tp, assign_grid, lc, MF_CONTROL, st, a0, a1);
+    const cudaError_t e = launch_evolve_kernels<DIM>(v, tp, assign_grid, lc, MF_CONTROL, st, a0, a1,
+                                                     pdl && follows_pass);
     if (e != cudaSuccess) return e;
     return launch_pdl(pdl, k_decimate<DIM, 512>, std::min(v.n_groups, v.n_sms * 2), 512,
                       dec_smem_bytes(v), st, v, lc.h, 1, lc.use_handle);
@@ -3425,10 +3433,11 @@ cudaError_t prepare_pass(int dim, const EngineView& v, const TuneParams& tp)
 }
 
 cudaError_t launch_pass(int dim, const EngineView& v, const TuneParams& tp, int assign_grid,
-                        const LoopCond& lc, cudaStream_t st, cudaEvent_t a0, cudaEvent_t a1)
+                        const LoopCond& lc, cudaStream_t st, cudaEvent_t a0, cudaEvent_t a1,
+                        bool follows_pass)
 {
     return with_dim(dim, [&](auto D) {
-        return launch_pass_dim<decltype(D)::value>(v, tp, assign_grid, lc, st, a0, a1);
+        return launch_pass_dim<decltype(D)::value>(v, tp, assign_grid, lc, st, a0, a1, follows_pass);
     });
 }
 
