@@ -1681,13 +1681,13 @@ __device__ float fold_rows(const float* __restrict__ rows, const int n, float* b
 // region of the grouped lists, from pass to pass.  In a cloud that regroups
 // (rebuilds) the scatter has just written the lists anew; otherwise the key's
 // edits of this pass are merged in.  The edits are sorted by position in shared
-// memory (each counts the smaller ones).  Seven warps take the old list in
-// chunks of MF_ROWS rows, the next two chunks' loads in flight.  The position of
+// memory (each counts the smaller ones).  All warps but one take the old list in
+// chunks of one row per thread, the next two chunks' loads in flight.  The position of
 // each chunk's first row says which edits fall into the chunk; a row finds by
 // binary search how many of them come before it, which gives its new place (or
 // that it leaves), and takes along the points that join right before it; a
 // chunk without edits moves as a whole.  New rows go to a ring in shared memory
-// and to the other buffer; the eighth warp folds the ring behind them with the
+// and to the other buffer; the last warp folds the ring behind them with the
 // reference's chain of rounded adds (lane d: coordinate d;
 // rd/cpu/brute_force/evolve.hpp:71-74) and applies the movement test
 // (evolve.hpp:143-177).  A list that outgrows its region is folded all the
@@ -1700,24 +1700,26 @@ __device__ float fold_rows(const float* __restrict__ rows, const int n, float* b
 // 1,266 members, most with edits), 12-20 us (few keys with edits), 45-50 us (116
 // keys of 8,300 members, 20 us of it the add chain of the longest).
 // ---------------------------------------------------------------------------
-constexpr int MF_BLOCK = 256;
-constexpr int MF_PROD = MF_BLOCK - 32;      // threads that merge
-constexpr int MF_ROWS = MF_PROD;            // rows per chunk, one per thread
+// CTA size: 256 threads for one cloud; 128 for several, whose pass has thousands
+// of short lists, each a chain of loads and barriers: seven CTAs per SM instead
+// of four (2,048 clouds: 635 -> 600 ms)
+constexpr int MF_BLOCK = 256, MF_BLOCK_MANY = 128;
 constexpr int MF_RING = 1024;               // two chunks and every edit fit
 constexpr int MF_STAGES = 3;                // chunks of the old list in flight
 constexpr int MF_CUTS = 256;                // chunks whose edits are looked up at once
 constexpr int MF_CHAIN = 32;                // terms the chain takes at a time
-static_assert(2 * MF_ROWS + EDIT_MAX + MF_CHAIN <= MF_RING && MF_RING % MF_CHAIN == 0,
+static_assert(2 * (MF_BLOCK - 32) + EDIT_MAX + MF_CHAIN <= MF_RING && MF_RING % MF_CHAIN == 0,
               "ring of new rows");
 
-template <int DIM>
+template <int DIM, int BLOCK>
 struct MergeSmem {
+    static constexpr int PROD = BLOCK - 32;   // threads that merge, rows per chunk
     union {
         float ring[DIM][MF_RING + 4];   // per coordinate: the chain loads four terms at once
-        SegFoldSmem<MF_BLOCK / 32, DIM> seg;
+        SegFoldSmem<BLOCK / 32, DIM> seg;
     };
-    alignas(16) float old[MF_STAGES][MF_ROWS * PadDim<DIM>::v];   // chunks of the old list
-    int pos[MF_STAGES][MF_ROWS + 1];                  // their positions, after the row before's
+    alignas(16) float old[MF_STAGES][PROD * PadDim<DIM>::v];   // chunks of the old list
+    int pos[MF_STAGES][PROD + 1];                     // their positions, after the row before's
     alignas(16) float joins[EDIT_MAX * PadDim<DIM>::v];   // coordinates of the joining edits
     int raw[EDIT_MAX];        // edits as listed
     int ed[EDIT_MAX];         // by position
@@ -1846,17 +1848,17 @@ __device__ __noinline__ float chain_tail(const uint32_t a, const int m, float su
 }
 
 // apart, so that its registers do not weigh on the merge
-template <int DIM>
-__device__ __noinline__ void fold_long_list(const float* rows, const int n,
-                                            SegFoldSmem<MF_BLOCK / 32, DIM>& sm)
+template <int DIM, int W>
+__device__ __noinline__ void fold_long_list(const float* rows, const int n, SegFoldSmem<W, DIM>& sm)
 {
-    fold_members_seg_src<MF_BLOCK / 32, DIM>(RowSrc<DIM>{rows}, n, sm);
+    fold_members_seg_src<W, DIM>(RowSrc<DIM>{rows}, n, sm);
 }
 
-template <int DIM>
+template <int DIM, int BLOCK>
 __device__ void merge_fold_key(const EngineView& v, const int slot, const bool seg_ok,
-                               MergeSmem<DIM>& sm)
+                               MergeSmem<DIM, BLOCK>& sm)
 {
+    constexpr int MF_PROD = BLOCK - 32, MF_ROWS = MF_PROD;
     constexpr int DP = PadDim<DIM>::v;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int c = v.single ? 0 : v.slot_cloud[slot];
@@ -1872,9 +1874,9 @@ __device__ void merge_fold_key(const EngineView& v, const int slot, const bool s
     const int ne = fresh ? 0 : edits;          // at most EDIT_MAX, or the cloud rebuilds
     const float* src = v.Lr[par] + at * DP;
     __syncthreads();  // the previous key's scratch, and its state, are read no more
-    for (int i = tid; i < ne; i += MF_BLOCK) sm.raw[i] = v.edit[at + i];
+    for (int i = tid; i < ne; i += BLOCK) sm.raw[i] = v.edit[at + i];
     __syncthreads();
-    for (int i = tid; i < ne; i += MF_BLOCK) {
+    for (int i = tid; i < ne; i += BLOCK) {
         const int e = sm.raw[i], x = e & ~EDIT_IN;
         int r = 0;
         float p[DIM];
@@ -1903,7 +1905,7 @@ __device__ void merge_fold_key(const EngineView& v, const int slot, const bool s
     const int32_t* pos = v.cull ? v.Ls[par] + at : nullptr;
     // edits before chunk s's first row (those before the list's first row go to chunk 0)
     auto find_cuts = [&](const int s0) {
-        for (int i = tid; i <= MF_CUTS; i += MF_BLOCK) {
+        for (int i = tid; i <= MF_CUTS; i += BLOCK) {
             const int s = s0 + i;
             sm.cut[i] = (s == 0 || ne == 0) ? 0
                         : (s < steps) ? edits_below(sm.ed, 0, ne, pos[s * MF_ROWS]) : ne;
@@ -2012,7 +2014,7 @@ __device__ void merge_fold_key(const EngineView& v, const int slot, const bool s
     if (seg) {
         const float* rows = (ne > 0) ? v.Lr[par ^ 1] + at * DP : src;
         __syncthreads();  // the ring is read no more
-        fold_long_list<DIM>(rows, n_new, sm.seg);
+        fold_long_list<DIM, BLOCK / 32>(rows, n_new, sm.seg);
         if (warp == 0 && lane < DIM) sum = sm.seg.out[lane];
     }
     if (warp == 0) {
@@ -2033,16 +2035,16 @@ __device__ void merge_fold_key(const EngineView& v, const int slot, const bool s
 // same clouds): make ready for the next pass.
 enum : int { MF_CONTROL = 1, MF_STEP = 2 };
 
-template <int DIM>
-__global__ void __launch_bounds__(MF_BLOCK, 4) k_merge_fold(EngineView v, cudaGraphConditionalHandle h,
+template <int DIM, int BLOCK>
+__global__ void __launch_bounds__(BLOCK, BLOCK == MF_BLOCK ? 4 : 7) k_merge_fold(EngineView v, cudaGraphConditionalHandle h,
                                                             int control, int use_handle)
 {
     pdl_enter();
-    __shared__ __align__(16) MergeSmem<DIM> sm;
+    __shared__ __align__(16) MergeSmem<DIM, BLOCK> sm;
     __shared__ int s_last;
     const int nd = v.ctr[CTR_NDIRTY];
     for (int t = blockIdx.x; t < nd; t += gridDim.x)
-        merge_fold_key<DIM>(v, v.dlist[t], nd <= (int)gridDim.x, sm);
+        merge_fold_key<DIM, BLOCK>(v, v.dlist[t], nd <= (int)gridDim.x, sm);
     // every thread's writes (chosen points, moved flags) before the count
     __threadfence();
     __syncthreads();
@@ -3254,13 +3256,13 @@ cudaError_t launch_assign_cull(const EngineView& v, int pdl, cudaStream_t st)
 }
 
 // grid of k_merge_fold: every resident CTA, at most one per chosen point
-template <int DIM>
+template <int DIM, int BLOCK>
 int merge_grid(const EngineView& v)
 {
     static std::atomic<int> per_sm{0};
     int b = per_sm.load(std::memory_order_relaxed);
     if (b == 0) {
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_merge_fold<DIM>, MF_BLOCK, 0) !=
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_merge_fold<DIM, BLOCK>, BLOCK, 0) !=
                 cudaSuccess || b < 1)
             b = 1;
         per_sm.store(b, std::memory_order_relaxed);
@@ -3331,8 +3333,12 @@ cudaError_t launch_evolve_kernels(const EngineView& v, const TuneParams& tp, int
                        scatter_cta_smem_bytes(v), st, v);
     if (e != cudaSuccess) return e;
     if (v.n_slots > 0) {
-        e = launch_pdl(pdl, k_merge_fold<DIM>, merge_grid<DIM>(v), MF_BLOCK, 0, st, v, lc.h, control,
-                       lc.use_handle);
+        if (v.n_clouds == 1)
+            e = launch_pdl(pdl, k_merge_fold<DIM, MF_BLOCK>, merge_grid<DIM, MF_BLOCK>(v), MF_BLOCK, 0,
+                           st, v, lc.h, control, lc.use_handle);
+        else
+            e = launch_pdl(pdl, k_merge_fold<DIM, MF_BLOCK_MANY>, merge_grid<DIM, MF_BLOCK_MANY>(v),
+                           MF_BLOCK_MANY, 0, st, v, lc.h, control, lc.use_handle);
     } else {
         e = launch_pdl(pdl, k_control, std::min((v.n_clouds + 255) / 256, sms), 256, 0, st, v);
     }
