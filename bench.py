@@ -46,13 +46,14 @@ METRIC = "evolve pairs/s"
 UNIT = "pairs/s"
 # DRAM traffic of one assignment launch on the helix3d_1m workload, from one
 # ncu capture each (dram__bytes_read.sum + dram__bytes_write.sum):
-#   k_assign_cull (culled, the default): 16,034,816 + 0 bytes against 20 B of
-#     algorithmic traffic per point (12 B sorted point + 4 B slot read, 4 B key
-#     written, the keys staying in L2);
+#   k_assign_cull (culled, the default) evaluates only the blocks of points whose
+#     keys can have changed, so one launch stands for no other and none is
+#     given; the 20 B per point (12 B sorted point + 4 B slot read, 4 B key
+#     written) are what a launch that evaluates every point needs;
 #   k_assign (all pairs): 12,039,936 + 0 bytes, the 1,000,000 points x 12 B
 #     read once.
 # Applies to helix3d_1m only.
-ASSIGN_TRAFFIC_BYTES = {"helix3d_1m": 16_034_816}
+ASSIGN_TRAFFIC_BYTES = {}
 ALL_PAIRS_TRAFFIC_BYTES = {"helix3d_1m": 12_039_936}
 
 
@@ -388,7 +389,8 @@ def run_b200_bf(args, world, rank, local):
     L.check(lib.rd_probe_fp32_peak(ctypes.byref(peak), ctypes.c_void_p(stream.cuda_stream)))
     nominal = 148 * 128 * 2 * 1.965e9 / 1e12
     hbm_peak, hbm_src = measured_hbm_gbs()
-    # culled kernel: per point a sorted point and its slot read, its key written
+    # culled kernel, when it evaluates every point: a sorted point and its slot
+    # read, its key written (an average launch evaluates fewer)
     cull_bytes = n * (4 * dim + 4 + 4)
     cull_gbs = cull_bytes / (assign_ms_avg * 1e-3) / 1e9
     all_pairs = {"kernel": "k_assign", "bound": "fp32", "achieved": ap_tflops,
