@@ -523,6 +523,7 @@ int Engine::run(cudaStream_t st, bool use_graph, int mode)
 {
     if (h_cl_.empty()) return 0;
     stats_ = RunStats();
+    read_switches();
     flags_ = (mode == RUN_EVOLVE_ONLY) ? ENG_EVOLVE_ONLY : 0;
     RD_CK(upload(bCl_, h_cl_, st));
     RD_CK(upload(bGr_, h_gr_, st));
@@ -648,10 +649,18 @@ int Engine::start_passes(cudaStream_t st)
     return 0;
 }
 
+// Another thread may flip the switch at any time, and both the layout of the
+// grouped lists (finish_setup_after_choose) and the choice of kernels and buffers
+// follow from it: every run reads it once.
+void Engine::read_switches()
+{
+    cull_on_ = cull_assign && assign_cull_enabled();
+}
+
 // whether the lockstep passes of this batch assign with culling
 bool Engine::cull_possible() const
 {
-    return cull_assign && cull_allowed_ && assign_cull_enabled() && spatial_ok_ && total_points_ > 0;
+    return cull_on_ && cull_allowed_ && spatial_ok_ && total_points_ > 0;
 }
 
 // buffers of the culled assignment (sizes known after choose)
@@ -715,6 +724,7 @@ int Engine::plan_workspace(int mode)
         last_error = "workspace planning needs a measuring arena";
         return 1;
     }
+    read_switches();
     // the buffers run() takes, in its order, for a single-cloud device step
     RD_CK(upload(bCl_, h_cl_, nullptr));
     RD_CK(upload(bGr_, h_gr_, nullptr));
@@ -758,6 +768,7 @@ int Engine::adjoint_setup(cudaStream_t st)
     stats_ = RunStats();
     flags_ = ENG_ALWAYS_MOVE;
     fused_ = false;
+    read_switches();
     cull_ = cull_possible();
     RD_CK(upload(bCl_, h_cl_, st));
     RD_CK(upload(bGr_, h_gr_, st));

@@ -151,6 +151,8 @@ private:
     int finish_setup_after_choose(cudaStream_t st, bool ns_given = false);
     // per cloud 64-bit pairs and 32-bit chosen count, passes and errors; then the counters
     static size_t res_bytes(size_t nc) { return 20 * (nc + 1) + 4 * CTR_COUNT; }
+    // once per run: the process-wide culling switch as this run takes it
+    void read_switches();
     bool cull_possible() const;
     int ensure_cull_buffers();
     int start_passes(cudaStream_t st);
@@ -185,6 +187,7 @@ private:
     int dec_smem_max_ = 0;
     int dec_nb_pp_ = DEC_NB_MIN_PER_POINT;
     bool fused_ = false;
+    bool cull_on_ = true;         // the culling switch when this run started
     bool cull_ = false;           // this run assigns with culling
     bool spatial_ok_ = false;     // the batch layout allows the spatial order
     bool cull_allowed_ = true;    // and its size, and the kind of run, the culled assignment
