@@ -4,6 +4,7 @@
 #pragma once
 
 #include "rd_internal.cuh"
+#include "rd_listfit.hpp"
 
 namespace rdb {
 namespace {
@@ -374,7 +375,8 @@ __device__ void decimate_scan_lists(const float* X, const int total, const float
     // candidate bitmap (alive and removable right now), 16-byte aligned after the flags
     uint32_t* cand = reinterpret_cast<uint32_t*>(
         smem + ((2 * sizeof(int16_t) * smem_max + smem_max + 15) / 16) * 16);
-    __shared__ int s_carry, s_overflow;
+    __shared__ int s_overflow;
+    __shared__ int64_t s_total;
     __shared__ int s_w[BLOCK / 32];
 
     if (prepared) {  // buckets, counts and lists were built by the GPU-wide kernels
@@ -389,7 +391,7 @@ __device__ void decimate_scan_lists(const float* X, const int total, const float
         __syncthreads();
     } else {
     for (int h = tid; h <= (int)hmask + 1; h += BLOCK) bstart[h] = 0;
-    if (tid == 0) { s_carry = 0; s_overflow = 0; }
+    if (tid == 0) { s_total = 0; s_overflow = 0; }
     __syncthreads();
     for (int i = tid; i < total; i += BLOCK) {
         int cc[DIM];
@@ -447,7 +449,7 @@ __device__ void decimate_scan_lists(const float* X, const int total, const float
     // exclusive prefix of list lengths
     for (int i0 = 0; i0 < total; i0 += BLOCK) {
         const int i = i0 + tid;
-        const int x = (i < total) ? nb_off[i] : 0;
+        const int x = (i < total) ? list_len(nb_off[i]) : 0;
         int incl = x;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -456,20 +458,20 @@ __device__ void decimate_scan_lists(const float* X, const int total, const float
         }
         if (lane == 31) s_w[warp] = incl;
         __syncthreads();
-        int pre = 0, tot = 0;
+        int64_t pre = 0, tot = 0;
         for (int w = 0; w < BLOCK / 32; ++w) {
             pre += (w < warp) ? s_w[w] : 0;
             tot += s_w[w];
         }
-        const int carry = s_carry;
-        if (i < total) nb_off[i] = carry + pre + incl - x;
+        const int64_t carry = s_total;
+        if (i < total) nb_off[i] = (int)(carry + pre + incl - x);
         __syncthreads();
-        if (tid == 0) s_carry = carry + tot;
+        if (tid == 0) s_total = carry + tot;
         __syncthreads();
     }
     if (tid == 0) {
-        nb_off[total] = s_carry;
-        s_overflow = (int64_t)s_carry > nb_cap;
+        nb_off[total] = (int)s_total;
+        s_overflow = !lists_fit(s_total, nb_cap);
     }
     __syncthreads();
     if (s_overflow) {  // lists do not fit: bucket-walk version

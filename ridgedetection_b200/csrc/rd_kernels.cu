@@ -2830,7 +2830,7 @@ __global__ void __launch_bounds__(1024) k_decbig_scan_lists(EngineView v)
 {
     if (v.dbig[0] != 1) return;
     __shared__ int s_w[32];
-    __shared__ int s_carry;
+    __shared__ int64_t s_carry;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int g = v.dbig[1], total = v.dbig[2];
     const GroupDesc gd = v.gr[g];
@@ -2839,7 +2839,7 @@ __global__ void __launch_bounds__(1024) k_decbig_scan_lists(EngineView v)
     __syncthreads();
     for (int i0 = 0; i0 < total; i0 += 1024) {
         const int i = i0 + tid;
-        const int x = (i < total) ? nb_off[i] : 0;
+        const int x = (i < total) ? list_len(nb_off[i]) : 0;
         int incl = x;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -2848,20 +2848,20 @@ __global__ void __launch_bounds__(1024) k_decbig_scan_lists(EngineView v)
         }
         if (lane == 31) s_w[warp] = incl;
         __syncthreads();
-        int pre = 0, tot = 0;
+        int64_t pre = 0, tot = 0;
         for (int w = 0; w < 32; ++w) {
             pre += (w < warp) ? s_w[w] : 0;
             tot += s_w[w];
         }
-        const int carry = s_carry;
-        if (i < total) nb_off[i] = carry + pre + incl - x;
+        const int64_t carry = s_carry;
+        if (i < total) nb_off[i] = (int)(carry + pre + incl - x);
         __syncthreads();
         if (tid == 0) s_carry = carry + tot;
         __syncthreads();
     }
     if (tid == 0) {
-        nb_off[total] = s_carry;
-        if ((int64_t)s_carry > (int64_t)v.dec_nb_pp * gd.s_cap) v.dbig[0] = 2;
+        nb_off[total] = (int)s_carry;
+        if (!lists_fit(s_carry, (int64_t)v.dec_nb_pp * gd.s_cap)) v.dbig[0] = 2;
     }
 }
 
