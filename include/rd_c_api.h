@@ -61,7 +61,7 @@ typedef struct rd_run_stats {
     int64_t max_passes;     /* evolve passes of the cloud that needed most           */
     double  pairs;          /* sum over passes of (cloud points x chosen points)     */
     int32_t err_bits;       /* device error bits (0 when clean)                      */
-    int32_t pad;
+    int32_t handed_tiles;   /* tiled runs: light tiles handed over to a cluster      */
     double  assign_ms;      /* profiling runs only: summed assign-kernel time (ms)   */
     int64_t assign_launches;/* profiling runs only: assign-kernel launches timed     */
     double  point_passes;   /* sum over clouds of (points x evolve passes): point   */
@@ -111,8 +111,12 @@ RD_API rd_status rd_get_assign_cull(int* enable);
  * instead of one CTA, and each of its keys with at least seg_min members is
  * folded in 64 warp segments (8 per CTA) whose exact FP32 sums are composed
  * in index order.
- * enable = 0: one CTA per tile.  0 for a threshold keeps its default (100,000
- * points, 8,192 members).  Process-wide, read when a run starts. */
+ * enable = 0: one CTA per tile.  A threshold of 0 (the default) leaves it to a rule:
+ * min_points is then a (4 x SMs)-th of the run's evolve points, at least 4,096 and
+ * at most 100,000, single CTAs may hand tiles over to their cluster once no light
+ * tile waits, and seg_min is 12,288.  Any other value holds as given, and a tile
+ * below it stays on one CTA.  rd_get_tile_clusters answers 100,000 and 8,192 for
+ * thresholds left to the rule.  Process-wide, read when a run starts. */
 RD_API rd_status rd_set_tile_clusters(int enable, int64_t min_points, int64_t seg_min);
 RD_API rd_status rd_get_tile_clusters(int* enable, int64_t* min_points, int64_t* seg_min);
 /* Times the supported shapes of the assignment the run would use (culled or

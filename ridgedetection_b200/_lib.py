@@ -38,7 +38,7 @@ class RDError(RuntimeError):
 class RunStats(ctypes.Structure):
     _fields_ = [("loop_iters", ctypes.c_int64), ("evolve_passes", ctypes.c_int64),
                 ("max_passes", ctypes.c_int64), ("pairs", ctypes.c_double),
-                ("err_bits", ctypes.c_int32), ("pad", ctypes.c_int32),
+                ("err_bits", ctypes.c_int32), ("handed_tiles", ctypes.c_int32),
                 ("assign_ms", ctypes.c_double), ("assign_launches", ctypes.c_int64),
                 ("point_passes", ctypes.c_double), ("dec_passes", ctypes.c_int64),
                 ("dec_rounds", ctypes.c_int64)]

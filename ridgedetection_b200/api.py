@@ -352,8 +352,9 @@ def get_assign_cull() -> bool:
 def set_tile_clusters(enable: bool, min_points: int = 0, seg_min: int = 0) -> None:
     """Cluster evolve of heavy tiles in tiled runs (changes no result): tiles
     with at least min_points evolve points are evolved by a thread-block
-    cluster, keys with at least seg_min members folded in segments across it
-    (0 = default threshold).  Process-wide."""
+    cluster, keys with at least seg_min members folded in segments across it.
+    0 leaves a threshold to a rule over the run's points (rd_c_api.h); any other
+    value holds as given.  Process-wide."""
     L.check(L.lib().rd_set_tile_clusters(1 if enable else 0, int(min_points), int(seg_min)))
 
 

@@ -164,6 +164,7 @@ void fill_stats(const RunStats& s, rd_run_stats* o)
     o->point_passes = s.point_passes;
     o->dec_passes = s.dec_passes;
     o->dec_rounds = s.dec_rounds;
+    o->handed_tiles = (int32_t)s.handed_tiles;
 }
 
 // independent FMA chains: 8 per thread, ITER rounds
@@ -305,9 +306,7 @@ rd_status rd_set_tile_clusters(int enable, int64_t min_points, int64_t seg_min)
 {
     if (min_points < 0 || seg_min < 0 || min_points > INT32_MAX || seg_min > INT32_MAX)
         return set_err(RD_ERR_ARG, "negative or too large threshold");
-    const TileClusterParams d = tile_cluster_defaults();
-    set_tile_cluster_params(TileClusterParams{enable != 0, min_points ? (int)min_points : d.min_points,
-                                              seg_min ? (int)seg_min : d.seg_min});
+    set_tile_cluster_params(TileClusterParams{enable != 0, (int)min_points, (int)seg_min});
     return RD_OK;
 }
 
@@ -316,8 +315,8 @@ rd_status rd_get_tile_clusters(int* enable, int64_t* min_points, int64_t* seg_mi
     if (!enable || !min_points || !seg_min) return set_err(RD_ERR_ARG, "null argument");
     const TileClusterParams p = tile_cluster_params();
     *enable = p.enabled ? 1 : 0;
-    *min_points = p.min_points;
-    *seg_min = p.seg_min;
+    *min_points = p.min_points > 0 ? p.min_points : TCL_MIN_POINTS;
+    *seg_min = p.seg_min > 0 ? p.seg_min : TSEG_MIN;
     return RD_OK;
 }
 

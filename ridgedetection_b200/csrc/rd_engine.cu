@@ -362,6 +362,7 @@ EngineView Engine::view() const
     v.tile_order = bTileOrder_.as<int32_t>();
     v.n_heavy = n_heavy_;
     v.tile_clusters = tile_clusters_ ? 1 : 0;
+    v.tile_hand = tile_hand_ ? 1 : 0;
     v.tile_cl_grid = tile_cl_grid_;
     v.tile_seg_min = tile_seg_min_;
     v.n_sms = sms_;
@@ -695,26 +696,14 @@ void Engine::build_tile_order()
     for (size_t c = 0; c < nc; ++c) h_tile_order_[c] = (int32_t)c;
     std::stable_sort(h_tile_order_.begin(), h_tile_order_.end(),
                      [&](int32_t a, int32_t b) { return h_cl_[a].n_all > h_cl_[b].n_all; });
+    const TileRule rule = tile_rule(tile_cluster_params(), total_points_, sms_,
+                                    nc > 1 ? h_cl_[h_tile_order_[0]].n_all : 0);
+    tile_seg_min_ = rule.seg_min;
+    tile_clusters_ = rule.clusters && nc > 1;
+    tile_hand_ = rule.hand_over && nc > 1;
     n_heavy_ = 0;
-    const TileClusterParams tp = tile_cluster_params();
-    tile_seg_min_ = std::max(1, tp.seg_min == tile_cluster_defaults().seg_min ? tp.seg_min * 3 / 2 : tp.seg_min);
-    // With the default threshold a tile is also heavy from a 4 x SMs-th of all
-    // evolve points on (half of what each of the resident CTAs would get): a
-    // larger one evolved by one CTA outlasts the other tiles.  Below 4,096 points
-    // one CTA's passes are shorter than the cluster's barriers.  And with the
-    // default threshold a key is folded in segments from 12,288 members on, not
-    // 8,192: where its coordinates lie on both sides of zero the segments' runs
-    // break at every change of binade, and one warp's add chain is faster.  Whole
-    // solves, ms, thresholds of 100,000 points and 8,192 members / these rules with
-    // the hand-over of rd_tile_cluster.cuh: 1M spiral in 70 leaves 190 / 35, in
-    // 1,024 tiles 46 / 18, 2M in 582 leaves 69 / 32, 300,000 in 256 tiles 48 / 17;
-    // the 10M spiral in 4,096 tiles keeps its 100,000 (34.9 / 32.7; 48 with 10,000).
-    int64_t min_points = tp.min_points;
-    if (tp.min_points == tile_cluster_defaults().min_points)
-        min_points = std::min(min_points, std::max<int64_t>(4096, total_points_ / (4 * sms_)));
-    tile_clusters_ = tp.enabled && nc > 1 && h_cl_[h_tile_order_[0]].n_all >= 4096;
-    if (tp.enabled && nc > 1)
-        while (n_heavy_ < (int)nc && h_cl_[h_tile_order_[n_heavy_]].n_all >= min_points) ++n_heavy_;
+    if (tile_clusters_)
+        while (n_heavy_ < (int)nc && h_cl_[h_tile_order_[n_heavy_]].n_all >= rule.heavy) ++n_heavy_;
 }
 
 int Engine::plan_workspace(int mode)
@@ -814,6 +803,7 @@ int Engine::collect(cudaStream_t st)
     h_err_.assign(er, er + nc);
     stats_.loop_iters = ctr[CTR_ITERS];
     stats_.err_bits = ctr[CTR_ERR];
+    stats_.handed_tiles = ctr[CTR_HANDED];
     stats_.dec_passes = ctr[CTR_DEC_PASSES];
     stats_.dec_rounds = ctr[CTR_DEC_ROUNDS];
     for (size_t c = 0; c < nc; ++c) {

@@ -14,6 +14,7 @@
 #pragma once
 
 #include "rd_internal.cuh"
+#include "rd_tile_rule.hpp"
 
 #include <cstddef>
 #include <cstdint>
@@ -61,7 +62,8 @@ enum : int {
     CTR_DEC_PASSES = 10,  // decimation passes resolved in parallel rounds (this run)
     CTR_DEC_ROUNDS = 11,  // rounds they took
     CTR_COND_DONE = 12,   // k_merge_fold ended this iteration (no group was ready)
-    CTR_COUNT = 13,
+    CTR_HANDED = 13,      // light tiles handed over to a cluster (this run)
+    CTR_COUNT = 14,
 };
 
 struct EngineView {
@@ -161,7 +163,8 @@ struct EngineView {
     // evolved by whole thread-block clusters (rd_tile_cluster.cuh)
     const int32_t* tile_order;
     int32_t n_heavy;
-    int32_t tile_clusters;       // tiles large enough for the cluster kernel
+    int32_t tile_clusters;       // the cluster kernel runs
+    int32_t tile_hand;           // and hands over light tiles
     int32_t tile_cl_grid;        // CTAs of the cluster tile kernel (0 = one-CTA kernel)
     int32_t tile_seg_min;        // members of a key the cluster folds in segments
 };
@@ -185,18 +188,10 @@ struct TuneParams {
 
 // host-side launchers (rd_kernels.cu); all enqueue on `st`
 cudaError_t launch_choose(int dim, const EngineView& v, cudaStream_t st);
-// The cluster path of fused tiled runs (process-wide, read when a run
-// starts): on/off (off = one CTA per tile), the evolve points from which a
-// tile is evolved by a whole cluster and the members from which a key is
-// folded in segments across it.
-struct TileClusterParams {
-    bool enabled;
-    int min_points;
-    int seg_min;
-};
+// the settings of the cluster path of fused tiled runs (process-wide, read when a
+// run starts; rd_tile_rule.hpp)
 TileClusterParams tile_cluster_params();
 void set_tile_cluster_params(const TileClusterParams& p);
-TileClusterParams tile_cluster_defaults();
 // choose of one large cloud c (n own points) in GPU-wide rounds; v.hash must
 // hold choose_hash_buckets() ints and surv n bytes
 cudaError_t launch_choose_rounds(int dim, const EngineView& v, int c, int n, uint8_t* surv,

@@ -57,6 +57,7 @@ struct RunStats {
     double point_passes = 0;      // sum over clouds of n_all * evolve passes
     int64_t dec_passes = 0;       // decimation passes resolved in parallel rounds
     int64_t dec_rounds = 0;       // rounds they took
+    int64_t handed_tiles = 0;     // tiled runs: light tiles handed over to a cluster
 };
 
 // Process-wide tuning table: (dim, size bucket, r1 bucket) -> assignment
@@ -200,6 +201,7 @@ private:
     std::vector<int32_t> h_tile_order_;
     int n_heavy_ = 0;
     bool tile_clusters_ = false;  // fused tiled runs: the cluster kernel
+    bool tile_hand_ = false;      // and its hand-over of light tiles
     int tile_cl_grid_ = 0;
     int tile_seg_min_ = 1 << 30;
     DevBuf bDx_, bDcell_, bDalive_, bDc1_, bDc2_, bDbstart_, bDitems_, bDecHoff_, bDecHbits_;

@@ -3454,8 +3454,7 @@ cudaError_t launch_loopcond(const EngineView& v, cudaGraphConditionalHandle h, i
     return cudaGetLastError();
 }
 
-static std::atomic<int> g_tile_cl_on{1}, g_tile_cl_min{TCL_MIN_POINTS}, g_tile_seg_min{TSEG_MIN};
-TileClusterParams tile_cluster_defaults() { return TileClusterParams{true, TCL_MIN_POINTS, TSEG_MIN}; }
+static std::atomic<int> g_tile_cl_on{1}, g_tile_cl_min{0}, g_tile_seg_min{0};
 TileClusterParams tile_cluster_params()
 {
     return TileClusterParams{g_tile_cl_on.load() != 0, g_tile_cl_min.load(), g_tile_seg_min.load()};
@@ -3510,7 +3509,7 @@ cudaError_t prepare_tile_pass(int dim, const EngineView& v, int* cl_grid)
                                              cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              tile_evolve_smem_bytes(DIM));
         if (e != cudaSuccess) return e;
-        if (v.n_heavy > 0 || v.tile_clusters) {
+        if (v.tile_clusters) {
             e = tile_cl_prepare<DIM>(cl_grid);
             if (e != cudaSuccess) return e;
         }

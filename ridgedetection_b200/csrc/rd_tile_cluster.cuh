@@ -42,8 +42,6 @@ namespace {
 namespace cg = cooperative_groups;
 
 constexpr int TCL = 8;                  // CTAs per cluster (portable size)
-constexpr int TCL_MIN_POINTS = 100000;  // default: evolve points of a tile evolved by a cluster
-constexpr int TSEG_MIN = 8192;          // default: members of a key folded across the cluster
 constexpr int TSEG_KEYS = 4;            // such keys per pass (the first in key order)
 constexpr int TCL_W = 8;                // warps per CTA of the cluster kernel (256 threads)
 
@@ -366,12 +364,15 @@ __global__ void __launch_bounds__(BLOCK) k_tile_evolve_cl(EngineView v)
         if (c < 0) break;
         if (v.phase[c] != PH_EVOLVE) continue;
         ClusterSmem<DIM>* c0 = cl.map_shared_rank(&cs, 0);
-        const bool can = v.cl[c].n_all >= TCL_HAND_MIN;
+        const bool can = v.tile_hand && v.cl[c].n_all >= TCL_HAND_MIN;
         const bool handed = tile_evolve_one<DIM, BLOCK>(v, c, FOLD_CTA_MIN_LIGHT, smem_raw, ts, [&] {
             return can && *reinterpret_cast<volatile int32_t*>(&v.ctr[CTR_WORK]) >= n_light &&
                    *reinterpret_cast<volatile int*>(&c0->idle) >= TCL_HAND_IDLE;
         });
-        if (handed && tid == 0) c0->req[atomicAdd(&c0->nreq, 1)] = c;
+        if (handed && tid == 0) {
+            c0->req[atomicAdd(&c0->nreq, 1)] = c;
+            atomicAdd(&v.ctr[CTR_HANDED], 1);
+        }
     }
     if (tid == 0) atomicAdd(&cl.map_shared_rank(&cs, 0)->idle, 1);
     // every write of a handed tile's CTA (its chosen points) before the cluster's reads

@@ -82,3 +82,19 @@ def test_handed_over_tiles_match_oracle(rdb, n, tiles):
     for mode in (rdb.LOOP_GRAPH, rdb.LOOP_HOST):
         S, st, _ = rdb.tiled_ridge_detection(P, 0.2, 0.4, n + 1, tiles, loop_mode=mode)
         assert st.err_bits == 0 and bits_equal(S, S_ref)
+
+
+def test_light_tiles_are_handed_over(rdb):
+    """The hand-over takes place (tens of tiles here), and the bits stay; with a threshold
+    given by the caller none is handed over."""
+    n, tiles = 200_000, (16, 16)
+    P = G.spiral2d(n, seed=47)
+    S_ref, _, _ = O.ridge_tiled(P, 0.2, 0.4, n + 1, tiles)
+    S, st, _ = rdb.tiled_ridge_detection(P, 0.2, 0.4, n + 1, tiles)
+    assert st.handed_tiles > 0 and bits_equal(S, S_ref)
+    rdb.set_tile_clusters(True, 5_000, 8192)
+    try:
+        S, st, _ = rdb.tiled_ridge_detection(P, 0.2, 0.4, n + 1, tiles)
+    finally:
+        rdb.set_tile_clusters(True, 0, 0)
+    assert st.handed_tiles == 0 and bits_equal(S, S_ref)
