@@ -29,6 +29,40 @@ __host__ __device__ inline int64_t dec_bits_matrix(int total)
     return (int64_t)8 * total * dec_bits_pitch(total);
 }
 
+// both in shared memory
+__host__ __device__ inline int64_t dec_matrix_bytes(int total)
+{
+    return (dec_bits_fixed(total) + 15) / 16 * 16 + dec_bits_matrix(total);
+}
+
+// Pairs of DEC_SAMPLES points of a set, spread over its order, with a point of it
+// within 2 r2 (themselves included), by the whole CTA, the same in every thread.
+// coord(i, d): coordinate d of point i.
+template <int DIM, int BLOCK, class F>
+__device__ int dec_near_samples(F&& coord, const int total, const float r2)
+{
+    __shared__ int s_near;
+    __syncthreads();   // coordinates are there, the last reader of s_near is done
+    if (threadIdx.x == 0) s_near = 0;
+    __syncthreads();
+    const float rsq4 = __fmul_rn(4.0f, sqr_rn(r2));
+    int near = 0;
+    for (int t = threadIdx.x; t < DEC_SAMPLES * total; t += BLOCK) {
+        const int i = (int)((int64_t)(t / total) * total / DEC_SAMPLES), j = t % total;
+        float p[DIM], q[DIM];
+#pragma unroll
+        for (int d = 0; d < DIM; ++d) {
+            p[d] = coord(i, d);
+            q[d] = coord(j, d);
+        }
+        near += sqdist_exact<DIM>(p, q) <= rsq4;
+    }
+    near = __reduce_add_sync(FULL, near);
+    if ((threadIdx.x & 31) == 0) atomicAdd(&s_near, near);
+    __syncthreads();
+    return s_near;
+}
+
 // mat: two matrices of total x dec_bits_pitch(total) words (shared or global
 // memory); smem: dec_bits_fixed(total) bytes.  alive[i] = 1 for the survivors.
 template <int DIM, int BLOCK>

@@ -175,6 +175,7 @@ struct EngineView {
 inline int dec_list_bytes(int points) { return ((points * 5 + 15) / 16) * 16 + 4 * ((points + 31) / 32) + 16; }
 constexpr int DEC_BITS_MAX = 4096;           // points decimated over bit matrices
 constexpr int DEC_BITS_SMEM = 200 * 1024;    // shared memory for them
+constexpr int DEC_SAMPLES = 32;              // points sampled for the choice between them and lists
 inline int dec_smem_bytes(const EngineView& v) { return v.dec_dyn; }
 // bytes for groups of up to `points` points
 int dec_dyn_bytes(int points);

@@ -2554,11 +2554,20 @@ __device__ void decimate_group(const EngineView& v, const int g)
     // small sets over bit matrices, in shared memory where they fit behind the
     // counts, else in the room of the neighbour lists
     const int64_t mat = dec_bits_matrix(total);
-    const bool bits_smem = (dec_bits_fixed(total) + 15) / 16 * 16 + mat <= v.dec_dyn;
-    const bool bits = !prepared && total <= DEC_BITS_MAX && dec_bits_fixed(total) <= v.dec_dyn &&
-                      (bits_smem || mat <= (int64_t)4 * v.dec_nb_pp * gd.s_cap);
+    const bool bits_smem = dec_matrix_bytes(total) <= v.dec_dyn;
+    bool bits = !prepared && total <= DEC_BITS_MAX && dec_bits_fixed(total) <= v.dec_dyn &&
+                (bits_smem || mat <= (int64_t)4 * v.dec_nb_pp * gd.s_cap);
+    __syncthreads();   // X is complete
+    // Matrices in global memory cost the square of the points whatever lies near them,
+    // the lists' walks (thread per point, 3^DIM cells each) grow with the neighbours.
+    // 2D, 1,500 / 3,000 / 4,096 points, us, lists / matrices: 12 neighbours within 2 r2
+    // 335 / 617, 546 / 1,642, 814 / 2,550; 48: 564 / 545, 1,189 / 1,507, 1,817 / 2,392;
+    // 160: 1,044 / 498, 2,716 / 1,413, 4,079 / 2,280.  3D, 24: 780 / 830, 1,672 / 1,999,
+    // 3,835 / 3,180; 96: 1,628 / 642, 4,104 / 1,874, 7,377 / 3,044.
+    if (bits && !bits_smem)
+        bits = dec_near_samples<DIM, BLOCK>([&](int i, int d) { return X[(int64_t)i * DIM + d]; }, total,
+                                            c0.r2) > DEC_SAMPLES * (DIM <= 2 ? 48 : 24);
     if (bits) {
-        __syncthreads();   // X is complete
         uint32_t* m = bits_smem ? reinterpret_cast<uint32_t*>(dec_smem + (dec_bits_fixed(total) + 15) / 16 * 16)
                                 : reinterpret_cast<uint32_t*>(v.dnb + (int64_t)v.dec_nb_pp * gd.s_scratch);
         decimate_bits<DIM, BLOCK>(X, total, c0.r2, gd.nocopy, alive, m, dec_smem, &v.err[gd.cloud_begin],
@@ -2647,16 +2656,20 @@ __device__ void decimate_group(const EngineView& v, const int g)
 }
 
 // ---------------------------------------------------------------------------
-// GPU-wide preparation of a large decimation (tiled runs: one group of
-// thousands of tiles).  When exactly one group is ready and it holds more
-// than DEC_BIG_MIN points, these kernels build its gathered points, hash
-// buckets, neighbour counts and neighbour lists across all SMs; k_decimate
-// then only runs the in-order scan.  dbig = {state, group, total}: state 1 =
+// GPU-wide preparation of a large decimation (tiled runs, whose one group may
+// hold thousands of tiles, and rd_decimate).  When exactly one group is ready and it
+// holds more than DEC_BIG_MIN points, these kernels build its gathered points, hash
+// buckets, neighbour counts and neighbour lists across all SMs, and k_dec_rounds
+// resolves its passes.  dbig = {state, group, total}: state 1 =
 // prepared, 2 = lists overflowed (k_decimate rebuilds on its own), 3 = prepared
 // and its rounds done (k_dec_rounds), 0 = idle.
 // ---------------------------------------------------------------------------
-constexpr int DEC_BIG_MIN = 4096;
+// About the largest set whose bit matrices one CTA keeps in shared memory (205-250
+// us for 790 points); from there on the kernels below take 200-350 us up to 4,097
+// points and 40 neighbours, one CTA 500-3,200.
+constexpr int DEC_BIG_MIN = 704;
 
+template <int DIM>
 __global__ void __launch_bounds__(1024) k_decbig_setup(EngineView v)
 {
     __shared__ int s_w[32];
@@ -2692,6 +2705,23 @@ __global__ void __launch_bounds__(1024) k_decbig_setup(EngineView v)
     }
     const int total = s_carry;
     if (total <= DEC_BIG_MIN) return;
+    // a quarter of the set around every point: lists as long as that take longer than
+    // the bit matrices of one CTA (all within 2 r2, 1,000 / 4,000 points: 965 / 3,649
+    // us, matrices 273 / 2,148; 40% of 790 in 3D 375 and 231; 4% of 4,096 349 and 2,280)
+    if (total <= DEC_BITS_MAX) {
+        auto coord = [&](int i, int d) {
+            int lo = 0, hi = gd.n_clouds - 1;   // last member with dcpre <= i
+            while (lo < hi) {
+                const int mid = (lo + hi + 1) >> 1;
+                if (v.dcpre[mid] <= i) lo = mid;
+                else hi = mid - 1;
+            }
+            const CloudDesc& cd = v.cl[gd.cloud_begin + lo];
+            return v.S[(cd.s_off + i - v.dcpre[lo]) * DIM + d];
+        };
+        if (dec_near_samples<DIM, 1024>(coord, total, v.cl[gd.cloud_begin].r2) > DEC_SAMPLES / 4 * total)
+            return;
+    }
     const int hbits = v.dec_hbits[g];
     int32_t* bstart = v.dbstart + v.dec_hoff[g];
     for (int h = tid; h <= (1 << hbits); h += 1024) bstart[h] = 0;
@@ -3050,7 +3080,7 @@ template <int DIM>
 cudaError_t launch_decbig(const EngineView& v, cudaStream_t st)
 {
     const int grid = v.n_sms * 8;
-    k_decbig_setup<<<1, 1024, 0, st>>>(v);
+    k_decbig_setup<DIM><<<1, 1024, 0, st>>>(v);
     k_decbig_gather<DIM><<<grid, 256, 0, st>>>(v);
     k_decbig_scan_buckets<<<1, 1024, 0, st>>>(v);
     k_decbig_fill<DIM><<<grid, 256, 0, st>>>(v);
@@ -3599,13 +3629,18 @@ int dec_dyn_bytes(int points)
     // the largest group's matrices where they fit; otherwise its counts, and room
     // for the matrices of groups of up to about 700 points
     const int b = std::min(points, DEC_BITS_MAX);
-    const int64_t all = (dec_bits_fixed(b) + 15) / 16 * 16 + dec_bits_matrix(b);
+    const int64_t all = dec_matrix_bytes(b);
     const int bits = all <= DEC_BITS_SMEM ? (int)all : std::max(dec_bits_fixed(b), 128 * 1024);
     return std::max(dec_list_bytes(points), bits);
 }
 
-cudaError_t launch_decimate(int dim, const EngineView& v, int64_t points, cudaStream_t st)
+cudaError_t launch_decimate(int dim, const EngineView& view, int64_t points, cudaStream_t st)
 {
+    EngineView v = view;
+    // the one group's size is known: its matrices fit shared memory, or (more than
+    // DEC_BITS_MAX points) it has none
+    const bool big = v.n_groups == 1 && v.dec_dyn < dec_matrix_bytes((int)std::min<int64_t>(points, DEC_BITS_MAX));
+    if (big && points > DEC_BITS_MAX) v.dec_dyn = dec_list_bytes(v.dec_smem_max);
     const int grid = std::max(1, std::min(v.n_groups, v.n_sms * 2));
     const int smem = dec_smem_bytes(v);
     cudaError_t e = cudaSuccess;
@@ -3614,7 +3649,7 @@ cudaError_t launch_decimate(int dim, const EngineView& v, int64_t points, cudaSt
         cudaError_t r = cudaFuncSetAttribute(k_decimate<DIM, 512>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         // one large group: its buckets, lists and rounds over more of the GPU
-        if (r == cudaSuccess && v.n_groups == 1 && points > DEC_BIG_MIN) r = launch_decbig<DIM>(v, st);
+        if (r == cudaSuccess && big) r = launch_decbig<DIM>(v, st);
         if (r == cudaSuccess) k_decimate<DIM, 512><<<grid, 512, smem, st>>>(v, 0, 0, 0);
         return r;
     });

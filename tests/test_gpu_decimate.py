@@ -47,3 +47,24 @@ def test_decimate_nan_inf_duplicates(torch):
     S[100:140] = S[100]
     for n in (300, 2000, 5000):
         assert bits_equal(_decimate(torch, S[:n], 0.03), O.decimate(S[:n], 0.03))
+
+
+# around the largest set of one CTA's shared memory, and where lists or matrices are taken by
+# how dense a sample of the set is
+@pytest.mark.parametrize("near", [3.0, 60.0, 1e6])
+@pytest.mark.parametrize("n,dim", [(705, 1), (864, 2), (865, 2), (865, 3), (900, 4), (2047, 1), (2048, 4)])
+def test_decimate_between_matrices_and_lists(torch, n, dim, near):
+    S = np.random.default_rng(n + dim).random((n, dim)).astype(np.float32)
+    ball = {1: 2.0, 2: np.pi, 3: 4.19, 4: 4.93}[dim]
+    r2 = float((near / n / ball) ** (1.0 / dim))
+    assert bits_equal(_decimate(torch, S, r2), O.decimate(S, r2))
+
+
+def test_solves_that_decimate_large_sets(torch):
+    """A solve's own decimations of 900 to 4,096 points, sparse and dense, against the oracle."""
+    import ridgedetection_b200 as rdb
+    r = np.random.default_rng(3)
+    for n, dim, r1, k in ((2500, 2, 0.004, 2.0), (4000, 3, 0.02, 2.0), (2500, 2, 0.004, 30.0), (3000, 1, 1e-5, 2.0)):
+        P = r.random((n, dim)).astype(np.float32)
+        S, st = rdb.ridge_detection(P, r1, k * r1)
+        assert st.err_bits == 0 and bits_equal(S, O.ridge_bf(P, r1, k * r1)[0])
