@@ -17,7 +17,7 @@
 // one warp then grows the chains with a word of the alive mask per lane.  The
 // serial chain of steps is what bounds either kernel; a step of the bit walk
 // is one shared-memory load, a ballot and a shuffle instead of three barriers
-// of 1,024 threads: 300 points in 3D 202 us -> 75 us.
+// of 1,024 threads: a call with 300 points in 3D 284 us -> 127 us, 1,000 points 811 -> 274.
 #include "rd_engine.cuh"
 
 #include <climits>
@@ -111,8 +111,10 @@ __global__ void __launch_bounds__(ORDER_BLOCK)
 }
 
 constexpr int ORDER_BITS_MAX = 1024;   // one alive word per lane
+// words of a bit row: odd, so that rows start in different banks
+__host__ __device__ constexpr int order_pitch(int ns) { return ((ns + 31) / 32) | 1; }
 
-// chains by one warp over the bit matrix adj[i * words + w] (words = ceil(ns/32)):
+// chains by one warp over the bit matrix adj[i * order_pitch(ns) + w]:
 // bit j of row i = points i and j within r2.  Every alive point is later than
 // the seed (earlier ones are in a chain already), so the first alive neighbour
 // of either end is the lowest set bit of (row(front) | row(back)) & alive.
@@ -123,9 +125,11 @@ __global__ void __launch_bounds__(ORDER_BLOCK)
 {
     extern __shared__ uint32_t adj[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int words = (ns + 31) / 32;
-    for (int64_t t = tid; t < (int64_t)ns * words; t += ORDER_BLOCK) {
-        const int i = (int)(t / words), w = (int)(t - (int64_t)i * words);
+    const int words = (ns + 31) / 32, pitch = order_pitch(ns);
+    // a warp shares the word, its points are broadcast reads (with lanes on words of one
+    // row every read touched 32 lines: 1,000 points 1,713 us, the serial search 811)
+    for (int t = tid; t < ns * words; t += ORDER_BLOCK) {
+        const int w = t / ns, i = t - w * ns;
         float f[DIM];
 #pragma unroll
         for (int d = 0; d < DIM; ++d) f[d] = S[i * DIM + d];
@@ -137,7 +141,7 @@ __global__ void __launch_bounds__(ORDER_BLOCK)
             for (int d = 0; d < DIM; ++d) q[d] = S[(w * 32 + b) * DIM + d];
             m |= (sqdist_exact<DIM>(q, f) <= rsq) ? (1u << b) : 0u;
         }
-        adj[t] = m;
+        adj[i * pitch + w] = m;
     }
     __syncthreads();
     if (warp != 0) return;
@@ -151,7 +155,7 @@ __global__ void __launch_bounds__(ORDER_BLOCK)
         const int sl = __ffs(left) - 1;
         const int p = sl * 32 + __ffs(__shfl_sync(0xffffffffu, alive, sl)) - 1;
         if (lane == sl) alive &= alive - 1;
-        uint32_t af = on ? adj[p * words + lane] : 0u, ab = af;
+        uint32_t af = on ? adj[p * pitch + lane] : 0u, ab = af;
         int head = ns, tail = ns;
         if (lane == 0) deq[ns] = p;
         for (;;) {
@@ -166,7 +170,7 @@ __global__ void __launch_bounds__(ORDER_BLOCK)
             const int hit = hl * 32 + (c & 31);
             const bool front = (c >> 5) & 1;
             if (lane == hl) alive &= ~(1u << (c & 31));
-            const uint32_t a = on ? adj[hit * words + lane] : 0u;
+            const uint32_t a = on ? adj[hit * pitch + lane] : 0u;
             if (front) { af = a; --head; }
             else { ab = a; ++tail; }
             if (lane == 0) deq[front ? head : tail] = hit;
@@ -191,13 +195,13 @@ cudaError_t launch_order_chains(int dim, const float* S, int ns, float rsq, unsi
                                 int32_t* n_chains, cudaStream_t st)
 {
     return with_dim(dim, [&](auto D) {
-        // up to 128 KB of shared memory for the bit matrix; larger ridges search
+        // up to 132 KB of shared memory for the bit matrix; larger ridges search
         // their candidates in every step
         if (ns <= ORDER_BITS_MAX) {
-            const int bytes = ns * ((ns + 31) / 32) * 4;
+            const int bytes = ns * order_pitch(ns) * 4;
             const cudaError_t e = cudaFuncSetAttribute(
                 k_order_bits<decltype(D)::value>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                ORDER_BITS_MAX * (ORDER_BITS_MAX / 32) * 4);
+                ORDER_BITS_MAX * order_pitch(ORDER_BITS_MAX) * 4);
             if (e != cudaSuccess) return e;
             k_order_bits<decltype(D)::value><<<1, ORDER_BLOCK, bytes, st>>>(S, ns, rsq, deq, order,
                                                                          chain_start, n_chains);
