@@ -359,6 +359,7 @@ EngineView Engine::view() const
     v.dmax = bDmax_.as<int32_t>();
     v.mv = bMv_.as<float>();
     v.cull = cull_ ? 1 : 0;
+    v.long_lists = n_slots_ > 0 && total_points_ / n_slots_ >= long_list_avg() ? 1 : 0;
     v.tile_order = bTileOrder_.as<int32_t>();
     v.n_heavy = n_heavy_;
     v.tile_clusters = tile_clusters_ ? 1 : 0;

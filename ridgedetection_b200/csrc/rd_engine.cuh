@@ -159,6 +159,7 @@ struct EngineView {
     float* mv;                   // 2*DIM+1 arrays of n_slots: each cloud's moves at its key_off
                                  // (old place, new place, length rounded up)
     int32_t cull;                // passes assign with k_assign_cull
+    int32_t long_lists;          // few chosen points: k_merge_fold's variant for long lists
     // fused tiled runs: tiles by decreasing evolve points, the first n_heavy
     // evolved by whole thread-block clusters (rd_tile_cluster.cuh)
     const int32_t* tile_order;
@@ -264,6 +265,8 @@ cudaError_t launch_spatial_prep(int dim, const EngineView& v, int items, int64_t
 // forward), again and again over the work lists of one launch_loopcond
 cudaError_t launch_evolve_step(int dim, const EngineView& v, const TuneParams& tp, int assign_grid,
                                cudaStream_t st);
+// points per chosen point from which a run takes the variant for long lists
+int long_list_avg();
 int assign_smem_bytes(int dim, const TuneParams& tp, int hist_ints);
 int max_assign_blocks_per_sm(int dim, const TuneParams& tp, int hist_ints);
 bool tune_supported(int dim, const TuneParams& tp);

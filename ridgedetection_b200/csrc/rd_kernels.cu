@@ -26,11 +26,25 @@ namespace rdb {
 
 namespace {
 
-// members from which a key is folded by its whole CTA (the warp-segmented exact
-// fold of rd_segfold.cuh) instead of by one warp's add chain -- while the pass
-// has no more keys to fold than CTAs; with more (a batch of large clouds) every
-// key is folded by a chain, which does less work in all.
-constexpr int SUM_BIG_MIN = 16384;
+// Long member lists.  The fold by a whole CTA (the warp-segmented exact fold of
+// rd_segfold.cuh) needs more than 128 registers a thread; the merge of k_merge_fold
+// wants four CTAs per SM, and with the 64 registers those leave the fold spills and
+// takes twice as long (lists of 500,000 members: 2,850 us, 1,350 with its registers).
+// And a CTA merges the edits of a list at about 4.5 ns a row, while a regrouping of
+// the cloud scatters over the whole GPU.  So runs of few chosen points (LONG_AVG points
+// for each) take a variant of k_merge_fold that has the registers, folds lists of
+// SUM_BIG_MIN members that way -- while the pass has no more keys to fold than CTAs;
+// with more every key is folded by a chain, which does less work in all -- and
+// regroups when such a list has an edit.  Others do so from larger lengths on, as the
+// slower fold and the cost of regrouping everybody ask for.  1M-point helix, evolve
+// from the chosen set, one variant for all / this, ms: r1 0.6 (35 chosen points) 18.8 /
+// 11.1, 0.4 (55) 17.9 / 12.4, 3 (2) 10.7 / 5.3.  What it does not reach: a list of most
+// of a cloud's points beside thousands of short ones (900,000 of 1M points beside
+// 4,714: one pass 3.9 ms, 1.9 if its fold had the registers).
+constexpr int LONG_AVG = 8192;
+constexpr int SUM_BIG_MIN = 16384, SUM_BIG_MIN_SLOW = 65536;
+// capacities of regions (list_cap) of 16,384 and 32,768 members
+constexpr int MERGE_CAP_LONG = 20480, MERGE_CAP = 40960;
 
 // Programmatic dependent launch: the loop-body kernels are launched with
 // programmatic stream serialisation, so a kernel's CTAs may become resident
@@ -766,6 +780,7 @@ __device__ __forceinline__ void push_edit(const EngineView& v, const int c, cons
     const int2 reg = *reinterpret_cast<const int2*>(v.kinfo + s);   // base, capacity
     if (at < min(EDIT_MAX, reg.y)) v.edit[cd.reg_off + reg.x + at] = edit;
     else v.reb[c] = 1;
+    if (reg.y > (v.long_lists ? MERGE_CAP_LONG : MERGE_CAP)) v.reb[c] = 1;
 }
 
 // resident CTAs the registers are held to: the evaluation waits on memory
@@ -1848,13 +1863,13 @@ __device__ __noinline__ float chain_tail(const uint32_t a, const int m, float su
 }
 
 // apart, so that its registers do not weigh on the merge
-template <int DIM, int W>
+template <int DIM, int W, bool LONG>
 __device__ __noinline__ void fold_long_list(const float* rows, const int n, SegFoldSmem<W, DIM>& sm)
 {
     fold_members_seg_src<W, DIM>(RowSrc<DIM>{rows}, n, sm);
 }
 
-template <int DIM, int BLOCK>
+template <int DIM, int BLOCK, bool LONG>
 __device__ void merge_fold_key(const EngineView& v, const int slot, const bool seg_ok,
                                MergeSmem<DIM, BLOCK>& sm)
 {
@@ -1899,8 +1914,8 @@ __device__ void merge_fold_key(const EngineView& v, const int slot, const bool s
     }
     __syncthreads();
     const int n_new = n_old + 2 * sm.ins[ne] - ne;
-    const bool seg = seg_ok && n_new >= SUM_BIG_MIN && n_new <= cap;
-    const int steps = seg && ne == 0 ? 0 : (max(n_old, 1) + MF_ROWS - 1) / MF_ROWS;
+    const bool seg = seg_ok && ne == 0 && n_old >= (LONG ? SUM_BIG_MIN : SUM_BIG_MIN_SLOW);
+    const int steps = seg ? 0 : (max(n_old, 1) + MF_ROWS - 1) / MF_ROWS;
     float sum = 0.0f;
     const int32_t* pos = v.cull ? v.Ls[par] + at : nullptr;
     // edits before chunk s's first row (those before the list's first row go to chunk 0)
@@ -1925,7 +1940,7 @@ __device__ void merge_fold_key(const EngineView& v, const int slot, const bool s
         if (warp == 0) {
             // the chain follows the merge one chunk behind
             for (int s = s0; s <= s1; ++s) {
-                if (s > s0 && !seg) {
+                if (s > s0) {
                     // whole groups; the rest waits for the next chunk
                     const int end = rows_before(s, s0), n = (end - r) / MF_CHAIN;
                     if (lane < DIM) {
@@ -2012,9 +2027,8 @@ __device__ void merge_fold_key(const EngineView& v, const int slot, const bool s
         __syncthreads();   // cut is looked up anew
     }
     if (seg) {
-        const float* rows = (ne > 0) ? v.Lr[par ^ 1] + at * DP : src;
         __syncthreads();  // the ring is read no more
-        fold_long_list<DIM, BLOCK / 32>(rows, n_new, sm.seg);
+        fold_long_list<DIM, BLOCK / 32, LONG>(src, n_old, sm.seg);
         if (warp == 0 && lane < DIM) sum = sm.seg.out[lane];
     }
     if (warp == 0) {
@@ -2035,16 +2049,16 @@ __device__ void merge_fold_key(const EngineView& v, const int slot, const bool s
 // same clouds): make ready for the next pass.
 enum : int { MF_CONTROL = 1, MF_STEP = 2 };
 
-template <int DIM, int BLOCK>
-__global__ void __launch_bounds__(BLOCK, BLOCK == MF_BLOCK ? 4 : 7) k_merge_fold(EngineView v, cudaGraphConditionalHandle h,
-                                                            int control, int use_handle)
+template <int DIM, int BLOCK, bool LONG>
+__global__ void __launch_bounds__(BLOCK, LONG ? 1 : BLOCK == MF_BLOCK ? 4 : 7)
+    k_merge_fold(EngineView v, cudaGraphConditionalHandle h, int control, int use_handle)
 {
     pdl_enter();
     __shared__ __align__(16) MergeSmem<DIM, BLOCK> sm;
     __shared__ int s_last;
     const int nd = v.ctr[CTR_NDIRTY];
     for (int t = blockIdx.x; t < nd; t += gridDim.x)
-        merge_fold_key<DIM, BLOCK>(v, v.dlist[t], nd <= (int)gridDim.x, sm);
+        merge_fold_key<DIM, BLOCK, LONG>(v, v.dlist[t], nd <= (int)gridDim.x, sm);
     // every thread's writes (chosen points, moved flags) before the count
     __threadfence();
     __syncthreads();
@@ -3286,13 +3300,13 @@ cudaError_t launch_assign_cull(const EngineView& v, int pdl, cudaStream_t st)
 }
 
 // grid of k_merge_fold: every resident CTA, at most one per chosen point
-template <int DIM, int BLOCK>
+template <int DIM, int BLOCK, bool LONG>
 int merge_grid(const EngineView& v)
 {
     static std::atomic<int> per_sm{0};
     int b = per_sm.load(std::memory_order_relaxed);
     if (b == 0) {
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_merge_fold<DIM, BLOCK>, BLOCK, 0) !=
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_merge_fold<DIM, BLOCK, LONG>, BLOCK, 0) !=
                 cudaSuccess || b < 1)
             b = 1;
         per_sm.store(b, std::memory_order_relaxed);
@@ -3363,12 +3377,17 @@ cudaError_t launch_evolve_kernels(const EngineView& v, const TuneParams& tp, int
                        scatter_cta_smem_bytes(v), st, v);
     if (e != cudaSuccess) return e;
     if (v.n_slots > 0) {
-        if (v.n_clouds == 1)
-            e = launch_pdl(pdl, k_merge_fold<DIM, MF_BLOCK>, merge_grid<DIM, MF_BLOCK>(v), MF_BLOCK, 0,
-                           st, v, lc.h, control, lc.use_handle);
-        else
-            e = launch_pdl(pdl, k_merge_fold<DIM, MF_BLOCK_MANY>, merge_grid<DIM, MF_BLOCK_MANY>(v),
-                           MF_BLOCK_MANY, 0, st, v, lc.h, control, lc.use_handle);
+        auto merge = [&](auto block, auto lng) {
+            constexpr int B = decltype(block)::value;
+            constexpr bool LONG = decltype(lng)::value;
+            return launch_pdl(pdl, k_merge_fold<DIM, B, LONG>, merge_grid<DIM, B, LONG>(v), B, 0, st, v,
+                              lc.h, control, lc.use_handle);
+        };
+        using Many = std::integral_constant<int, MF_BLOCK_MANY>;
+        using One = std::integral_constant<int, MF_BLOCK>;
+        if (v.long_lists) e = merge(One{}, std::true_type{});
+        else if (v.n_clouds == 1) e = merge(One{}, std::false_type{});
+        else e = merge(Many{}, std::false_type{});
     } else {
         e = launch_pdl(pdl, k_control, std::min((v.n_clouds + 255) / 256, sms), 256, 0, st, v);
     }
@@ -3680,6 +3699,8 @@ bool tune_supported(int dim, const TuneParams& tp)
     return cull_ok && ((tp.block == 128 && (tp.items == 4 || tp.items == 8 || tp.items == 16)) ||
                        (tp.block == 256 && (tp.items == 4 || tp.items == 8)));
 }
+
+int long_list_avg() { return LONG_AVG; }
 
 int assign_smem_bytes(int dim, const TuneParams& tp, int hist_ints)
 {

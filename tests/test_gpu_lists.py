@@ -70,3 +70,45 @@ def test_lists_in_a_batch(rdb):
             S, _ = rdb.ridge_detection(P, r1, r2)
             assert bits_equal(b.chosen_points(c), S), c
     b.close()
+
+
+def _beside(n, k, dim, sigma, seed):
+    """k points of a blob away from zero, the rest far apart around it."""
+    r = np.random.default_rng(seed)
+    P = np.concatenate([r.normal(10.0, sigma, (k, dim)), r.uniform(0.0, 20.0, (n - k, dim))])
+    return P[r.permutation(n)].astype(np.float32)
+
+
+@pytest.mark.parametrize("name,gen,r1", [
+    # few chosen points: lists of 16,384 and more are folded in segments and regrouped when edited
+    ("few_keys", lambda: G.helix3d(200_000, seed=8), 1.5),
+    ("few_keys_2d", lambda: G.sine2d(150_000, seed=9), 1.0),
+    ("few_keys_1d", lambda: _blob(100_000, 1, 1.0, 10), 1.0),
+    ("few_keys_4d", lambda: _blob(60_000, 4, 0.3, 11), 1.0),
+    # many chosen points beside lists around 32,768 and 65,536 members
+    ("beside_40k", lambda: _beside(42_000, 40_000, 3, 0.1, 12), 0.5),
+    ("beside_70k", lambda: _beside(73_000, 70_000, 2, 0.1, 13), 0.5),
+])
+def test_long_lists_match_oracle(rdb, name, gen, r1):
+    import oracle as O
+    P = gen()
+    S_ref = O.ridge_bf(P, r1, 2.0 * r1)[0]
+    for cull in (True, False):
+        rdb.set_assign_cull(cull)
+        try:
+            S, st = rdb.ridge_detection(P, r1, 2.0 * r1)
+        finally:
+            rdb.set_assign_cull(True)
+        assert st.err_bits == 0 and bits_equal(S, S_ref)
+
+
+def test_long_lists_in_a_batch(rdb):
+    clouds = [(G.helix3d(60_000, seed=14), 1.5, 3.0), (_blob(40_000, 3, 0.2, 15), 0.9, 1.8),
+              (G.helix3d(90_000, seed=16), 2.0, 4.0)]
+    packed, descs = rdb.pack_clouds(clouds)
+    b = rdb.BatchedRidgeDetection()
+    b.run(packed, descs)
+    for c, (P, r1, r2) in enumerate(clouds):
+        S, _ = rdb.ridge_detection(P, r1, r2)
+        assert bits_equal(b.chosen_points(c), S), c
+    b.close()
