@@ -406,7 +406,7 @@ int Engine::finish_setup_after_choose(cudaStream_t st, bool ns_given)
         // rows of the grouped lists: every key's region (list_cap in rd_kernels.cu)
         cd.reg_off = culls ? rows : cd.p_off;
         rows += (int64_t)cd.n_all + cd.n_all / 4 + 8 * (int64_t)cd.ns_cap;
-        (cd.n_chunks > SCAN_ROWS_WARP ? kblk : kblk_warp) += (cd.ns_cap + KBLK - 1) / KBLK;
+        (scan_by_cta(cd.n_chunks, cd.ns_cap) ? kblk : kblk_warp) += (cd.ns_cap + KBLK - 1) / KBLK;
         for (int k = 0; k < cd.ns_cap; ++k) h_slot_cloud_.push_back((int32_t)c);
     }
     n_slots_ = (int32_t)key;

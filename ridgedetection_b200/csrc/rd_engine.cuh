@@ -41,12 +41,19 @@ constexpr int DEC_SMEM_MAX_POINTS = 32752;
 // fused per-tile evolve: chosen points per tile it can hold
 constexpr int TILE_NS_MAX = 1024;
 
-// kinds of work list over the evolving clouds (rebuilt by the control step
-// after every iteration): assignment chunks; blocks of KBLK chosen points of
-// clouds with more than SCAN_ROWS_WARP chunks (CTA-wide histogram scan) and of
-// the other clouds (one warp per block); chosen slots
+// kinds of work list over the evolving clouds (rebuilt by loop_condition when a cloud
+// converges): assignment chunks; blocks of KBLK chosen points of the clouds scanned by
+// CTAs (scan_by_cta) and of the others (one warp per block); chosen slots
 enum : int { ACT_CHUNK = 0, ACT_KBLK = 1, ACT_KBLK_WARP = 2, ACT_SLOT = 3, ACT_KINDS = 4 };
-constexpr int SCAN_ROWS_WARP = 64;
+// Clouds whose histogram a CTA scans per block of chosen points: those of many chunk
+// rows, and those of many chosen points, where the last block lays out every key's
+// region, 32 keys after 32 in one warp (one pass over 30,000 points with 29,849 chosen
+// ones 3.6 ms, by CTAs 2.8).
+constexpr int SCAN_ROWS_WARP = 64, SCAN_KEYS_WARP = 2048;
+__host__ __device__ inline bool scan_by_cta(const int n_chunks, const int ns_cap)
+{
+    return n_chunks > SCAN_ROWS_WARP || ns_cap > SCAN_KEYS_WARP;
+}
 
 enum : int {
     CTR_WORK = 0,      // assignment work ticket
@@ -130,7 +137,7 @@ struct EngineView {
     int32_t n_groups;
     int32_t n_chunks;
     int32_t n_slots;
-    int32_t n_kblk;              // blocks of KBLK chosen slots, clouds of > SCAN_ROWS_WARP chunks
+    int32_t n_kblk;              // blocks of KBLK chosen slots, clouds scanned by CTAs
     int32_t n_kblk_warp;         // the same over the other clouds
     int32_t chunk_pts;           // max points per assignment chunk (BLOCK*ITEMS)
     int32_t chunk_max;           // largest chunk actually used (scatter staging)

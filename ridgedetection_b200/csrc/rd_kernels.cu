@@ -1006,8 +1006,8 @@ __global__ void __launch_bounds__(AC_BLOCK, ITEMS <= 4 ? 4 : 2) k_assign_cull(En
 // chosen point k, the exclusive prefix over the cloud's chunks of the chunk x
 // key histogram (hpre row lc: members in earlier chunks) and the member count
 // cnt[k].  Work item = block of KBLK keys, one key per lane.
-//   k_chunkscan_cta   clouds with more than SCAN_ROWS_WARP chunk rows: one CTA
-//                     per item; the CS_W warps take contiguous row ranges, sum
+//   k_chunkscan_cta   clouds with many chunk rows or chosen points (scan_by_cta):
+//                     one CTA per item; the CS_W warps take contiguous row ranges, sum
 //                     them, exchange the warp totals, and rescan their rows
 //                     writing the prefixes;
 //   k_chunkscan_warp  the other clouds: one warp per item, a single pass.
@@ -3168,8 +3168,9 @@ __device__ void loop_condition(const EngineView& v, cudaGraphConditionalHandle h
         const int rows = ev ? v.cl[c].n_chunks : 0;
         const int nkb = ev ? (v.ns[c] + KBLK - 1) / KBLK : 0;
         x[1 + ACT_CHUNK] = rows;
-        x[1 + ACT_KBLK] = rows > SCAN_ROWS_WARP ? nkb : 0;
-        x[1 + ACT_KBLK_WARP] = rows > SCAN_ROWS_WARP ? 0 : nkb;
+        const bool by_cta = ev && scan_by_cta(rows, v.cl[c].ns_cap);
+        x[1 + ACT_KBLK] = by_cta ? nkb : 0;
+        x[1 + ACT_KBLK_WARP] = by_cta ? 0 : nkb;
         x[1 + ACT_SLOT] = ev ? v.ns[c] : 0;
         int incl[ACT_KINDS + 1];
 #pragma unroll

@@ -112,3 +112,21 @@ def test_long_lists_in_a_batch(rdb):
         S, _ = rdb.ridge_detection(P, r1, r2)
         assert bits_equal(b.chosen_points(c), S), c
     b.close()
+
+
+@pytest.mark.parametrize("n", [2000, 2049, 2600, 9000])
+def test_nearly_all_chosen(rdb, n):
+    """Chosen sets around the size from which CTAs scan a cloud of few chunks, alone and beside
+    clouds that warps scan."""
+    import oracle as O
+    P = np.random.default_rng(n).random((n, 3)).astype(np.float32)
+    r1 = 0.15 / n
+    S, st = rdb.ridge_detection(P, r1, 0.02)
+    assert st.err_bits == 0 and bits_equal(S, O.ridge_bf(P, r1, 0.02)[0])
+    clouds = [(P, r1, 0.02), (G.helix3d(700, seed=1), 0.2, 0.4), (G.helix3d(90_000, seed=2), 0.2, 0.4)]
+    packed, descs = rdb.pack_clouds(clouds)
+    b = rdb.BatchedRidgeDetection()
+    b.run(packed, descs)
+    for c, (Q, q1, q2) in enumerate(clouds):
+        assert bits_equal(b.chosen_points(c), rdb.ridge_detection(Q, q1, q2)[0]), c
+    b.close()
