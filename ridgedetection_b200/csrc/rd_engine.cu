@@ -403,9 +403,9 @@ int Engine::finish_setup_after_choose(cudaStream_t st, bool ns_given)
         hist += (int64_t)cd.n_chunks * cd.ns_cap;
         cd.key_off = key;
         key += cd.ns_cap;
-        // rows of the grouped lists: every key's region (list_cap in rd_kernels.cu)
+        // rows of the grouped lists: every key's region
         cd.reg_off = culls ? rows : cd.p_off;
-        rows += (int64_t)cd.n_all + cd.n_all / 4 + 8 * (int64_t)cd.ns_cap;
+        rows += list_rows(cd.n_all, cd.ns_cap);
         (scan_by_cta(cd.n_chunks, cd.ns_cap) ? kblk : kblk_warp) += (cd.ns_cap + KBLK - 1) / KBLK;
         for (int k = 0; k < cd.ns_cap; ++k) h_slot_cloud_.push_back((int32_t)c);
     }
@@ -678,7 +678,7 @@ int Engine::ensure_cull_buffers()
     RD_CK(bSlack_.ensure(sizeof(float) * (blocks + 1)));
     RD_CK(bLslack_.ensure(sizeof(float) * (blocks + 1)));
     RD_CK(bBlen_.ensure(sizeof(int32_t) * (blocks + 1)));
-    RD_CK(bBlist_.ensure(sizeof(int32_t) * (128 * blocks + 1)));   // LIST_MAX in rd_kernels.cu
+    RD_CK(bBlist_.ensure(sizeof(int32_t) * (CAND_MAX * blocks + 1)));
     for (int b = 0; b < 2; ++b) {
         RD_CK(bLr_[b].ensure(sizeof(float) * ((size_t)list_rows_ * pad_dim(dim_) + 4)));
         RD_CK(bLs_[b].ensure(sizeof(int32_t) * ((size_t)list_rows_ + 1)));

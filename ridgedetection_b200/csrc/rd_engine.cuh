@@ -14,6 +14,7 @@
 #pragma once
 
 #include "rd_internal.cuh"
+#include "rd_listroom.hpp"
 #include "rd_tile_rule.hpp"
 
 #include <cstddef>
@@ -159,7 +160,7 @@ struct EngineView {
     float* bslack;               // per block: moves that leave its keys as they are (see k_assign_cull)
     float* lslack;               // per block: moves that leave its candidate list complete
     int32_t* blen;               // per block: entries of its candidate list
-    int32_t* blist;              // per block: the list (LIST_MAX entries)
+    int32_t* blist;              // per block: the list (CAND_MAX entries)
     int32_t* full;               // per cloud: the next pass evaluates every block and every key
     int32_t* mvn;                // per cloud: chosen points moved in the last pass
     int32_t* dmax;               // per cloud: bits of the longest of those moves

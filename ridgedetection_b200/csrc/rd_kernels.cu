@@ -43,8 +43,8 @@ namespace {
 // 4,714: one pass 3.9 ms, 1.9 if its fold had the registers).
 constexpr int LONG_AVG = 8192;
 constexpr int SUM_BIG_MIN = 16384, SUM_BIG_MIN_SLOW = 65536;
-// capacities of regions (list_cap) of 16,384 and 32,768 members
-constexpr int MERGE_CAP_LONG = 20480, MERGE_CAP = 40960;
+// regions of 16,384 and 32,768 members
+constexpr int MERGE_CAP_LONG = list_room(16384), MERGE_CAP = list_room(32768);
 
 // Programmatic dependent launch: the loop-body kernels are launched with
 // programmatic stream serialisation, so a kernel's CTAs may become resident
@@ -687,7 +687,7 @@ __global__ void __launch_bounds__(BLOCK) k_assign(EngineView v)
 // of the whole chosen set found them, while the moves D since then -- taken
 // over the chosen points within R of the box, which covers those within r1 --
 // add up to less than r1/4: any other chosen point is then still more than
-// r1 (1 + 4.8e-4) away.  An evaluation reads that list, at most LIST_MAX
+// r1 (1 + 4.8e-4) away.  An evaluation reads that list, at most CAND_MAX
 // entries, instead of every chosen point; a block with more candidates keeps
 // none and scans.
 //
@@ -745,10 +745,6 @@ __device__ __forceinline__ void assign_one(const float* sk, const int k, const f
     }
 }
 
-// candidates of a block: the 1M helix has 17 blocks (of 7,812) with more than 32
-// (up to 119), over jumps of the spatial order that two boxes do not cover, and
-// scanning 790 chosen points for each of them outlasted the rest of the pass
-constexpr int LIST_MAX = 128;
 // moves of a single cloud staged in shared memory
 constexpr int AC_MOVES = 512;
 constexpr int EDIT_IN = (int)0x80000000;   // edit of a member list: this point joins (else it leaves)
@@ -759,7 +755,7 @@ constexpr int EDIT_MAX = 512;              // edits of one key that k_merge_fold
 // assignment every pass rebuilds)
 __device__ __forceinline__ int list_cap(const EngineView& v, const int n)
 {
-    return v.cull ? n + (n >> 2) + 8 : n;
+    return v.cull ? list_room(n) : n;
 }
 
 // A pass regroups all points of a cloud by key: its chosen points are new or
@@ -780,7 +776,7 @@ __device__ __forceinline__ void push_edit(const EngineView& v, const int c, cons
     const int2 reg = *reinterpret_cast<const int2*>(v.kinfo + s);   // base, capacity
     if (at < min(EDIT_MAX, reg.y)) v.edit[cd.reg_off + reg.x + at] = edit;
     else v.reb[c] = 1;
-    if (reg.y > (v.long_lists ? MERGE_CAP_LONG : MERGE_CAP)) v.reb[c] = 1;
+    if (reg.y >= (v.long_lists ? MERGE_CAP_LONG : MERGE_CAP)) v.reb[c] = 1;
 }
 
 // resident CTAs the registers are held to: the evaluation waits on memory
@@ -890,7 +886,7 @@ __global__ void __launch_bounds__(AC_BLOCK, ITEMS <= 4 ? 4 : 2) k_assign_cull(En
             }
             const float list_left = full ? 0.0f : __fsub_rd(v.lslack[wb], dl);
             const int n_list = (list_left > 0.0f) ? v.blen[wb] : -1;
-            int32_t* list = v.blist + wb * LIST_MAX;
+            int32_t* list = v.blist + wb * CAND_MAX;
             float2 np2[ITEMS / 2][DIM];
             int old[ITEMS];
 #pragma unroll
@@ -957,13 +953,13 @@ __global__ void __launch_bounds__(AC_BLOCK, ITEMS <= 4 ? 4 : 2) k_assign_cull(En
                     const unsigned nb = __ballot_sync(FULL, near);
                     if (!nb) continue;
                     const int at = len + __popc(nb & lanemask_lt());
-                    if (near && at < LIST_MAX) list[at] = q;
+                    if (near && at < CAND_MAX) list[at] = q;
                     len += __popc(nb);
                     take(__ballot_sync(FULL, q < ns && !(may_skip && g2 > thr)), s, q);
                 }
                 if (lane == 0) {
                     v.blen[wb] = len;
-                    v.lslack[wb] = (may_skip && len <= LIST_MAX) ? 0.25f * cd.r1 : 0.0f;
+                    v.lslack[wb] = (may_skip && len <= CAND_MAX) ? 0.25f * cd.r1 : 0.0f;
                 }
             }
             const float r1 = cd.r1;
