@@ -249,7 +249,6 @@ int Engine::setup(int dim, const std::vector<CloudDesc>& clouds,
     RD_CK(bS_.ensure(sizeof(float) * (size_t)(s_off * dim + 4)));
     RD_CK(bNext_.ensure(sizeof(int32_t) * (size_t)(s_off + 1)));
     RD_CK(bKeys_.ensure(sizeof(int32_t) * (size_t)(total_points + 1)));
-    RD_CK(bGrouped_.ensure(sizeof(int32_t) * (size_t)(total_points + 4)));
     RD_CK(bRes_.ensure(res_bytes(nc)));
     RD_CK(bPhase_.ensure(4 * (nc + 1)));
     RD_CK(bCont_.ensure(4 * (nc + 1)));
@@ -281,7 +280,6 @@ EngineView Engine::view() const
     v.P = bP_.as<float>();
     v.S = bS_.as<float>();
     v.keys = bKeys_.as<int32_t>();
-    v.perm = bGrouped_.as<int32_t>();
     v.Pg = bPg_.as<float>();
     v.hist = bHist_.as<int32_t>();
     v.hpre = bHpre_.as<int32_t>();

@@ -44,8 +44,8 @@ constexpr int TILE_NS_MAX = 1024;
 
 // kinds of work list over the evolving clouds (rebuilt by loop_condition when a cloud
 // converges): assignment chunks; blocks of KBLK chosen points of the clouds scanned by
-// CTAs (scan_by_cta) and of the others (one warp per block); chosen slots
-enum : int { ACT_CHUNK = 0, ACT_KBLK = 1, ACT_KBLK_WARP = 2, ACT_SLOT = 3, ACT_KINDS = 4 };
+// CTAs (scan_by_cta) and of the others (one warp per block)
+enum : int { ACT_CHUNK = 0, ACT_KBLK = 1, ACT_KBLK_WARP = 2, ACT_KINDS = 3 };
 // Clouds whose histogram a CTA scans per block of chosen points: those of many chunk
 // rows, and those of many chosen points, where the last block lays out every key's
 // region, 32 keys after 32 in one warp (one pass over 30,000 points with 29,849 chosen
@@ -82,8 +82,6 @@ struct EngineView {
     float* P;                    // packed evolve points, ROW_MAJOR
     float* S;                    // chosen points, ROW_MAJOR, capacity n_own per cloud
     int32_t* keys;               // per point slot: assigned chosen index or -1
-    int32_t* perm;               // per point slot: point indices grouped by key, index order
-                                 // (tiled kernels)
     float* Pg;                   // per point slot: the points' coordinates grouped by key in
                                  // index order, PadDim floats each (tiled kernels)
     // lockstep passes: each key's members in index order, in its region

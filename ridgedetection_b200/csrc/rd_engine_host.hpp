@@ -181,7 +181,7 @@ private:
     RunStats stats_;
 
     DevBuf bCl_, bGr_, bChunkCloud_, bSlotCloud_;
-    DevBuf bP_, bS_, bKeys_, bGrouped_, bPg_, bHist_, bCnt_, bBase_, bNext_, bHash_, bSurv_;
+    DevBuf bP_, bS_, bKeys_, bPg_, bHist_, bCnt_, bBase_, bNext_, bHash_, bSurv_;
     DevBuf bRes_, bPhase_, bCont_, bPasses_, bOuter_, bKbDone_;
     std::vector<uint64_t> h_res_;
     DevBuf bActCloud_, bActPre_, bGroupConv_, bReady_, bDnbOff_, bDnb_, bDbig_, bDcpre_;

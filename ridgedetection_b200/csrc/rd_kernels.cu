@@ -3154,7 +3154,7 @@ __device__ void loop_condition(const EngineView& v, cudaGraphConditionalHandle h
     for (int c = tid; c < v.n_clouds; c += blockDim.x) act += (v.phase[c] != PH_DONE);
     if (act) atomicAdd(&s_act, act);
     // work lists of the next iteration: evolving clouds, prefixes of their
-    // chunks, chosen-point blocks and chosen slots
+    // chunks and chosen-point blocks
     const int nc = v.n_clouds;
     for (int c0 = 0; c0 < nc; c0 += blockDim.x) {
         const int c = c0 + tid;
@@ -3167,7 +3167,6 @@ __device__ void loop_condition(const EngineView& v, cudaGraphConditionalHandle h
         const bool by_cta = ev && scan_by_cta(rows, v.cl[c].ns_cap);
         x[1 + ACT_KBLK] = by_cta ? nkb : 0;
         x[1 + ACT_KBLK_WARP] = by_cta ? 0 : nkb;
-        x[1 + ACT_SLOT] = ev ? v.ns[c] : 0;
         int incl[ACT_KINDS + 1];
 #pragma unroll
         for (int q = 0; q <= ACT_KINDS; ++q) {
