@@ -62,12 +62,13 @@ def evolve_adjoint_device(P, S0, r1: float, iters: int, W, checkpoint_every: int
 def evolve_means_device(P, S0, r1: float, iters: int):
     """The forward of :func:`evolve_adjoint_device` alone: S_final."""
     import torch
+    n, dim = P.shape
     P, S0 = P.contiguous(), S0.contiguous()
     Sf = torch.empty_like(S0)
     vp = ctypes.c_void_p
     st = vp(torch.cuda.current_stream(P.device).cuda_stream)
-    L.check(L.lib().rd_evolve_means(int(P.shape[1]), vp(P.data_ptr()), int(P.shape[0]),
-                                    vp(S0.data_ptr()), int(S0.shape[0]), float(r1), int(iters),
+    L.check(L.lib().rd_evolve_means(dim, vp(P.data_ptr()), n, vp(S0.data_ptr()),
+                                    int(S0.shape[0]), float(r1), int(iters),
                                     vp(Sf.data_ptr()), st))
     return Sf
 
@@ -80,6 +81,10 @@ def _autograd_function():
 
         @staticmethod
         def forward(ctx, P, chosen_idx, r1, iters, checkpoint_every=0):
+            # the forward has no use for it, but a bad value is refused here and not
+            # only when the backward runs
+            if int(checkpoint_every) < 0:
+                raise L.RDError(L.RD_ERR_ARG, "bad iteration counts")
             S0 = P.detach()[chosen_idx].contiguous()
             Sf = evolve_means_device(P.detach(), S0, r1, iters)
             ctx.save_for_backward(P.detach(), chosen_idx)
