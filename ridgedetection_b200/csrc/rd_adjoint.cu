@@ -17,7 +17,9 @@
 // The reverse of a segment is two kernels: g before every pass of it, one
 // thread per chosen coordinate (a pass with members resets it), then one thread
 // per point that adds its terms in the order of the passes, so that dL/dP is
-// read and written once per segment instead of once per pass.  262,144 points,
+// read and written once per segment instead of once per pass.  g before every pass
+// is ns x dim doubles a pass, more than the kept assignments where nearly every
+// point is chosen: passes are taken in blocks of at most ADJ_G_BYTES of it.  262,144 points,
 // 20 passes in segments of 5: 40 kernel pairs and 256 us before, 4 and 64 us now.
 #include "rd_adjoint.hpp"
 
@@ -67,6 +69,8 @@ __global__ void __launch_bounds__(256) k_adj_members(const int32_t* __restrict__
     }
 }
 
+constexpr int64_t ADJ_G_BYTES = int64_t(64) << 20;
+
 int grid_for(int64_t n) { return (int)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, 148 * 16)); }
 
 }  // namespace
@@ -109,11 +113,13 @@ int AdjointRunner::run(int dim, const float* d_P, int64_t np, const float* d_S0,
     float* S = eng_.chosen_mut();
     const size_t sbytes = sizeof(float) * ns * dim;
     const int64_t nk = ns * dim;
+    // passes reversed by one pair of kernels
+    const int block = (int)std::max<int64_t>(1, std::min<int64_t>(seg, ADJ_G_BYTES / (8 * nk)));
     if (reverse) {
         AK(bKeys_.ensure(sizeof(int32_t) * (size_t)np * seg + 16));
         AK(bCnt_.ensure(sizeof(int32_t) * (size_t)ns * seg + 16));
         AK(bCkpt_.ensure(sizeof(float) * (size_t)nk * (nseg + 1) + 16));
-        AK(bG_.ensure(sizeof(double) * (size_t)nk * (seg + 1) + 16));
+        AK(bG_.ensure(sizeof(double) * (size_t)nk * (block + 1) + 16));
     }
     double* g = bG_.as<double>();
     double* G = g + nk;
@@ -151,13 +157,17 @@ int AdjointRunner::run(int dim, const float* d_P, int64_t np, const float* d_S0,
                 if (int rc = keep(q)) return rc;
             }
         }
-        k_adj_carry<<<(int)((nk + 255) / 256), 256, 0, st>>>(bCnt_.as<int32_t>(), ns, dim, len, g, G);
-        AK(with_dim(dim, [&](auto D) {
-            constexpr int DIM = decltype(D)::value;
-            k_adj_members<DIM><<<grid_for(np), 256, 0, st>>>(bKeys_.as<int32_t>(), bCnt_.as<int32_t>(),
-                                                            G, np, ns, len, d_gP);
-            return cudaGetLastError();
-        }));
+        for (int q1 = len; q1 > 0; q1 -= block) {
+            const int q0 = std::max(0, q1 - block);
+            const int32_t* kt = bKeys_.as<int32_t>() + (size_t)q0 * np;
+            const int32_t* ct = bCnt_.as<int32_t>() + (size_t)q0 * ns;
+            k_adj_carry<<<(int)((nk + 255) / 256), 256, 0, st>>>(ct, ns, dim, q1 - q0, g, G);
+            AK(with_dim(dim, [&](auto D) {
+                constexpr int DIM = decltype(D)::value;
+                k_adj_members<DIM><<<grid_for(np), 256, 0, st>>>(kt, ct, G, np, ns, q1 - q0, d_gP);
+                return cudaGetLastError();
+            }));
+        }
     }
     if (d_gS0) AK(cudaMemcpyAsync(d_gS0, bG_.p, sizeof(double) * ns * dim, cudaMemcpyDeviceToDevice, st));
     AK(cudaStreamSynchronize(st));

@@ -176,3 +176,28 @@ def test_segments_agree(iters, every):
     for x, y in zip(a, b):
         assert torch.equal(x, y)
     assert torch.equal(adj.evolve_means_device(P, S0, 0.2, iters), a[0])
+
+
+def test_reverse_in_blocks_of_passes(adj):
+    """So many chosen points that the gradients before 60 passes are more than one block of
+    them: the same bits as with segments of seven passes, each one block."""
+    torch = require_cuda()
+    import ctypes
+
+    from ridgedetection_b200 import _lib as L
+    P = torch.from_numpy(G.helix3d(60_000, seed=77)).cuda()
+    r1, iters = 0.004, 60
+    S = torch.zeros_like(P)
+    ns = ctypes.c_int64(0)
+    L.check(L.lib().rd_choose(3, ctypes.c_void_p(P.data_ptr()), P.shape[0], r1,
+                              ctypes.c_void_p(S.data_ptr()), ctypes.byref(ns),
+                              ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))
+    assert ns.value * 3 * 8 * iters > 64 << 20
+    S0 = S[:ns.value].contiguous()
+    W = torch.randn(S0.shape, dtype=torch.float64, device="cuda",
+                    generator=torch.Generator("cuda").manual_seed(1))
+    whole = adj.evolve_adjoint_device(P, S0, r1, iters, W, 0)
+    parts = adj.evolve_adjoint_device(P, S0, r1, iters, W, 7)
+    for x, y in zip(whole, parts):
+        assert bits_equal(x.cpu().numpy(), y.cpu().numpy())
+    assert float(whole[1].abs().sum()) > 0
