@@ -243,8 +243,6 @@ int Engine::setup(int dim, const std::vector<CloudDesc>& clouds,
         next_off += cd.n_all;
     }
     spatial_ok_ = spatial_ok_ && next_off == total_points;
-    // list positions and edits are 31-bit, with a quarter more rows than points
-    cull_allowed_ = total_points <= (int64_t(1) << 30);
     RD_CK(bP_.ensure(sizeof(float) * (size_t)(total_points * dim + 4)));
     RD_CK(bS_.ensure(sizeof(float) * (size_t)(s_off * dim + 4)));
     RD_CK(bNext_.ensure(sizeof(int32_t) * (size_t)(s_off + 1)));
@@ -282,13 +280,13 @@ EngineView Engine::view() const
     v.keys = bKeys_.as<int32_t>();
     v.Pg = bPg_.as<float>();
     v.hist = bHist_.as<int32_t>();
-    v.hpre = bHpre_.as<int32_t>();
+    v.hpre = lists_ ? bHpre_.as<int32_t>() : bHist_.as<int32_t>();
     v.cnt = bCnt_.as<int32_t>();
     v.base = bBase_.as<int32_t>();
     for (int b = 0; b < 2; ++b) {
-        // without the culled assignment the lists are regrouped in every pass
-        v.Lr[b] = cull_ ? bLr_[b].as<float>() : bPg_.as<float>();
-        v.Ls[b] = cull_ ? bLs_[b].as<int32_t>() : nullptr;
+        // otherwise the points are regrouped in every pass
+        v.Lr[b] = lists_ ? bLr_[b].as<float>() : bPg_.as<float>();
+        v.Ls[b] = lists_ ? bLs_[b].as<int32_t>() : nullptr;
     }
     v.kinfo = bKinfo_.as<int4>();
     v.edit = bEdit_.as<int32_t>();
@@ -357,6 +355,8 @@ EngineView Engine::view() const
     v.dmax = bDmax_.as<int32_t>();
     v.mv = bMv_.as<float>();
     v.cull = cull_ ? 1 : 0;
+    v.lists = lists_ ? 1 : 0;
+    v.hist_ints = hist_ints_;
     v.long_lists = n_slots_ > 0 && total_points_ / n_slots_ >= long_list_avg() ? 1 : 0;
     v.tile_order = bTileOrder_.as<int32_t>();
     v.n_heavy = n_heavy_;
@@ -389,8 +389,7 @@ int Engine::finish_setup_after_choose(cudaStream_t st, bool ns_given)
         RD_CK(cudaMemcpyAsync(h_ns_.data(), view().ns, 4 * nc, cudaMemcpyDeviceToHost, st));
         RD_CK(cudaStreamSynchronize(st));
     }
-    int64_t hist = 0, key = 0, kblk = 0, kblk_warp = 0, rows = 0;
-    const bool culls = cull_possible();
+    int64_t hist = 0, key = 0, kblk = 0, kblk_warp = 0;
     int max_ns = 0;
     h_slot_cloud_.clear();
     for (size_t c = 0; c < nc; ++c) {
@@ -401,15 +400,12 @@ int Engine::finish_setup_after_choose(cudaStream_t st, bool ns_given)
         hist += (int64_t)cd.n_chunks * cd.ns_cap;
         cd.key_off = key;
         key += cd.ns_cap;
-        // rows of the grouped lists: every key's region
-        cd.reg_off = culls ? rows : cd.p_off;
-        rows += list_rows(cd.n_all, cd.ns_cap);
         (scan_by_cta(cd.n_chunks, cd.ns_cap) ? kblk : kblk_warp) += (cd.ns_cap + KBLK - 1) / KBLK;
         for (int k = 0; k < cd.ns_cap; ++k) h_slot_cloud_.push_back((int32_t)c);
     }
     n_slots_ = (int32_t)key;
-    list_rows_ = rows;
     hist_ints_ = hist;
+    lay_out_lists(cull_possible());
     n_kblk_ = (int32_t)kblk;
     n_kblk_warp_ = (int32_t)kblk_warp;
     // group decimation scratch
@@ -438,7 +434,6 @@ int Engine::finish_setup_after_choose(cudaStream_t st, bool ns_given)
     RD_CK(upload(bDecHoff_, h_dec_hoff_, st));
     RD_CK(upload(bDecHbits_, h_dec_hbits_, st));
     RD_CK(bHist_.ensure(4 * (size_t)(hist + 1)));
-    RD_CK(bHpre_.ensure(4 * (size_t)(hist + 1)));
     RD_CK(bCnt_.ensure(4 * (size_t)(key + 1)));
     RD_CK(bBase_.ensure(4 * (size_t)(key + 1)));
     RD_CK(bKinfo_.ensure(sizeof(int4) * (size_t)(key + 1)));
@@ -631,21 +626,42 @@ int Engine::run(cudaStream_t st, bool use_graph, int mode)
     return collect(st);
 }
 
+// Where each cloud's grouped lists start.  With lists (keep), every key has a region
+// with room to grow; otherwise a cloud's lists take its points' places.
+void Engine::lay_out_lists(bool keep)
+{
+    lists_ = keep;
+    for (const CloudDesc& cd : h_cl_) lists_ = lists_ && lists_possible(cd.n_all, cd.ns_cap);
+    list_rows_ = 0;
+    for (CloudDesc& cd : h_cl_) {
+        cd.reg_off = list_rows_;
+        list_rows_ += list_rows(cd.n_all, cd.ns_cap);
+    }
+    // A caller's scratch stays within LIST_WS_MAX of what it is without lists.
+    if (current_arena() && list_bytes() > LIST_WS_MAX) lists_ = false;
+    if (!lists_)
+        for (CloudDesc& cd : h_cl_) cd.reg_off = cd.p_off;
+}
+
+int64_t Engine::list_bytes() const
+{
+    return list_rows_ * (2 * (pad_dim(dim_) * 4 + 4) + 4) + 4 * hist_ints_ + 4 * total_points_ +
+           4 * CAND_MAX * cull_blocks() + (int64_t)(2 * dim_ + 1) * 4 * n_slots_;
+}
+
 // buffers and state of the lockstep passes (cull_ is set)
 int Engine::start_passes(cudaStream_t st)
 {
-    if (cull_) {
-        if (int rc = ensure_cull_buffers()) return rc;
-        const EngineView vs = view();
-        RD_CK(launch_spatial_prep(dim_, vs, tune.cull_items, total_points_, bSpatialTmp_.p,
-                                  spatial_prep_scratch_bytes(total_points_), bPs_.as<float>(),
-                                  bSorder_.as<int32_t>(), bBox_.as<float>(), st));
-        // no point has a key yet: the culled assignment keeps the counts by its
-        // changes
-        RD_CK(cudaMemsetAsync(bHist_.p, 0, 4 * (size_t)(hist_ints_ + 1), st));
-    } else {
-        RD_CK(bPg_.ensure(sizeof(float) * (size_t)(total_points_ * pad_dim(dim_) + 4)));
-    }
+    if (!cull_) lists_ = false;
+    if (int rc = ensure_pass_buffers(st)) return rc;
+    if (!cull_) return 0;
+    const EngineView vs = view();
+    RD_CK(launch_spatial_prep(dim_, vs, tune.cull_items, total_points_, bSpatialTmp_.p,
+                              spatial_prep_scratch_bytes(total_points_), bPs_.as<float>(),
+                              bSorder_.as<int32_t>(), bBox_.as<float>(), st));
+    // no point has a key yet: with lists the assignment keeps the counts by its
+    // changes
+    RD_CK(cudaMemsetAsync(bHist_.p, 0, 4 * (size_t)(hist_ints_ + 1), st));
     return 0;
 }
 
@@ -660,30 +676,58 @@ void Engine::read_switches()
 // whether the lockstep passes of this batch assign with culling
 bool Engine::cull_possible() const
 {
-    return cull_on_ && cull_allowed_ && spatial_ok_ && total_points_ > 0;
+    return cull_on_ && spatial_ok_ && total_points_ > 0;
 }
 
-// buffers of the culled assignment (sizes known after choose)
-int Engine::ensure_cull_buffers()
+// blocks of points of the culled assignment
+int64_t Engine::cull_blocks() const { return (int64_t)n_chunks_ * (chunk_pts_ / (32 * tune.cull_items)); }
+
+// Buffers of the lockstep passes (sizes known after choose).  The kept lists take 60
+// to 70 bytes a point and a second histogram more than regrouping in every pass does;
+// where the device has no room for them the run goes without.
+int Engine::ensure_pass_buffers(cudaStream_t st)
 {
     const size_t n = (size_t)total_points_;
-    const size_t blocks = (size_t)n_chunks_ * (chunk_pts_ / (32 * tune.cull_items));
-    RD_CK(bPs_.ensure(sizeof(float) * (n * pad_dim(dim_) + 4)));
-    RD_CK(bSorder_.ensure(sizeof(int32_t) * (2 * n + 1)));
-    RD_CK(bSpatialTmp_.ensure(spatial_prep_scratch_bytes(total_points_)));
-    RD_CK(bKsp_.ensure(sizeof(int32_t) * (n + 1)));
-    RD_CK(bBox_.ensure(sizeof(float) * (4 * dim_ * blocks + 1)));
-    RD_CK(bSlack_.ensure(sizeof(float) * (blocks + 1)));
-    RD_CK(bLslack_.ensure(sizeof(float) * (blocks + 1)));
-    RD_CK(bBlen_.ensure(sizeof(int32_t) * (blocks + 1)));
-    RD_CK(bBlist_.ensure(sizeof(int32_t) * (CAND_MAX * blocks + 1)));
-    for (int b = 0; b < 2; ++b) {
-        RD_CK(bLr_[b].ensure(sizeof(float) * ((size_t)list_rows_ * pad_dim(dim_) + 4)));
-        RD_CK(bLs_[b].ensure(sizeof(int32_t) * ((size_t)list_rows_ + 1)));
+    const size_t blocks = (size_t)cull_blocks();
+    if (cull_) {
+        RD_CK(bPs_.ensure(sizeof(float) * (n * pad_dim(dim_) + 4)));
+        RD_CK(bSorder_.ensure(sizeof(int32_t) * (2 * n + 1)));
+        RD_CK(bSpatialTmp_.ensure(spatial_prep_scratch_bytes(total_points_)));
+        RD_CK(bBox_.ensure(sizeof(float) * (4 * dim_ * blocks + 1)));
+        RD_CK(bSlack_.ensure(sizeof(float) * (blocks + 1)));
+        RD_CK(bLslack_.ensure(sizeof(float) * (blocks + 1)));
+        RD_CK(bBlen_.ensure(sizeof(int32_t) * (blocks + 1)));
     }
-    RD_CK(bEdit_.ensure(sizeof(int32_t) * ((size_t)list_rows_ + 1)));
-    RD_CK(bMv_.ensure(sizeof(float) * ((size_t)(2 * dim_ + 1) * n_slots_ + 1)));
+    if (lists_) {
+        const cudaError_t e = ensure_list_buffers();
+        if (e == cudaErrorMemoryAllocation && !current_arena()) {
+            (void)cudaGetLastError();
+            for (DevBuf* b : {&bLr_[0], &bLr_[1], &bLs_[0], &bLs_[1], &bEdit_, &bHpre_, &bKsp_, &bBlist_, &bMv_})
+                b->release();
+            lay_out_lists(false);
+            RD_CK(upload(bCl_, h_cl_, st));
+        } else if (e != cudaSuccess) {
+            return fail("buffers of the member lists", e);
+        }
+    }
+    if (!lists_) RD_CK(bPg_.ensure(sizeof(float) * (n * pad_dim(dim_) + 4)));
     return 0;
+}
+
+cudaError_t Engine::ensure_list_buffers()
+{
+    const size_t rows = (size_t)list_rows_, blocks = (size_t)cull_blocks();
+    cudaError_t e = bHpre_.ensure(4 * (size_t)(hist_ints_ + 1));
+    auto take = [&](DevBuf& b, size_t bytes) { if (e == cudaSuccess) e = b.ensure(bytes); };
+    take(bKsp_, sizeof(int32_t) * ((size_t)total_points_ + 1));
+    take(bBlist_, sizeof(int32_t) * (CAND_MAX * blocks + 1));
+    for (int b = 0; b < 2; ++b) {
+        take(bLr_[b], sizeof(float) * (rows * pad_dim(dim_) + 4));
+        take(bLs_[b], sizeof(int32_t) * (rows + 1));
+    }
+    take(bEdit_, sizeof(int32_t) * (rows + 1));
+    take(bMv_, sizeof(float) * ((size_t)(2 * dim_ + 1) * n_slots_ + 1));
+    return e;
 }
 
 // Tiles (clouds) by decreasing evolve points; the heavy ones (evolved by a
@@ -722,11 +766,8 @@ int Engine::plan_workspace(int mode)
     if (mode == RUN_EVOLVE_ONLY || mode == RUN_DECIMATE_ONLY) {
         if (int rc = finish_setup_after_choose(nullptr)) return rc;
         if (mode == RUN_EVOLVE_ONLY) {
-            if (cull_possible()) {
-                if (int rc = ensure_cull_buffers()) return rc;
-            } else {
-                RD_CK(bPg_.ensure(sizeof(float) * (size_t)(total_points_ * pad_dim(dim_) + 4)));
-            }
+            cull_ = cull_possible();
+            if (int rc = ensure_pass_buffers(nullptr)) return rc;
         }
         return 0;
     }

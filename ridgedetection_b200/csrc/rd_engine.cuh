@@ -88,7 +88,7 @@ struct EngineView {
     // [base, base + kcap) of its cloud's part (reg_off) of two buffers; the
     // current list is in buffer par
     float* Lr[2];                // coordinates, PadDim floats per row
-    int32_t* Ls[2];              // the points' positions in their cloud (culled assignment only)
+    int32_t* Ls[2];              // the points' positions in their cloud (with lists)
     int4* kinfo;                 // per chosen slot: base, kcap, members, par
     int32_t* edit;               // per row: edits of this pass, at the key's region
     int32_t* ecnt;               // per chosen slot: edits of this pass
@@ -96,7 +96,8 @@ struct EngineView {
     int32_t* reb;                // per cloud: regroup all points in this pass
     int32_t* rebnext;            // per cloud: and in the next one
     int32_t* hist;               // per cloud: n_chunks x ns_cap key histogram
-    int32_t* hpre;               // the same shape: its exclusive prefix over the chunks
+    int32_t* hpre;               // the same shape: its exclusive prefix over the chunks (hist itself
+                                 // in runs without lists, which count anew in every pass)
     int32_t* cnt;                // per chosen slot: members in the last pass
     int32_t* base;               // per chosen slot: first row of its region
     int32_t* kbdone;             // per cloud: key blocks of the chunk scan finished in this pass
@@ -165,6 +166,9 @@ struct EngineView {
     float* mv;                   // 2*DIM+1 arrays of n_slots: each cloud's moves at its key_off
                                  // (old place, new place, length rounded up)
     int32_t cull;                // passes assign with k_assign_cull
+    int32_t lists;               // and keep member lists, candidates and slacks from pass to pass
+                                 // (else every pass evaluates and regroups every point)
+    int64_t hist_ints;           // entries of hist
     int32_t long_lists;          // few chosen points: k_merge_fold's variant for long lists
     // fused tiled runs: tiles by decreasing evolve points, the first n_heavy
     // evolved by whole thread-block clusters (rd_tile_cluster.cuh)

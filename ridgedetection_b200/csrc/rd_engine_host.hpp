@@ -32,6 +32,9 @@ struct ArenaScope {
     ~ArenaScope();
 };
 
+// bytes by which kept member lists may enlarge a caller's scratch
+constexpr int64_t LIST_WS_MAX = int64_t(16) << 30;
+
 // A device buffer that only grows; reused across runs of one engine.
 struct DevBuf {
     void* p = nullptr;
@@ -155,7 +158,11 @@ private:
     // once per run: the process-wide culling switch as this run takes it
     void read_switches();
     bool cull_possible() const;
-    int ensure_cull_buffers();
+    void lay_out_lists(bool keep);
+    int64_t list_bytes() const;
+    int64_t cull_blocks() const;
+    int ensure_pass_buffers(cudaStream_t st);
+    cudaError_t ensure_list_buffers();
     int start_passes(cudaStream_t st);
     void build_tile_order();
     int collect(cudaStream_t st);
@@ -191,7 +198,7 @@ private:
     bool cull_on_ = true;         // the culling switch when this run started
     bool cull_ = false;           // this run assigns with culling
     bool spatial_ok_ = false;     // the batch layout allows the spatial order
-    bool cull_allowed_ = true;    // and its size, and the kind of run, the culled assignment
+    bool lists_ = false;          // and keeps member lists from pass to pass
     int64_t list_rows_ = 0;       // rows of the grouped lists of the culled assignment
     DevBuf bLr_[2], bLs_[2], bKinfo_, bEdit_, bEcnt_, bDlist_, bReb_, bRebNext_;
     DevBuf bPs_, bSorder_, bSpatialTmp_, bHpre_;

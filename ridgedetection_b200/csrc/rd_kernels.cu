@@ -751,18 +751,18 @@ constexpr int EDIT_IN = (int)0x80000000;   // edit of a member list: this point 
 constexpr int EDIT_MAX = 512;              // edits of one key that k_merge_fold takes
 
 // rows of a key's region of the grouped lists with n members at the rebuild:
-// room for its list to grow before the next rebuild (without the culled
-// assignment every pass rebuilds)
+// room for its list to grow before the next rebuild (without lists every pass
+// rebuilds)
 __device__ __forceinline__ int list_cap(const EngineView& v, const int n)
 {
-    return v.cull ? list_room(n) : n;
+    return v.lists ? list_room(n) : n;
 }
 
 // A pass regroups all points of a cloud by key: its chosen points are new or
 // renumbered, or a key got more edits than it takes.
 __device__ __forceinline__ bool rebuilds(const EngineView& v, const int c)
 {
-    return !v.cull || v.full[c] != 0 || v.reb[c] != 0;
+    return !v.lists || v.full[c] != 0 || v.reb[c] != 0;
 }
 
 // One edit of key k's member list.  The first one of the pass lists the key as
@@ -820,7 +820,7 @@ __global__ void __launch_bounds__(AC_BLOCK, ITEMS <= 4 ? 4 : 2) k_assign_cull(En
             if ((int64_t)my_i * WPTS < my_n) {
                 const int64_t wb =
                     ((v.single ? v.one.chunk_begin : v.cl[my_c].chunk_begin) << wpc_log) + my_i;
-                my_full = v.full[my_c];
+                my_full = v.lists ? v.full[my_c] : 1;
                 const float dmax = __int_as_float(v.dmax[my_c]);
                 my_slack = v.bslack[wb];
                 need = my_full || !(my_slack > dmax);
@@ -898,7 +898,8 @@ __global__ void __launch_bounds__(AC_BLOCK, ITEMS <= 4 ? 4 : 2) k_assign_cull(En
                 old[j] = -1;
                 if (i < cd.n_all) {
                     load_chosen<DIM>(Ps, i, p);
-                    old[j] = ksp[i];
+                    // without lists: every key is written anew
+                    old[j] = v.lists ? ksp[i] : -2;
                 }
 #pragma unroll
                 for (int d = 0; d < DIM; ++d) {
@@ -953,7 +954,7 @@ __global__ void __launch_bounds__(AC_BLOCK, ITEMS <= 4 ? 4 : 2) k_assign_cull(En
                     const unsigned nb = __ballot_sync(FULL, near);
                     if (!nb) continue;
                     const int at = len + __popc(nb & lanemask_lt());
-                    if (near && at < CAND_MAX) list[at] = q;
+                    if (near && at < CAND_MAX && v.lists) list[at] = q;
                     len += __popc(nb);
                     take(__ballot_sync(FULL, q < ns && !(may_skip && g2 > thr)), s, q);
                 }
@@ -978,7 +979,7 @@ __global__ void __launch_bounds__(AC_BLOCK, ITEMS <= 4 ? 4 : 2) k_assign_cull(En
                     const int slot = v.sorder[cd.p_off + i];
                     int32_t* row = hist + (int64_t)v.srow[cd.p_off + i] * cd.ns_cap;
                     v.keys[slot] = k;
-                    ksp[i] = k;
+                    if (v.lists) ksp[i] = k;
                     if (old[j] >= 0) {
                         atomicAdd(&row[old[j]], -1);
                         if (!full) push_edit(v, c, cd, old[j], (int)(slot - cd.p_off));
@@ -1411,7 +1412,7 @@ __global__ void __launch_bounds__(SCAT_W * 32) k_scatter_cta(EngineView v)
                 for (int d = 0; d < DIM; ++d) qv[d] = __shfl_sync(FULL, pc[q][d], r.src);
                 if (r.key >= 0) {
                     store_row<DIM>(Pg, b + r.rank, qv);
-                    if (v.cull) Ls[b + r.rank] = start + i0 + r.src;
+                    if (v.lists) Ls[b + r.rank] = start + i0 + r.src;
                 }
             }
         }
@@ -1494,7 +1495,7 @@ __device__ void scatter_chunk(const EngineView& v, int c, int lc, int* s_keys, i
         for (int d = 0; d < DIM; ++d) q[d] = __shfl_sync(FULL, pc[d], r.src);
         if (r.key >= 0) {
             store_row<DIM>(Pg, b + r.rank, q);
-            if (v.cull) Ls[b + r.rank] = start + off + r.src;
+            if (v.lists) Ls[b + r.rank] = start + off + r.src;
         }
         __syncwarp();
     }
@@ -1602,7 +1603,7 @@ __device__ void apply_shift(const EngineView& v, int c, const CloudDesc& cd, int
         }
     }
     if (__any_sync(FULL, moved) && lane == 0) v.cont[c] = 1;
-    if (!v.cull || !__any_sync(FULL, changed)) return;
+    if (!v.lists || !__any_sync(FULL, changed)) return;
     // the move, for the blocks of points near it (k_assign_cull): old and new
     // place, and its length rounded up
     const float dd = fabsf(__fsub_rn(now, was));
@@ -1913,7 +1914,7 @@ __device__ void merge_fold_key(const EngineView& v, const int slot, const bool s
     const bool seg = seg_ok && ne == 0 && n_old >= (LONG ? SUM_BIG_MIN : SUM_BIG_MIN_SLOW);
     const int steps = seg ? 0 : (max(n_old, 1) + MF_ROWS - 1) / MF_ROWS;
     float sum = 0.0f;
-    const int32_t* pos = v.cull ? v.Ls[par] + at : nullptr;
+    const int32_t* pos = v.lists ? v.Ls[par] + at : nullptr;
     // edits before chunk s's first row (those before the list's first row go to chunk 0)
     auto find_cuts = [&](const int s0) {
         for (int i = tid; i <= MF_CUTS; i += BLOCK) {
@@ -1952,7 +1953,7 @@ __device__ void merge_fold_key(const EngineView& v, const int slot, const bool s
             }
         } else {
             float* dst = v.Lr[par ^ 1] + at * DP;
-            int32_t* dpos = (v.cull ? v.Ls[par ^ 1] + at : nullptr);
+            int32_t* dpos = (v.lists ? v.Ls[par ^ 1] + at : nullptr);
             const int pt = tid - 32;
             auto load = [&](const int s) {
                 const int j = s * MF_ROWS + pt, b = s % MF_STAGES;
@@ -3340,6 +3341,12 @@ cudaError_t launch_evolve_kernels(const EngineView& v, const TuneParams& tp, int
     if (a0) cudaEventRecord(a0, st);
     if (v.cull) {
         cudaError_t e;
+        if (!v.lists) {
+            // counted anew (its rows hold the last pass's prefixes)
+            e = cudaMemsetAsync(v.hist, 0, 4 * (size_t)v.hist_ints, st);
+            if (e != cudaSuccess) return e;
+            assign_pdl = 0;   // follows no kernel
+        }
         if (tp.cull_items == 2) e = launch_assign_cull<DIM, 2>(v, assign_pdl, st);
         else if (tp.cull_items == 8) e = launch_assign_cull<DIM, 8>(v, assign_pdl, st);
         else e = launch_assign_cull<DIM, 4>(v, assign_pdl, st);

@@ -25,4 +25,11 @@ RD_ROOM_HD constexpr int list_room(const int n) { return n + (n >> 2) + 8; }
 // rows that the regions of ns keys with n members in all can take
 RD_ROOM_HD constexpr int64_t list_rows(const int64_t n, const int64_t ns) { return n + n / 4 + 8 * ns; }
 
+// Whether a cloud's lists can be kept: their rows and the points' positions in them
+// are 31-bit numbers.
+RD_ROOM_HD constexpr bool lists_possible(const int64_t n, const int64_t ns)
+{
+    return n <= (int64_t(1) << 30) && list_rows(n, ns) <= INT32_MAX;
+}
+
 }  // namespace rdb

@@ -130,3 +130,45 @@ def test_nearly_all_chosen(rdb, n):
     for c, (Q, q1, q2) in enumerate(clouds):
         assert bits_equal(b.chosen_points(c), rdb.ridge_detection(Q, q1, q2)[0]), c
     b.close()
+
+
+@pytest.mark.parametrize("batch", [False, True])
+def test_lists_that_do_not_fit_the_device(rdb, batch):
+    """With room for the points but not for the kept lists the run regroups in every pass:
+    same bits, same passes."""
+    torch = require_cuda()
+    n = 6_000_000
+    P = torch.from_numpy(G.helix3d(n, seed=21)).cuda()
+    flat = P.reshape(-1)
+    descs = [(0, 3_500_000, 3, 0.3, 0.6), (10_500_000, 2_500_000, 3, 0.4, 0.8)]
+
+    def run():
+        if batch:
+            h = rdb.BatchedRidgeDetection()
+            h.run(flat, descs)
+            out = [h.chosen_points(0), h.chosen_points(1)], h.stats().evolve_passes
+        else:
+            h = rdb.BruteForceRidgeDetection(n, 0.3, 0.6, 3)
+            h.set_points(P)
+            h.ridge_detection()
+            out = [h.chosen_points()], h.stats().evolve_passes
+        used = free0 - torch.cuda.mem_get_info()[0]
+        h.close()
+        return out, used
+
+    free0 = 0
+    run()   # whatever a first run leaves on the device
+    torch.cuda.empty_cache()
+    free0 = torch.cuda.mem_get_info()[0]
+    (want, passes), used = run()
+    lists = 63 * n
+    assert used > 3 * lists // 2
+    torch.cuda.synchronize()
+    free0 = torch.cuda.mem_get_info()[0]
+    hold = torch.empty(free0 - (used - 2 * lists // 5), dtype=torch.uint8, device="cuda")
+    try:
+        (got, p), _ = run()
+    finally:
+        del hold
+        torch.cuda.empty_cache()
+    assert p == passes and all(bits_equal(x, y) for x, y in zip(got, want))

@@ -51,3 +51,20 @@ def test_sizes_are_stated_once():
     host, dev = (open(os.path.join(csrc, f)).read() for f in ("rd_engine.cu", "rd_kernels.cu"))
     assert "list_rows(" in host and "CAND_MAX * blocks" in host
     assert "list_room(n)" in dev and "at < CAND_MAX" in dev
+
+
+def test_limits_are_per_cloud(tmp_path):
+    src, exe = tmp_path / "l.cpp", tmp_path / "l"
+    src.write_text('#include "rd_listroom.hpp"\n#include <cstdio>\n#include <cstdlib>\n'
+                   'int main(int, char** a) { printf("%d", rdb::lists_possible(atoll(a[1]), atoll(a[2]))); }\n')
+    subprocess.run(["g++", "-std=c++17", "-I", os.path.join(ROOT, "ridgedetection_b200", "csrc"), str(src),
+                    "-o", str(exe)], check=True)
+
+    def possible(n, ns):
+        return subprocess.run([str(exe), str(n), str(ns)], check=True, capture_output=True, text=True).stdout == "1"
+    assert possible(10 ** 6, 10 ** 6) and possible(2 ** 30, 1000) and possible(0, 5)
+    assert not possible(2 ** 30 + 1, 1)                 # positions of the edits
+    assert not possible(2 ** 28, 2 ** 28)               # rows past 2^31
+    # the batch has no say: the engine asks for every cloud, and sorts up to 2^31 points
+    host = open(os.path.join(ROOT, "ridgedetection_b200", "csrc", "rd_engine.cu")).read()
+    assert "lists_possible(cd.n_all, cd.ns_cap)" in host and "total_points <= (int64_t(1) << 30)" not in host
