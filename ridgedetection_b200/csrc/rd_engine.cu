@@ -357,7 +357,9 @@ EngineView Engine::view() const
     v.cull = cull_ ? 1 : 0;
     v.lists = lists_ ? 1 : 0;
     v.hist_ints = hist_ints_;
+    v.n_points = total_points_;
     v.long_lists = n_slots_ > 0 && total_points_ / n_slots_ >= long_list_avg() ? 1 : 0;
+    v.merge_cap = merge_cap(v.long_lists != 0);
     v.tile_order = bTileOrder_.as<int32_t>();
     v.n_heavy = n_heavy_;
     v.tile_clusters = tile_clusters_ ? 1 : 0;
@@ -645,8 +647,8 @@ void Engine::lay_out_lists(bool keep)
 
 int64_t Engine::list_bytes() const
 {
-    return list_rows_ * (2 * (pad_dim(dim_) * 4 + 4) + 4) + 4 * hist_ints_ + 4 * total_points_ +
-           4 * CAND_MAX * cull_blocks() + (int64_t)(2 * dim_ + 1) * 4 * n_slots_;
+    return list_rows_ * (2 * (pad_dim(dim_) * 4 + 4) + 4) + 4 * hist_ints_ +
+           (int64_t)(2 * dim_ + 1) * 4 * n_slots_;
 }
 
 // buffers and state of the lockstep passes (cull_ is set)
@@ -682,8 +684,8 @@ bool Engine::cull_possible() const
 // blocks of points of the culled assignment
 int64_t Engine::cull_blocks() const { return (int64_t)n_chunks_ * (chunk_pts_ / (32 * tune.cull_items)); }
 
-// Buffers of the lockstep passes (sizes known after choose).  The kept lists take 60
-// to 70 bytes a point and a second histogram more than regrouping in every pass does;
+// Buffers of the lockstep passes (sizes known after choose).  The kept lists take 25
+// to 55 bytes a point and a second histogram more than regrouping in every pass does;
 // where the device has no room for them the run goes without.
 int Engine::ensure_pass_buffers(cudaStream_t st)
 {
@@ -697,12 +699,14 @@ int Engine::ensure_pass_buffers(cudaStream_t st)
         RD_CK(bSlack_.ensure(sizeof(float) * (blocks + 1)));
         RD_CK(bLslack_.ensure(sizeof(float) * (blocks + 1)));
         RD_CK(bBlen_.ensure(sizeof(int32_t) * (blocks + 1)));
+        RD_CK(bKsp_.ensure(sizeof(int32_t) * (n + 1)));
+        RD_CK(bBlist_.ensure(sizeof(int32_t) * (CAND_MAX * blocks + 1)));
     }
     if (lists_) {
         const cudaError_t e = ensure_list_buffers();
         if (e == cudaErrorMemoryAllocation && !current_arena()) {
             (void)cudaGetLastError();
-            for (DevBuf* b : {&bLr_[0], &bLr_[1], &bLs_[0], &bLs_[1], &bEdit_, &bHpre_, &bKsp_, &bBlist_, &bMv_})
+            for (DevBuf* b : {&bLr_[0], &bLr_[1], &bLs_[0], &bLs_[1], &bEdit_, &bHpre_, &bMv_})
                 b->release();
             lay_out_lists(false);
             RD_CK(upload(bCl_, h_cl_, st));
@@ -716,11 +720,9 @@ int Engine::ensure_pass_buffers(cudaStream_t st)
 
 cudaError_t Engine::ensure_list_buffers()
 {
-    const size_t rows = (size_t)list_rows_, blocks = (size_t)cull_blocks();
+    const size_t rows = (size_t)list_rows_;
     cudaError_t e = bHpre_.ensure(4 * (size_t)(hist_ints_ + 1));
     auto take = [&](DevBuf& b, size_t bytes) { if (e == cudaSuccess) e = b.ensure(bytes); };
-    take(bKsp_, sizeof(int32_t) * ((size_t)total_points_ + 1));
-    take(bBlist_, sizeof(int32_t) * (CAND_MAX * blocks + 1));
     for (int b = 0; b < 2; ++b) {
         take(bLr_[b], sizeof(float) * (rows * pad_dim(dim_) + 4));
         take(bLs_[b], sizeof(int32_t) * (rows + 1));

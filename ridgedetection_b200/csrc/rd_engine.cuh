@@ -169,7 +169,9 @@ struct EngineView {
     int32_t lists;               // and keep member lists, candidates and slacks from pass to pass
                                  // (else every pass evaluates and regroups every point)
     int64_t hist_ints;           // entries of hist
+    int64_t n_points;
     int32_t long_lists;          // few chosen points: k_merge_fold's variant for long lists
+    int32_t merge_cap;           // a key with a region this large regroups its cloud when edited
     // fused tiled runs: tiles by decreasing evolve points, the first n_heavy
     // evolved by whole thread-block clusters (rd_tile_cluster.cuh)
     const int32_t* tile_order;
@@ -277,6 +279,7 @@ cudaError_t launch_evolve_step(int dim, const EngineView& v, const TuneParams& t
                                cudaStream_t st);
 // points per chosen point from which a run takes the variant for long lists
 int long_list_avg();
+int merge_cap(bool long_lists);   // EngineView::merge_cap
 int assign_smem_bytes(int dim, const TuneParams& tp, int hist_ints);
 int max_assign_blocks_per_sm(int dim, const TuneParams& tp, int hist_ints);
 bool tune_supported(int dim, const TuneParams& tp);

@@ -776,7 +776,6 @@ __device__ __forceinline__ void push_edit(const EngineView& v, const int c, cons
     const int2 reg = *reinterpret_cast<const int2*>(v.kinfo + s);   // base, capacity
     if (at < min(EDIT_MAX, reg.y)) v.edit[cd.reg_off + reg.x + at] = edit;
     else v.reb[c] = 1;
-    if (reg.y >= (v.long_lists ? MERGE_CAP_LONG : MERGE_CAP)) v.reb[c] = 1;
 }
 
 // resident CTAs the registers are held to: the evaluation waits on memory
@@ -820,7 +819,7 @@ __global__ void __launch_bounds__(AC_BLOCK, ITEMS <= 4 ? 4 : 2) k_assign_cull(En
             if ((int64_t)my_i * WPTS < my_n) {
                 const int64_t wb =
                     ((v.single ? v.one.chunk_begin : v.cl[my_c].chunk_begin) << wpc_log) + my_i;
-                my_full = v.lists ? v.full[my_c] : 1;
+                my_full = v.full[my_c];
                 const float dmax = __int_as_float(v.dmax[my_c]);
                 my_slack = v.bslack[wb];
                 need = my_full || !(my_slack > dmax);
@@ -898,8 +897,7 @@ __global__ void __launch_bounds__(AC_BLOCK, ITEMS <= 4 ? 4 : 2) k_assign_cull(En
                 old[j] = -1;
                 if (i < cd.n_all) {
                     load_chosen<DIM>(Ps, i, p);
-                    // without lists: every key is written anew
-                    old[j] = v.lists ? ksp[i] : -2;
+                    old[j] = ksp[i];
                 }
 #pragma unroll
                 for (int d = 0; d < DIM; ++d) {
@@ -954,7 +952,7 @@ __global__ void __launch_bounds__(AC_BLOCK, ITEMS <= 4 ? 4 : 2) k_assign_cull(En
                     const unsigned nb = __ballot_sync(FULL, near);
                     if (!nb) continue;
                     const int at = len + __popc(nb & lanemask_lt());
-                    if (near && at < CAND_MAX && v.lists) list[at] = q;
+                    if (near && at < CAND_MAX) list[at] = q;
                     len += __popc(nb);
                     take(__ballot_sync(FULL, q < ns && !(may_skip && g2 > thr)), s, q);
                 }
@@ -979,7 +977,7 @@ __global__ void __launch_bounds__(AC_BLOCK, ITEMS <= 4 ? 4 : 2) k_assign_cull(En
                     const int slot = v.sorder[cd.p_off + i];
                     int32_t* row = hist + (int64_t)v.srow[cd.p_off + i] * cd.ns_cap;
                     v.keys[slot] = k;
-                    if (v.lists) ksp[i] = k;
+                    ksp[i] = k;
                     if (old[j] >= 0) {
                         atomicAdd(&row[old[j]], -1);
                         if (!full) push_edit(v, c, cd, old[j], (int)(slot - cd.p_off));
@@ -1034,7 +1032,8 @@ __device__ __forceinline__ void clear_moves(const EngineView& v, const int first
 __device__ __forceinline__ void place_key(const EngineView& v, const int64_t s, const int at, const int cap)
 {
     v.base[s] = at;
-    v.kinfo[s] = make_int4(at, cap, v.cnt[s], 0);
+    // a long list takes no edits: the first one regroups the cloud
+    v.kinfo[s] = make_int4(at, cap < v.merge_cap ? cap : 0, v.cnt[s], 0);
     if (v.ecnt[s] == 0) v.dlist[atomicAdd(&v.ctr[CTR_NDIRTY], 1)] = (int)s;  // else push_edit did
 }
 
@@ -1742,7 +1741,7 @@ struct MergeSmem {
 // cloud c after a pass: the next one evaluates and regroups what this one left
 __device__ __forceinline__ void next_pass(const EngineView& v, const int c)
 {
-    v.full[c] = 0;
+    v.full[c] = v.lists ? 0 : 1;
     v.reb[c] = v.rebnext[c];
     v.rebnext[c] = 0;
 }
@@ -2033,7 +2032,7 @@ __device__ void merge_fold_key(const EngineView& v, const int slot, const bool s
             v.ecnt[slot] = 0;
             v.cnt[slot] = n_new;
             v.kinfo[slot] = make_int4(info.x, cap, n_new, (ne > 0) ? par ^ 1 : par);
-            if (n_new > cap) v.rebnext[c] = 1;
+            if (ne > 0 && n_new > cap) v.rebnext[c] = 1;
         }
         if (n_new > 0) apply_shift<DIM>(v, c, cd, k, n_new, sum, lane);
     }
@@ -3342,8 +3341,10 @@ cudaError_t launch_evolve_kernels(const EngineView& v, const TuneParams& tp, int
     if (v.cull) {
         cudaError_t e;
         if (!v.lists) {
-            // counted anew (its rows hold the last pass's prefixes)
+            // assigned and counted anew (the counts' rows hold the last pass's prefixes)
             e = cudaMemsetAsync(v.hist, 0, 4 * (size_t)v.hist_ints, st);
+            if (e == cudaSuccess) e = cudaMemsetAsync(v.keys, 0xff, 4 * (size_t)v.n_points, st);
+            if (e == cudaSuccess) e = cudaMemsetAsync(v.ksp, 0xff, 4 * (size_t)v.n_points, st);
             if (e != cudaSuccess) return e;
             assign_pdl = 0;   // follows no kernel
         }
@@ -3704,6 +3705,7 @@ bool tune_supported(int dim, const TuneParams& tp)
 }
 
 int long_list_avg() { return LONG_AVG; }
+int merge_cap(bool long_lists) { return long_lists ? MERGE_CAP_LONG : MERGE_CAP; }
 
 int assign_smem_bytes(int dim, const TuneParams& tp, int hist_ints)
 {

@@ -123,7 +123,7 @@ __global__ void __launch_bounds__(256) k_gather_spatial(EngineView v, int items,
             if (in) {
                 sorder[n + pos] = slot_chunk((int)(s - cd.p_off), cd.n_all, cd.n_chunks, ratio);
                 sorder[pos] = s;
-                if (v.lists) v.ksp[pos] = -1;
+                v.ksp[pos] = -1;
             }
 #pragma unroll
             for (int d = 0; d < DIM; ++d) {

@@ -161,7 +161,7 @@ def test_lists_that_do_not_fit_the_device(rdb, batch):
     torch.cuda.empty_cache()
     free0 = torch.cuda.mem_get_info()[0]
     (want, passes), used = run()
-    lists = 63 * n
+    lists = 55 * n
     assert used > 3 * lists // 2
     torch.cuda.synchronize()
     free0 = torch.cuda.mem_get_info()[0]
