@@ -127,7 +127,7 @@ cudaError_t DevBuf::ensure(size_t want)
         gen = a->gen;
         return cudaSuccess;
     }
-    if (want <= bytes && !borrowed) return cudaSuccess;
+    if (want <= bytes && (!borrowed || in_slab)) return cudaSuccess;
     release();
     cudaError_t e = cudaMalloc(&p, want);
     if (e != cudaSuccess) {
@@ -144,7 +144,65 @@ void DevBuf::release()
     if (p && !borrowed) cudaFree(p);
     p = nullptr;
     bytes = 0;
-    borrowed = false;
+    borrowed = in_slab = false;
+}
+
+cudaError_t ensure_together(DevBuf& slab, const std::vector<SlabItem>& items)
+{
+    cudaError_t e = cudaSuccess;
+    if (t_arena) {
+        for (const SlabItem& it : items)
+            if ((e = it.buf->ensure(it.bytes)) != cudaSuccess) return e;
+        return cudaSuccess;
+    }
+    bool fits = true;
+    for (const SlabItem& it : items) {
+        const bool own = it.buf->p && !it.buf->borrowed;
+        if (it.bytes > SLAB_ITEM_MAX || (own && it.buf->bytes >= it.bytes)) {
+            if (it.buf->in_slab) it.buf->release();
+            if ((e = it.buf->ensure(it.bytes)) != cudaSuccess) return e;
+        } else {
+            if (own) it.buf->release();
+            fits = fits && it.buf->in_slab && it.buf->bytes >= std::max<size_t>(it.bytes, 1);
+        }
+    }
+    if (fits) return cudaSuccess;
+    // the second try is for exactly what is asked
+    const bool first = slab.p == nullptr;
+    for (int exact = first ? 1 : 0; exact < 2; ++exact) {
+        std::vector<size_t> off(items.size()), len(items.size());
+        size_t total = 0;
+        for (size_t i = 0; i < items.size(); ++i) {
+            const SlabItem& it = items[i];
+            if (it.buf->p && !it.buf->borrowed) continue;   // has its own
+            len[i] = std::max<size_t>(it.bytes, 16);
+            if (!exact) {
+                const size_t had = it.buf->in_slab ? it.buf->bytes : 0;
+                len[i] = std::max(had, len[i] > had ? len[i] + len[i] / 8 : len[i]);
+            }
+            total = (total + ARENA_ALIGN - 1) / ARENA_ALIGN * ARENA_ALIGN;
+            off[i] = total;
+            total += len[i];
+        }
+        slab.release();
+        if (exact)
+            for (const SlabItem& it : items)
+                if (it.buf->borrowed) it.buf->release();
+        if ((e = slab.ensure(total)) != cudaSuccess) {
+            if (!exact) (void)cudaGetLastError();
+            continue;
+        }
+        for (size_t i = 0; i < items.size(); ++i) {
+            if (!len[i]) continue;
+            DevBuf& b = *items[i].buf;
+            b.release();
+            b.p = static_cast<char*>(slab.p) + off[i];
+            b.bytes = len[i];
+            b.borrowed = b.in_slab = true;
+        }
+        return cudaSuccess;
+    }
+    return e;
 }
 
 Engine::Engine() {}
@@ -243,27 +301,19 @@ int Engine::setup(int dim, const std::vector<CloudDesc>& clouds,
         next_off += cd.n_all;
     }
     spatial_ok_ = spatial_ok_ && next_off == total_points;
-    RD_CK(bP_.ensure(sizeof(float) * (size_t)(total_points * dim + 4)));
-    RD_CK(bS_.ensure(sizeof(float) * (size_t)(s_off * dim + 4)));
-    RD_CK(bNext_.ensure(sizeof(int32_t) * (size_t)(s_off + 1)));
-    RD_CK(bKeys_.ensure(sizeof(int32_t) * (size_t)(total_points + 1)));
-    RD_CK(bRes_.ensure(res_bytes(nc)));
-    RD_CK(bPhase_.ensure(4 * (nc + 1)));
-    RD_CK(bCont_.ensure(4 * (nc + 1)));
-    RD_CK(bPasses_.ensure(4 * (nc + 1)));
-    RD_CK(bOuter_.ensure(4 * (nc + 1)));
-    RD_CK(bKbDone_.ensure(4 * (nc + 1)));
-    RD_CK(bFull_.ensure(4 * (nc + 1)));
-    RD_CK(bReb_.ensure(4 * (nc + 1)));
-    RD_CK(bRebNext_.ensure(4 * (nc + 1)));
-    RD_CK(bMvn_.ensure(4 * (nc + 1)));
-    RD_CK(bDmax_.ensure(4 * (nc + 1)));
-    RD_CK(bActCloud_.ensure(4 * (nc + 1)));
-    RD_CK(bActPre_.ensure(4 * ACT_KINDS * (nc + 1)));
-    RD_CK(bGroupConv_.ensure(4 * (h_gr_.size() + 1)));
-    RD_CK(bReady_.ensure(4 * (h_gr_.size() + 1)));
-    RD_CK(bDbig_.ensure(4 * 4));
-    RD_CK(bDcpre_.ensure(4 * (nc + 1)));
+    const size_t per = 4 * (nc + 1), per_group = 4 * (h_gr_.size() + 1);
+    RD_CK(ensure_together(slab_setup_, {
+        {&bRes_, res_bytes(nc)}, {&bPhase_, per}, {&bCont_, per}, {&bPasses_, per}, {&bOuter_, per},
+        {&bKbDone_, per}, {&bFull_, per}, {&bReb_, per}, {&bRebNext_, per}, {&bMvn_, per},
+        {&bDmax_, per}, {&bActCloud_, per}, {&bActPre_, ACT_KINDS * per}, {&bGroupConv_, per_group},
+        {&bReady_, per_group}, {&bDbig_, 4 * 4}, {&bDcpre_, per},
+        {&bCl_, sizeof(CloudDesc) * (nc + 1)}, {&bGr_, sizeof(GroupDesc) * (h_gr_.size() + 1)},
+        {&bTileOrder_, per}, {&bChunkCloud_, 4 * (h_chunk_cloud_.size() + 1)},
+        {&bP_, sizeof(float) * (size_t)(total_points * dim + 4)},
+        {&bS_, sizeof(float) * (size_t)(s_off * dim + 4)},
+        {&bNext_, sizeof(int32_t) * (size_t)(s_off + 1)},
+        {&bKeys_, sizeof(int32_t) * (size_t)(total_points + 1)},
+    }));
     return 0;
 }
 
@@ -324,7 +374,7 @@ EngineView Engine::view() const
     v.dbig = bDbig_.as<int32_t>();
     v.dcpre = bDcpre_.as<int32_t>();
     v.dec_smem_max = dec_smem_max_;
-    v.dec_dyn = dec_dyn_bytes(dec_smem_max_);
+    v.dec_dyn = dec_dyn_;
     v.dec_nb_pp = dec_nb_pp_;
     v.dec_hoff = bDecHoff_.as<int64_t>();
     v.dec_hbits = bDecHbits_.as<int32_t>();
@@ -380,7 +430,24 @@ static int ceil_log2(int64_t x)
     return b;
 }
 
-int Engine::finish_setup_after_choose(cudaStream_t st, bool ns_given)
+// The chosen points a run of one cloud is laid out for: a few more than it has, and as
+// many as the last one where that does, so that the clouds of a handle share their
+// buffers and their graph (1,000 points, another cloud each time: 1,340 us, the same
+// cloud 790, where every count was laid out exactly).
+int Engine::chosen_room(int ns)
+{
+    const CloudDesc& cd = h_cl_[0];
+    int step = 64;
+    while (8 * step <= ns) step *= 2;
+    int64_t room = (int64_t)(ns + step - 1) / step * step;
+    // the histogram has a row of them for every chunk
+    if (4 * room * cd.n_chunks > int64_t(64) << 20 || current_arena()) return ns;
+    if (room_points_ == cd.n_all && room_ >= ns && room_ <= 2 * room) return room_;
+    room_points_ = cd.n_all;
+    return room_ = (int)room;
+}
+
+int Engine::finish_setup_after_choose(cudaStream_t st, bool ns_given, bool exact)
 {
     const size_t nc = h_cl_.size();
     h_ns_.resize(nc);
@@ -396,7 +463,7 @@ int Engine::finish_setup_after_choose(cudaStream_t st, bool ns_given)
     h_slot_cloud_.clear();
     for (size_t c = 0; c < nc; ++c) {
         CloudDesc& cd = h_cl_[c];
-        cd.ns_cap = h_ns_[c];
+        cd.ns_cap = nc == 1 && !exact ? chosen_room(h_ns_[c]) : h_ns_[c];
         max_ns = std::max(max_ns, cd.ns_cap);
         cd.hist_off = hist;
         hist += (int64_t)cd.n_chunks * cd.ns_cap;
@@ -430,31 +497,33 @@ int Engine::finish_setup_after_choose(cudaStream_t st, bool ns_given)
     // shared-memory budgets (ints)
     hist_smem_ = std::min(max_ns, 24 * 1024);
     scat_smem_ = std::min(max_ns, 4 * 1024);
+    dec_nb_pp_ = (int)std::max<int64_t>(
+        DEC_NB_MIN_PER_POINT,
+        std::min({(int64_t)DEC_NB_MAX_PER_POINT, DEC_NB_BUDGET / std::max<int64_t>(sscr, 1), max_tot}));
+    const size_t slots = (size_t)key + 1, scr = (size_t)sscr + 1;
+    RD_CK(ensure_together(slab_chosen_, {
+        {&bSlotCloud_, 4 * (h_slot_cloud_.size() + 1)},
+        {&bDecHoff_, 8 * (h_dec_hoff_.size() + 1)}, {&bDecHbits_, 4 * (h_dec_hbits_.size() + 1)},
+        {&bHist_, 4 * (size_t)(hist + 1)},
+        {&bCnt_, 4 * slots}, {&bBase_, 4 * slots}, {&bKinfo_, sizeof(int4) * slots},
+        {&bEcnt_, 4 * slots}, {&bDlist_, 4 * slots},
+        {&bDx_, 4 * scr * dim_}, {&bDcell_, 4 * scr * dim_}, {&bDalive_, 4 * scr},
+        {&bDc1_, 4 * scr}, {&bDc2_, 4 * scr}, {&bDitems_, 4 * scr},
+        {&bDbstart_, 4 * (size_t)(hoff + 1)},
+        {&bDnbOff_, 4 * (size_t)(sscr + h_gr_.size() + 1)},
+        {&bDnb_, 4 * (size_t)((int64_t)dec_nb_pp_ * sscr + 1)},
+    }));
     RD_CK(upload(bCl_, h_cl_, st));
     RD_CK(upload(bGr_, h_gr_, st));
     RD_CK(upload(bSlotCloud_, h_slot_cloud_, st));
     RD_CK(upload(bDecHoff_, h_dec_hoff_, st));
     RD_CK(upload(bDecHbits_, h_dec_hbits_, st));
-    RD_CK(bHist_.ensure(4 * (size_t)(hist + 1)));
-    RD_CK(bCnt_.ensure(4 * (size_t)(key + 1)));
-    RD_CK(bBase_.ensure(4 * (size_t)(key + 1)));
-    RD_CK(bKinfo_.ensure(sizeof(int4) * (size_t)(key + 1)));
-    RD_CK(bEcnt_.ensure(4 * (size_t)(key + 1)));
-    RD_CK(bDlist_.ensure(4 * (size_t)(key + 1)));
     RD_CK(upload_zero(bEcnt_, 4 * (size_t)(key + 1), st));
-    RD_CK(bDx_.ensure(4 * (size_t)(sscr * dim_ + 1)));
-    RD_CK(bDcell_.ensure(4 * (size_t)(sscr * dim_ + 1)));
-    RD_CK(bDalive_.ensure(4 * (size_t)(sscr + 1)));
-    RD_CK(bDc1_.ensure(4 * (size_t)(sscr + 1)));
-    RD_CK(bDc2_.ensure(4 * (size_t)(sscr + 1)));
-    RD_CK(bDitems_.ensure(4 * (size_t)(sscr + 1)));
-    RD_CK(bDbstart_.ensure(4 * (size_t)(hoff + 1)));
-    RD_CK(bDnbOff_.ensure(4 * (size_t)(sscr + h_gr_.size() + 1)));
-    dec_nb_pp_ = (int)std::max<int64_t>(
-        DEC_NB_MIN_PER_POINT,
-        std::min<int64_t>(DEC_NB_MAX_PER_POINT, DEC_NB_BUDGET / std::max<int64_t>(sscr, 1)));
-    RD_CK(bDnb_.ensure(4 * (size_t)((int64_t)dec_nb_pp_ * sscr + 1)));
     dec_smem_max_ = (int)std::min<int64_t>(max_tot, DEC_SMEM_MAX_POINTS);
+    // where a room beyond the count would leave the sets whose matrices fit, the largest
+    // of those
+    dec_dyn_ = dec_dyn_bytes(h_gr_.size() == 1 && nc == 1 && h_ns_[0] <= dec_smem_points()
+                                 ? std::min(dec_smem_max_, dec_smem_points()) : dec_smem_max_);
     // persistent assignment grid: every resident CTA slot, at most one per chunk
     int dev = 0, sms = 0;
     RD_CK(cudaGetDevice(&dev));
@@ -516,6 +585,16 @@ int Engine::build_graph(cudaStream_t st)
     return 0;
 }
 
+// buffers of the choose of one large cloud
+cudaError_t Engine::ensure_choose()
+{
+    const int64_t n = h_cl_[0].n_own;
+    return ensure_together(slab_choose_, {{&bHash_, 4 * (size_t)choose_hash_buckets()},
+                                          {&bSurv_, (size_t)n + 16},
+                                          {&bSel_, 4 * (size_t)(n + 2)},
+                                          {&bSelTmp_, choose_select_scratch_bytes(n)}});
+}
+
 int Engine::run(cudaStream_t st, bool use_graph, int mode)
 {
     if (h_cl_.empty()) return 0;
@@ -542,7 +621,7 @@ int Engine::run(cudaStream_t st, bool use_graph, int mode)
         RD_CK(launch_reset(v0, st));
         RD_CK(cudaMemcpyAsync(v0.ns, given_ns.data(), 4 * given_ns.size(),
                               cudaMemcpyHostToDevice, st));
-        if (int rc = finish_setup_after_choose(st, true)) return rc;
+        if (int rc = finish_setup_after_choose(st, true, mode == RUN_DECIMATE_ONLY)) return rc;
         const EngineView v1 = view();
         RD_CK(launch_set_given(v1, mode == RUN_DECIMATE_ONLY ? 1 : 0, st));
         if (mode == RUN_DECIMATE_ONLY) {
@@ -555,10 +634,7 @@ int Engine::run(cudaStream_t st, bool use_graph, int mode)
         // one large cloud: GPU-wide choose rounds; otherwise one CTA per cloud
         const bool rounds = h_cl_.size() == 1 && h_cl_[0].n_own >= (1 << 16);
         if (rounds) {
-            RD_CK(bHash_.ensure(4 * (size_t)choose_hash_buckets()));
-            RD_CK(bSurv_.ensure((size_t)h_cl_[0].n_own + 16));
-            RD_CK(bSel_.ensure(4 * (size_t)(h_cl_[0].n_own + 2)));
-            RD_CK(bSelTmp_.ensure(choose_select_scratch_bytes(h_cl_[0].n_own)));
+            RD_CK(ensure_choose());
         }
         EngineView v0 = view();
         RD_CK(launch_reset(v0, st));
@@ -691,22 +767,23 @@ int Engine::ensure_pass_buffers(cudaStream_t st)
 {
     const size_t n = (size_t)total_points_;
     const size_t blocks = (size_t)cull_blocks();
-    if (cull_) {
-        RD_CK(bPs_.ensure(sizeof(float) * (n * pad_dim(dim_) + 4)));
-        RD_CK(bSorder_.ensure(sizeof(int32_t) * (2 * n + 1)));
-        RD_CK(bSpatialTmp_.ensure(spatial_prep_scratch_bytes(total_points_)));
-        RD_CK(bBox_.ensure(sizeof(float) * (4 * dim_ * blocks + 1)));
-        RD_CK(bSlack_.ensure(sizeof(float) * (blocks + 1)));
-        RD_CK(bLslack_.ensure(sizeof(float) * (blocks + 1)));
-        RD_CK(bBlen_.ensure(sizeof(int32_t) * (blocks + 1)));
-        RD_CK(bKsp_.ensure(sizeof(int32_t) * (n + 1)));
-        RD_CK(bBlist_.ensure(sizeof(int32_t) * (CAND_MAX * blocks + 1)));
-    }
+    if (cull_)
+        RD_CK(ensure_together(slab_pass_, {
+            {&bPs_, sizeof(float) * (n * pad_dim(dim_) + 4)},
+            {&bSorder_, sizeof(int32_t) * (2 * n + 1)},
+            {&bSpatialTmp_, spatial_prep_scratch_bytes(total_points_)},
+            {&bBox_, sizeof(float) * (4 * dim_ * blocks + 1)},
+            {&bSlack_, sizeof(float) * (blocks + 1)},
+            {&bLslack_, sizeof(float) * (blocks + 1)},
+            {&bBlen_, sizeof(int32_t) * (blocks + 1)},
+            {&bKsp_, sizeof(int32_t) * (n + 1)},
+            {&bBlist_, sizeof(int32_t) * (CAND_MAX * blocks + 1)},
+        }));
     if (lists_) {
         const cudaError_t e = ensure_list_buffers();
         if (e == cudaErrorMemoryAllocation && !current_arena()) {
             (void)cudaGetLastError();
-            for (DevBuf* b : {&bLr_[0], &bLr_[1], &bLs_[0], &bLs_[1], &bEdit_, &bHpre_, &bMv_})
+            for (DevBuf* b : {&bLr_[0], &bLr_[1], &bLs_[0], &bLs_[1], &bEdit_, &bHpre_, &bMv_, &slab_list_})
                 b->release();
             lay_out_lists(false);
             RD_CK(upload(bCl_, h_cl_, st));
@@ -721,15 +798,15 @@ int Engine::ensure_pass_buffers(cudaStream_t st)
 cudaError_t Engine::ensure_list_buffers()
 {
     const size_t rows = (size_t)list_rows_;
-    cudaError_t e = bHpre_.ensure(4 * (size_t)(hist_ints_ + 1));
-    auto take = [&](DevBuf& b, size_t bytes) { if (e == cudaSuccess) e = b.ensure(bytes); };
-    for (int b = 0; b < 2; ++b) {
-        take(bLr_[b], sizeof(float) * (rows * pad_dim(dim_) + 4));
-        take(bLs_[b], sizeof(int32_t) * (rows + 1));
-    }
-    take(bEdit_, sizeof(int32_t) * (rows + 1));
-    take(bMv_, sizeof(float) * ((size_t)(2 * dim_ + 1) * n_slots_ + 1));
-    return e;
+    return ensure_together(slab_list_, {
+        {&bHpre_, 4 * (size_t)(hist_ints_ + 1)},
+        {&bLr_[0], sizeof(float) * (rows * pad_dim(dim_) + 4)},
+        {&bLr_[1], sizeof(float) * (rows * pad_dim(dim_) + 4)},
+        {&bLs_[0], sizeof(int32_t) * (rows + 1)},
+        {&bLs_[1], sizeof(int32_t) * (rows + 1)},
+        {&bEdit_, sizeof(int32_t) * (rows + 1)},
+        {&bMv_, sizeof(float) * ((size_t)(2 * dim_ + 1) * n_slots_ + 1)},
+    });
 }
 
 // Tiles (clouds) by decreasing evolve points; the heavy ones (evolved by a
@@ -766,7 +843,7 @@ int Engine::plan_workspace(int mode)
     build_tile_order();
     RD_CK(upload(bTileOrder_, h_tile_order_, nullptr));
     if (mode == RUN_EVOLVE_ONLY || mode == RUN_DECIMATE_ONLY) {
-        if (int rc = finish_setup_after_choose(nullptr)) return rc;
+        if (int rc = finish_setup_after_choose(nullptr, false, mode == RUN_DECIMATE_ONLY)) return rc;
         if (mode == RUN_EVOLVE_ONLY) {
             cull_ = cull_possible();
             if (int rc = ensure_pass_buffers(nullptr)) return rc;
@@ -775,10 +852,7 @@ int Engine::plan_workspace(int mode)
     }
     if (mode == RUN_CHOOSE_ONLY) {
         if (h_cl_.size() == 1 && h_cl_[0].n_own >= (1 << 16)) {
-            RD_CK(bHash_.ensure(4 * (size_t)choose_hash_buckets()));
-            RD_CK(bSurv_.ensure((size_t)h_cl_[0].n_own + 16));
-            RD_CK(bSel_.ensure(4 * (size_t)(h_cl_[0].n_own + 2)));
-            RD_CK(bSelTmp_.ensure(choose_select_scratch_bytes(h_cl_[0].n_own)));
+            RD_CK(ensure_choose());
         }
         return 0;
     }

@@ -30,8 +30,8 @@ enum : int {
 };
 
 // neighbour-list capacity of the decimation, per chosen point: at least
-// DEC_NB_MIN_PER_POINT, more while the whole list buffer stays within
-// DEC_NB_BUDGET entries (lists that do not fit fall back to walking the hash
+// DEC_NB_MIN_PER_POINT, more (up to all points of the largest group) while the whole
+// list buffer stays within DEC_NB_BUDGET entries (lists that do not fit fall back to walking the hash
 // buckets)
 constexpr int DEC_NB_MIN_PER_POINT = 32;
 constexpr int DEC_NB_MAX_PER_POINT = 4096;
@@ -192,6 +192,8 @@ constexpr int DEC_SAMPLES = 32;              // points sampled for the choice be
 inline int dec_smem_bytes(const EngineView& v) { return v.dec_dyn; }
 // bytes for groups of up to `points` points
 int dec_dyn_bytes(int points);
+// largest set whose bit matrices that includes
+int dec_smem_points();
 
 // launch configuration picked by the tuner per (dim, cloud size, r1) bucket
 struct TuneParams {

@@ -39,7 +39,8 @@ constexpr int64_t LIST_WS_MAX = int64_t(16) << 30;
 struct DevBuf {
     void* p = nullptr;
     size_t bytes = 0;
-    bool borrowed = false;   // carved from an arena: never freed here
+    bool borrowed = false;   // carved from an arena or a slab: never freed here
+    bool in_slab = false;    // from a slab (ensure_together)
     uint64_t gen = 0;        // arena generation it was carved from
     cudaError_t ensure(size_t want);
     void release();
@@ -47,6 +48,24 @@ struct DevBuf {
     template <class T>
     T* as() const { return static_cast<T*>(p); }
 };
+
+// Buffers that are sized at the same time, carved from one allocation (the slab, 256-byte
+// aligned); those above SLAB_ITEM_MAX get one each.  All or none move: when one has outgrown its
+// place, the slab is allocated anew, with an eighth more for those that grew, and
+// the contents of all are lost.  Under an arena every buffer is carved from that.
+//
+// A new engine makes 4 device allocations for a solve instead of 60, and a second cloud
+// of the same size none, where each chosen point more moved ten buffers.  Solves, one
+// allocation per buffer and an exact layout / this (and Engine::chosen_room), ms:
+// ridge_detection() of 1,000 points 2.4 / 1.9, of 77,777 12.3 / 10.0, of 1M 46 / 33;
+// another cloud each time on one handle 10 points 0.54 / 0.23, 1,000 1.31 / 0.92, 20,000
+// 4.35 / 4.07; new handles of 4,000 small clouds 31 / 16.
+struct SlabItem {
+    DevBuf* buf;
+    size_t bytes;
+};
+constexpr size_t SLAB_ITEM_MAX = size_t(32) << 20;
+cudaError_t ensure_together(DevBuf& slab, const std::vector<SlabItem>& items);
 
 struct RunStats {
     int64_t loop_iters = 0;       // graph/host loop iterations
@@ -151,8 +170,9 @@ public:
     std::string last_error;
 
 private:
-    // ns_given: the chosen counts are those in given_ns
-    int finish_setup_after_choose(cudaStream_t st, bool ns_given = false);
+    // ns_given: the chosen counts are those in given_ns; exact: no room beyond them
+    int finish_setup_after_choose(cudaStream_t st, bool ns_given = false, bool exact = false);
+    cudaError_t ensure_choose();
     // per cloud 64-bit pairs and 32-bit chosen count, passes and errors; then the counters
     static size_t res_bytes(size_t nc) { return 20 * (nc + 1) + 4 * CTR_COUNT; }
     // once per run: the process-wide culling switch as this run takes it
@@ -161,6 +181,7 @@ private:
     void lay_out_lists(bool keep);
     int64_t list_bytes() const;
     int64_t cull_blocks() const;
+    int chosen_room(int ns);
     int ensure_pass_buffers(cudaStream_t st);
     cudaError_t ensure_list_buffers();
     int start_passes(cudaStream_t st);
@@ -187,12 +208,17 @@ private:
     int assign_grid_ = 0;
     RunStats stats_;
 
+    // buffers sized by the batch, by a large choose, by the chosen counts, for the passes
+    // and for the kept lists
+    DevBuf slab_setup_, slab_choose_, slab_chosen_, slab_pass_, slab_list_;
     DevBuf bCl_, bGr_, bChunkCloud_, bSlotCloud_;
     DevBuf bP_, bS_, bKeys_, bPg_, bHist_, bCnt_, bBase_, bNext_, bHash_, bSurv_;
     DevBuf bRes_, bPhase_, bCont_, bPasses_, bOuter_, bKbDone_;
     std::vector<uint64_t> h_res_;
     DevBuf bActCloud_, bActPre_, bGroupConv_, bReady_, bDnbOff_, bDnb_, bDbig_, bDcpre_;
-    int dec_smem_max_ = 0;
+    int dec_smem_max_ = 0, dec_dyn_ = 0;
+    int room_ = 0;                // chosen points a run of one cloud was last laid out for
+    int64_t room_points_ = -1;    // and its points
     int dec_nb_pp_ = DEC_NB_MIN_PER_POINT;
     bool fused_ = false;
     bool cull_on_ = true;         // the culling switch when this run started

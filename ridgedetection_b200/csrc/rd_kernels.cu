@@ -3647,6 +3647,16 @@ cudaError_t launch_set_given(const EngineView& v, int queue_decimation, cudaStre
     return cudaGetLastError();
 }
 
+int dec_smem_points()
+{
+    static const int n = [] {
+        int m = 1;
+        while (m < DEC_BITS_MAX && dec_matrix_bytes(m + 1) <= DEC_BITS_SMEM) ++m;
+        return m;
+    }();
+    return n;
+}
+
 int dec_dyn_bytes(int points)
 {
     // the largest group's matrices where they fit; otherwise its counts, and room
