@@ -1765,6 +1765,7 @@ __device__ __forceinline__ void next_iteration(const EngineView& v, int a, cudaG
     v.ctr[CTR_ITERS] = it;
     if (it >= v.max_iters && a > 0) {
         v.ctr[CTR_ERR] |= ERRB_EVOLVE_CAP;
+        v.ctr[CTR_NACT] = 0;   // nor do the graph round's passes after this one
         a = 0;
     }
     v.ctr[CTR_ACTIVE] = a;
