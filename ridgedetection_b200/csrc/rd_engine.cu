@@ -432,8 +432,8 @@ static int ceil_log2(int64_t x)
 
 // The chosen points a run of one cloud is laid out for: a few more than it has, and as
 // many as the last one where that does, so that the clouds of a handle share their
-// buffers and their graph (1,000 points, another cloud each time: 1,340 us, the same
-// cloud 790, where every count was laid out exactly).
+// buffers and their graph.  Capturing and instantiating it anew takes about 0.4 ms
+// (1,000 points, another cloud each time: 1.31 ms with exact counts, 0.92 with room).
 int Engine::chosen_room(int ns)
 {
     const CloudDesc& cd = h_cl_[0];

@@ -4,9 +4,11 @@
 // share the point dimension DIM:
 //   choose      one CTA per cloud, greedy r1-separated subset in input order
 //               over a hashed uniform grid (exact test, grid only prunes);
-//   evolve      passes of  assign -> chunk scan -> key bases -> stable
-//               scatter -> ordered sum + shift -> control, over all clouds still
-//               evolving; the per-chosen coordinate sums are formed in cloud-point
+//   evolve      passes over all clouds still evolving: assignment, of the blocks of
+//               points whose keys can have changed, then the member lists of the keys
+//               with changes (merge of the pass's edits, or chunk scan and stable
+//               scatter of a cloud that regroups), their ordered sums and shifts, and
+//               control; the per-chosen coordinate sums are formed in cloud-point
 //               index order, exactly as the reference's serial loop forms them;
 //   decimate    one CTA per group with the reference's in-order semantics;
 //   loop        a device flag says whether any cloud is unfinished; it drives a
@@ -31,8 +33,8 @@ enum : int {
 
 // neighbour-list capacity of the decimation, per chosen point: at least
 // DEC_NB_MIN_PER_POINT, more (up to all points of the largest group) while the whole
-// list buffer stays within DEC_NB_BUDGET entries (lists that do not fit fall back to walking the hash
-// buckets)
+// list buffer stays within DEC_NB_BUDGET entries (lists that do not fit fall back to
+// walking the hash buckets)
 constexpr int DEC_NB_MIN_PER_POINT = 32;
 constexpr int DEC_NB_MAX_PER_POINT = 4096;
 constexpr int64_t DEC_NB_BUDGET = int64_t(1) << 28;

@@ -65,8 +65,8 @@ __device__ __forceinline__ CloudDesc cloud_desc(const EngineView& v, const int c
     return v.single ? v.one : v.cl[c];
 }
 
-// Work lists over the clouds still evolving, rebuilt by k_loopcond after every
-// iteration: act_cloud[a] is the a-th evolving cloud and act_pre[kind] the
+// Work lists over the clouds still evolving, rebuilt by loop_condition when a cloud
+// has converged: act_cloud[a] is the a-th evolving cloud and act_pre[kind] the
 // exclusive prefix of its work items (ACT_* in rd_engine.cuh), so kernels
 // launched over fixed grids touch only active work.
 

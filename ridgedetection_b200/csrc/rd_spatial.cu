@@ -4,7 +4,8 @@
 // The brute-force assignment of rd/cpu/brute_force/evolve.hpp:43-66 keeps a
 // point's nearest chosen point only when it lies within r1.  A group of points
 // that are close together in space therefore needs only the chosen points
-// within r1 of the group's bounding box.  This file builds, once per run (the
+// within r1 of the group's bounding box (of the nearer of its two: the order is cut
+// where it jumps from one occupied place to another).  This file builds, once per run (the
 // evolve points never move), a copy of every cloud's points in a spatial
 // order -- cells of edge r1/4, Morton order of the cells, the packed slot
 // order inside a cell.  The copy pads DIM 3 to four floats per point, so that
