@@ -172,3 +172,28 @@ def test_lists_that_do_not_fit_the_device(rdb, batch):
         del hold
         torch.cuda.empty_cache()
     assert p == passes and all(bits_equal(x, y) for x, y in zip(got, want))
+
+
+@pytest.mark.parametrize("extra", [-1, 0, 1])
+@pytest.mark.parametrize("rows", [96, 224])
+def test_list_chunk_edges(rdb, rows, extra):
+    """Lists of whole chunks of the merge (96 rows where several clouds evolve, 224 for one) and
+    one row less or more, in a batch and alone, against the oracle."""
+    import oracle as O
+    clouds = []
+    for k in (1, 2, 3):
+        n = k * rows + extra
+        r = np.random.default_rng(100 * k + rows + extra)
+        # two clusters of n points whose chosen points travel, so that members change sides
+        x = np.concatenate([r.normal(0.0, 0.12, n), r.normal(0.7, 0.12, n)])
+        P = np.stack([x, r.normal(0.0, 0.1, 2 * n)], 1).astype(np.float32)
+        clouds.append((P[r.permutation(2 * n)], 0.5, 1.0))
+        clouds.append((r.normal(0.0, 0.05, (n, 2)).astype(np.float32), 0.5, 1.0))   # one list
+    packed, descs = rdb.pack_clouds(clouds)
+    b = rdb.BatchedRidgeDetection()
+    b.run(packed, descs)
+    for c, (P, r1, r2) in enumerate(clouds):
+        want = O.ridge_bf(P, r1, r2)[0]
+        assert bits_equal(b.chosen_points(c), want), c
+        assert bits_equal(rdb.ridge_detection(P, r1, r2)[0], want), c
+    b.close()
