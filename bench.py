@@ -44,16 +44,10 @@ sys.path.insert(0, ROOT)
 
 METRIC = "evolve pairs/s"
 UNIT = "pairs/s"
-# DRAM traffic of one assignment launch on the helix3d_1m workload, from one
-# ncu capture each (dram__bytes_read.sum + dram__bytes_write.sum):
-#   k_assign_cull (culled, the default) evaluates only the blocks of points whose
-#     keys can have changed, so one launch stands for no other and none is
-#     given; the 20 B per point (12 B sorted point + 4 B slot read, 4 B key
-#     written) are what a launch that evaluates every point needs;
-#   k_assign (all pairs): 12,039,936 + 0 bytes, the 1,000,000 points x 12 B
-#     read once.
-# Applies to helix3d_1m only.
-ASSIGN_TRAFFIC_BYTES = {}
+# DRAM traffic of one launch of the all-pairs assignment on the helix3d_1m workload,
+# from one ncu capture (dram__bytes_read.sum + dram__bytes_write.sum): the 1,000,000
+# points x 12 B read once.  The culled assignment looks only at the blocks of points
+# whose keys can have changed, so no launch stands for another and no rate is given.
 ALL_PAIRS_TRAFFIC_BYTES = {"helix3d_1m": 12_039_936}
 
 
@@ -388,11 +382,6 @@ def run_b200_bf(args, world, rank, local):
     peak = ctypes.c_double(0)
     L.check(lib.rd_probe_fp32_peak(ctypes.byref(peak), ctypes.c_void_p(stream.cuda_stream)))
     nominal = 148 * 128 * 2 * 1.965e9 / 1e12
-    hbm_peak, hbm_src = measured_hbm_gbs()
-    # culled kernel, when it evaluates every point: a sorted point and its slot
-    # read, its key written (an average launch evaluates fewer)
-    cull_bytes = n * (4 * dim + 4 + 4)
-    cull_gbs = cull_bytes / (assign_ms_avg * 1e-3) / 1e9
     all_pairs = {"kernel": "k_assign", "bound": "fp32", "achieved": ap_tflops,
                  "peak": peak.value, "unit": "TFLOP/s", "frac": ap_tflops / peak.value,
                  "peak_source": "measured FMA-chain probe (rd_probe_fp32_peak); "
@@ -404,18 +393,15 @@ def run_b200_bf(args, world, rank, local):
                  # ceiling in these units is half the FMA FLOP rate
                  "frac_of_nonfused_peak": ap_tflops / (peak.value / 2),
                  "traffic": ALL_PAIRS_TRAFFIC_BYTES.get(args.workload)}
-    if culled:
-        roofline = {"bound": "hbm", "kernel": "k_assign_cull", "achieved": cull_gbs,
-                    "peak": hbm_peak, "unit": "GB/s", "frac": cull_gbs / hbm_peak,
-                    "peak_source": hbm_src, "bytes_per_launch": cull_bytes,
-                    "ms_per_launch": assign_ms_avg, "launches": pst.assign_launches,
-                    "traffic": ASSIGN_TRAFFIC_BYTES.get(args.workload)}
-    else:
-        roofline = dict(all_pairs)
+    # the kernel whose work per launch is known; the culled one (most launches skip most
+    # blocks) is reported by its time alone
+    roofline = dict(all_pairs)
+    assign_cull = {"kernel": "k_assign_cull", "ms_per_launch": assign_ms_avg,
+                   "launches": pst.assign_launches} if culled else None
 
-    # like-for-like with the CPU baseline: evolve passes from the chosen set
-    # right after choose, nothing else
-    sw_pairs, sw_s, sw_passes = same_work_gpu(dP, r1)
+    # beside the CPU baseline: evolve passes from the chosen set right after choose,
+    # nothing else
+    sw_pairs, sw_first_s, sw_s, sw_passes = same_work_gpu(dP, r1)
     if world > 1:
         torch.distributed.barrier()
     rd.close()
@@ -456,25 +442,28 @@ def run_b200_bf(args, world, rank, local):
         "pairs_per_step": pairs_step, "loop_iters_per_step": iters_step,
         "ns_final": ns_final,
         "roofline": roofline,
-        "all_pairs": all_pairs,
+        "all_pairs": all_pairs, "assign_cull": assign_cull,
         "e2e": {"value": e2e_val, "unit": UNIT, "h2d_bytes_per_step": int(P.nbytes),
                 "d2h_bytes_per_step": int(ns_final * dim * 4)},
-        # per loop iteration: assign (culled: with the key histogram), chunk
-        # scan (with the key bases), scatter, sum+shift (with the control
-        # step), decimate (with the loop condition); per solve about 40 more
+        # per loop iteration: assign, chunk scan (with the key bases), scatter,
+        # merge and fold (with the control step), decimate (with the loop
+        # condition); per solve about 40 more
         # (reset, choose rounds with their survivor compaction, spatial order)
         "gpu_launches": args.steps * (5 * iters_step + 40),
         "clocks": clocks,
         "cpu_baseline": cpu,
     }
     line["same_work"] = {
-        "what": "evolve passes over the whole cloud from the chosen set right after choose "
-                "(the CPU baseline's work), rd_evolve_ws with caller scratch, per-pass time from "
-                "a (k+1)-pass minus a 1-pass call",
-        "gpu_pairs_per_s": sw_pairs / sw_s, "gpu_ms_per_pass": sw_s * 1e3,
-        "pairs_per_pass": sw_pairs, "passes": sw_passes,
+        "what": "one evolve pass over the whole cloud from the chosen set right after choose "
+                "(the CPU baseline's work): a 1-pass rd_evolve_ws call with caller scratch, "
+                "its spatial order and lists included",
+        "gpu_pairs_per_s": sw_pairs / sw_first_s, "gpu_ms_per_pass": sw_first_s * 1e3,
+        "pairs_per_pass": sw_pairs,
         "cpu_pairs_per_s": cpu["value"] if cpu else None,
-        "gpu_over_cpu": (sw_pairs / sw_s / cpu["value"]) if cpu and cpu.get("value") else None,
+        "gpu_over_cpu": (sw_pairs / sw_first_s / cpu["value"])
+        if cpu and cpu.get("value") else None,
+        # the passes after the first touch only what the last one changed
+        "later_passes": {"ms_per_pass": sw_s * 1e3, "passes": sw_passes - 1},
     }
     line.update(subs)
     print(json.dumps(line))
@@ -483,11 +472,12 @@ def run_b200_bf(args, world, rank, local):
 
 
 def same_work_gpu(dP, r1, passes=20):
-    """Evolve passes over the cloud dP from the chosen set right after choose
-    -- the work the CPU baseline times -- through rd_evolve_ws with caller
-    scratch.  A (passes+1)-pass call and a 1-pass call are timed with CUDA
-    events; their difference per pass removes the call's setup.  Returns
-    (pairs per pass, seconds per pass, passes run in the long call)."""
+    """Evolve passes over the cloud dP from the chosen set right after choose, through
+    rd_evolve_ws with caller scratch, timed with CUDA events: a 1-pass call, whose pass
+    evaluates every point as the CPU baseline's passes do, and the difference of a
+    (passes+1)-pass call per further pass, which touches only what changed.  Returns
+    (pairs per pass, seconds of the 1-pass call, seconds per further pass, passes run in
+    the long call)."""
     import torch
     from ridgedetection_b200 import _lib as L
     lib = L.lib()
@@ -519,7 +509,7 @@ def same_work_gpu(dP, r1, passes=20):
         times[k] = (a.elapsed_time(b), ran.value)   # the second round (warm) is kept
     (t1, p1), (tk, pk) = times[1], times[passes + 1]
     per_pass_s = max(1e-9, (tk - t1) * 1e-3 / max(1, pk - p1))
-    return float(n) * ns.value, per_pass_s, pk
+    return float(n) * ns.value, t1 * 1e-3, per_pass_s, pk
 
 
 def measured_hbm_gbs():
@@ -680,10 +670,10 @@ def run_b200_tiled(args, world, rank, local, embedded=False):
                      "launches": pst.assign_launches, "traffic": None},
         "e2e": {"value": world * n / (e2e_ms * 1e-3), "unit": "points/s",
                 "h2d_bytes_per_step": int(P.nbytes), "d2h_bytes_per_step": int(ns_final * dim * 4)},
-        # per loop iteration: tile evolve, seven neighbour-list kernels of the
-        # global decimation, decimate (with the loop condition); per solve
-        # about 12 more (tile build, reset, choose)
-        "gpu_launches": args.steps * (12 + 9 * max(1, st.loop_iters)),
+        # per loop iteration: tile evolve, seven neighbour-list kernels and the
+        # rounds of the global decimation, decimate (with the loop condition);
+        # per solve about 12 more (tile build, reset, choose)
+        "gpu_launches": args.steps * (12 + 10 * max(1, st.loop_iters)),
         "clocks": clocks,
         "cpu_baseline": cpu,
     }
