@@ -495,8 +495,8 @@ int Engine::finish_setup_after_choose(cudaStream_t st, bool ns_given, bool exact
         hoff += (int64_t(1) << hb) + 1;
     }
     // shared-memory budgets (ints)
-    hist_smem_ = std::min(max_ns, 24 * 1024);
-    scat_smem_ = std::min(max_ns, 4 * 1024);
+    hist_smem_ = std::min(max_ns, HIST_SMEM_MAX);
+    scat_smem_ = std::min(max_ns, SCAT_SMEM_MAX);
     dec_nb_pp_ = (int)std::max<int64_t>(
         DEC_NB_MIN_PER_POINT,
         std::min({(int64_t)DEC_NB_MAX_PER_POINT, DEC_NB_BUDGET / std::max<int64_t>(sscr, 1), max_tot}));
@@ -578,8 +578,10 @@ int Engine::build_graph(cudaStream_t st)
                     : launch_pass(dim_, v, tune, assign_grid_, lc, cap_stream_, nullptr, nullptr, p > 0);
     cudaGraph_t out = nullptr;
     cudaError_t e3 = cudaStreamEndCapture(cap_stream_, &out);
-    if (e1 != cudaSuccess) return fail("capture pass", e1);
-    if (e3 != cudaSuccess) return fail("end capture", e3);
+    if (e1 != cudaSuccess || e3 != cudaSuccess) {
+        graph_ = nullptr;   // half captured: left to the process, not destroyed
+        return fail(e1 != cudaSuccess ? "capture pass" : "end capture", e1 != cudaSuccess ? e1 : e3);
+    }
     RD_CK(cudaGraphInstantiate(&exec_, graph_, 0));
     graph_key_ = key;
     return 0;

@@ -190,12 +190,20 @@ struct EngineView {
 inline int dec_list_bytes(int points) { return ((points * 5 + 15) / 16) * 16 + 4 * ((points + 31) / 32) + 16; }
 constexpr int DEC_BITS_MAX = 4096;           // points decimated over bit matrices
 constexpr int DEC_BITS_SMEM = 200 * 1024;    // shared memory for them
+// most dynamic shared memory of the decimation: the matrices, or the counts and flags
+// of DEC_SMEM_MAX_POINTS points (dec_list_bytes)
+constexpr int DEC_SMEM_MOST = DEC_BITS_SMEM;
+static_assert(DEC_SMEM_MAX_POINTS * 5 + 16 + DEC_SMEM_MAX_POINTS / 8 + 32 <= DEC_SMEM_MOST, "decimation smem");
 constexpr int DEC_SAMPLES = 32;              // points sampled for the choice between them and lists
 inline int dec_smem_bytes(const EngineView& v) { return v.dec_dyn; }
 // bytes for groups of up to `points` points
 int dec_dyn_bytes(int points);
 // largest set whose bit matrices that includes
 int dec_smem_points();
+
+// points of an assignment chunk (block x items), and the most ints of shared memory for
+// a chunk's key histogram and a scatter warp's key starts
+constexpr int CHUNK_PTS_MAX = 2048, HIST_SMEM_MAX = 24 * 1024, SCAT_SMEM_MAX = 4 * 1024;
 
 // launch configuration picked by the tuner per (dim, cloud size, r1) bucket
 struct TuneParams {

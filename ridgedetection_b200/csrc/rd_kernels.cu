@@ -3248,11 +3248,27 @@ __global__ void k_reset(EngineView v)
     v.pairs[c] = 0;
 }
 
+// The dynamic shared memory a kernel may take is a property of the function, not of a
+// launch, and another thread's run sets it between this one's call and its launch: it is
+// always set to the most any run takes.  (Set to what the own run takes, a run of
+// larger sets beside one of smaller ones failed to launch or to capture.)
 template <int DIM, int BLOCK, int ITEMS>
-cudaError_t set_assign_attrs(int dyn)
+cudaError_t set_assign_attrs()
 {
     return cudaFuncSetAttribute(k_assign<DIM, BLOCK, ITEMS>,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize, dyn);
+                                cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * HIST_SMEM_MAX);
+}
+template <int DIM>
+cudaError_t set_decimate_attrs()
+{
+    return cudaFuncSetAttribute(k_decimate<DIM, 512>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                DEC_SMEM_MOST);
+}
+template <int DIM>
+cudaError_t set_scatter_attrs()
+{
+    return cudaFuncSetAttribute(k_scatter_cta<DIM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                4 * (CHUNK_PTS_MAX + std::max(SCAT_W * SCAT_HMAX, SCAT_SMEM_MAX)));
 }
 
 // launch with programmatic stream serialisation (pdl != 0): the kernel may
@@ -3314,19 +3330,17 @@ int merge_grid(const EngineView& v)
 template <int DIM>
 cudaError_t prepare_pass_dim(const EngineView& v, const TuneParams& tp)
 {
-    const int hist_bytes = v.hist_smem * 4;
     cudaError_t e = cudaErrorInvalidValue;
 #define RD_PREP_CASE(B, I) \
-    if (tp.block == B && tp.items == I) e = set_assign_attrs<DIM, B, I>(hist_bytes);
+    if (tp.block == B && tp.items == I) e = set_assign_attrs<DIM, B, I>();
     RD_PREP_CASE(128, 8) RD_PREP_CASE(128, 4) RD_PREP_CASE(256, 4) RD_PREP_CASE(256, 8)
     RD_PREP_CASE(128, 16)
 #undef RD_PREP_CASE
     if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(k_decimate<DIM, 512>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             dec_smem_bytes(v));
+    if (dec_smem_bytes(v) > DEC_SMEM_MOST || v.chunk_max > CHUNK_PTS_MAX) return cudaErrorInvalidValue;
+    e = set_decimate_attrs<DIM>();
     if (e != cudaSuccess) return e;
-    return cudaFuncSetAttribute(k_scatter_cta<DIM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                scatter_cta_smem_bytes(v));
+    return set_scatter_attrs<DIM>();
 }
 
 // the kernels of an evolve pass; control: see k_merge_fold
@@ -3567,8 +3581,7 @@ cudaError_t prepare_tile_pass(int dim, const EngineView& v, int* cl_grid)
             e = tile_cl_prepare<DIM>(cl_grid);
             if (e != cudaSuccess) return e;
         }
-        return cudaFuncSetAttribute(k_decimate<DIM, 512>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    dec_smem_bytes(v));
+        return set_decimate_attrs<DIM>();
     });
 }
 
@@ -3680,8 +3693,7 @@ cudaError_t launch_decimate(int dim, const EngineView& view, int64_t points, cud
     cudaError_t e = cudaSuccess;
     e = with_dim(dim, [&](auto D) {
         constexpr int DIM = decltype(D)::value;
-        cudaError_t r = cudaFuncSetAttribute(k_decimate<DIM, 512>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        cudaError_t r = set_decimate_attrs<DIM>();
         // one large group: its buckets, lists and rounds over more of the GPU
         if (r == cudaSuccess && big) r = launch_decbig<DIM>(v, st);
         if (r == cudaSuccess) k_decimate<DIM, 512><<<grid, 512, smem, st>>>(v, 0, 0, 0);
@@ -3729,7 +3741,7 @@ template <int DIM, int B, int I>
 static int occ_of(int dyn)
 {
     int nb = 0;
-    if (set_assign_attrs<DIM, B, I>(dyn) != cudaSuccess) return 0;
+    if (set_assign_attrs<DIM, B, I>() != cudaSuccess) return 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_assign<DIM, B, I>, B, dyn);
     return nb;
 }

@@ -70,3 +70,35 @@ def test_steps_on_sets_of_many_sizes(rdb):
         assert bits_equal(S[:ns.value].cpu().numpy(), Se)
         L.check(lib.rd_decimate(3, p(S), ns.value, 0.6, ctypes.byref(left), st))
         assert bits_equal(S[:left.value].cpu().numpy(), O.decimate(Se, 0.6))
+
+
+def test_handles_in_several_threads(rdb):
+    """Each thread solves clouds of changing sizes with a handle of its own and with the module
+    function, beside the others."""
+    import threading
+    want = {}
+    for t in range(4):
+        for k in range(3):
+            P = _scaled(800 + 900 * t, 2 + t % 2, (1.0, 3.0, 0.6)[k], 7 * t + k)
+            want[t, k] = (P, O.ridge_bf(P, 0.2, 0.4)[0])
+    bad = []
+
+    def work(t):
+        try:
+            h = rdb.BruteForceRidgeDetection(800 + 900 * t, 0.2, 0.4, 2 + t % 2)
+            for i in range(12):
+                P, S = want[t, i % 3]
+                h.set_points(P)
+                h.ridge_detection()
+                if not bits_equal(h.chosen_points(), S) or not bits_equal(rdb.ridge_detection(P, 0.2, 0.4)[0], S):
+                    bad.append((t, i))
+            h.close()
+        except Exception as e:  # noqa: BLE001
+            bad.append((t, repr(e)))
+
+    threads = [threading.Thread(target=work, args=(t,)) for t in range(4)]
+    for th in threads:
+        th.start()
+    for th in threads:
+        th.join()
+    assert not bad
