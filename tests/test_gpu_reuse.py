@@ -1,6 +1,7 @@
 """One handle, several clouds: buffers, lists and graph of one cloud serve the next one.
 Chosen sets grow, shrink and grow again; bits against the oracle."""
 import ctypes
+import functools
 
 import numpy as np
 import pytest
@@ -25,16 +26,22 @@ def _scaled(n, dim, scale, seed):
     return np.ascontiguousarray(P * np.float32(scale))
 
 
-@pytest.mark.parametrize("n,dim,r1", [(700, 2, 0.2), (6000, 2, 0.1), (70_000, 3, 0.3), (12, 3, 0.3)])
+@functools.lru_cache(maxsize=None)
+def _ridge(n, dim, scale, seed, r1):
+    P = _scaled(n, dim, scale, seed)
+    return P, O.ridge_bf(P, r1, 2 * r1)[0]
+
+
+@pytest.mark.parametrize("n,dim,r1", [(700, 2, 0.2), (6000, 2, 0.1), (66_000, 3, 0.4), (12, 3, 0.3)])
 @pytest.mark.parametrize("mode", ["LOOP_GRAPH", "LOOP_HOST"])
 def test_one_handle_many_clouds(rdb, n, dim, r1, mode):
     h = rdb.BruteForceRidgeDetection(n, r1, 2 * r1, dim, loop_mode=getattr(rdb, mode))
     counts = set()
     for k, scale in enumerate((1.0, 0.5, 3.0, 0.7, 1.0, 3.1, 0.1)):
-        P = _scaled(n, dim, scale, 50 + k)
+        P, want = _ridge(n, dim, scale, 50 + k, r1)
         h.set_points(P)
         h.ridge_detection()
-        assert bits_equal(h.chosen_points(), O.ridge_bf(P, r1, 2 * r1)[0]), scale
+        assert bits_equal(h.chosen_points(), want), scale
         counts.add(h.get_chosen_samples_count())
     assert len(counts) > 1 or n < 100
     h.close()
